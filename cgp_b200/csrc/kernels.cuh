@@ -2602,105 +2602,126 @@ __device__ __forceinline__ int32_t decide_sdir(const LevelCtl* ctl, unsigned lon
 // chunk whose last improvements are few scatters them.  Consumes (zeroes)
 // cedges and cpairs.
 template <int W>
-__device__ __forceinline__ void split_sssp_slots(LevelCtl* ctl, int32_t group_dir) {
+__device__ __forceinline__ void split_sssp_slots(LevelCtl* ctl, int32_t group_dir, int lane) {
   const bool per_chunk = ctl->chunk_dir && ctl->mode == 2 && ctl->forced_dir < 0 &&
                          ctl->sssp_gather;
-  bool g_any = false, s_any = false;
-  for (int i = 0; i < W; ++i) {
-    uint64_t gm = 0;
+  // lane c: 32-slot chunk c, half (c & 1) of word c / 2
+  uint32_t bits = 0, gat = 0;
+  if (lane < 2 * W) {
+    bits = reinterpret_cast<const uint32_t*>(ctl->sssp_bits)[lane];
     if (per_chunk) {
-      for (int h = 0; h < 2; ++h) {
-        const uint64_t half = 0xffffffffULL << (32 * h);
-        // as the group rule: enough frontier edges, and enough (edge, slot)
-        // pairs that a scatter would cost more than the chunk's gather
-        if (ctl->cedges[2 * i + h] >= ctl->sssp_pull_edge_threshold &&
-            (ctl->sssp_pull_pair_unit == 0 || ctl->cpairs[2 * i + h] >= ctl->sssp_pull_pair_unit))
-          gm |= half;
-      }
+      // as the group rule: enough frontier edges, and enough (edge, slot)
+      // pairs that a scatter would cost more than the chunk's gather
+      if (ctl->cedges[lane] >= ctl->sssp_pull_edge_threshold &&
+          (ctl->sssp_pull_pair_unit == 0 || ctl->cpairs[lane] >= ctl->sssp_pull_pair_unit))
+        gat = bits;
     } else if (group_dir == kDirPull) {
-      gm = ~0ULL;
+      gat = bits;
     }
-    ctl->gsel[i] = ctl->sssp_bits[i] & gm;
-    ctl->ssel[i] = ctl->sssp_bits[i] & ~gm;
-    g_any |= ctl->gsel[i] != 0;
-    s_any |= ctl->ssel[i] != 0;
-    for (int h = 0; h < 2; ++h) {
-      ctl->sssp_chunk_levels += static_cast<uint32_t>(ctl->sssp_bits[i] >> (32 * h)) != 0u;
-      ctl->gather_chunk_levels += static_cast<uint32_t>(ctl->gsel[i] >> (32 * h)) != 0u;
-    }
+    reinterpret_cast<uint32_t*>(ctl->gsel)[lane] = gat;
+    reinterpret_cast<uint32_t*>(ctl->ssel)[lane] = bits & ~gat;
   }
-  for (int c = 0; c < 2 * kMaxW; ++c) ctl->cedges[c] = ctl->cpairs[c] = 0;
-  ctl->sdir = g_any ? kDirPull : kDirPush;
-  ctl->sscatter = s_any ? 1 : 0;
+  if (lane < 2 * kMaxW) ctl->cedges[lane] = ctl->cpairs[lane] = 0;
+  const unsigned with = __ballot_sync(kFull, bits != 0u);
+  const unsigned gathering = __ballot_sync(kFull, gat != 0u);
+  const unsigned scattering = __ballot_sync(kFull, (bits & ~gat) != 0u);
+  if (lane == 0) {
+    ctl->sssp_chunk_levels += __popc(with);
+    ctl->gather_chunk_levels += __popc(gathering);
+    ctl->sdir = gathering ? kDirPull : kDirPush;
+    ctl->sscatter = scattering ? 1 : 0;
+  }
+  __syncwarp();
 }
 
-// Expand mask for `level`: k-hop slots stop once their depth reaches k.
+// Expand mask for `level`: k-hop slots stop once their depth reaches k.  Lane
+// j takes slot 32c + j of every 32-slot chunk c (one 16-byte load each, a
+// ballot per chunk): a single thread walking the slots paid one dependent
+// load per slot, 45 us per level end at 256 slots.
 template <int W>
-__device__ void compute_expand(LevelCtl* ctl, const SlotDev* slots, int Qg, int level) {
-  for (int i = 0; i < W; ++i) ctl->expand[i] = ~0ULL;
-  for (int q = 0; q < Qg; ++q) {
-    const SlotDev s = slots[q];
-    if (s.kind == 3 && level - s.base >= s.k) ctl->expand[q >> 6] &= ~(1ULL << (q & 63));
+__device__ __forceinline__ void compute_expand(LevelCtl* ctl, const SlotDev* slots, int Qg,
+                                               int level, int lane) {
+#pragma unroll
+  for (int c = 0; c < 2 * W; ++c) {
+    const int q = 32 * c + lane;
+    bool stop = false;
+    if (q < Qg) {
+      const int4 s = *reinterpret_cast<const int4*>(slots + q);  // kind, source, k, base
+      stop = s.x == 3 && level - s.w >= s.z;
+    }
+    const unsigned m = __ballot_sync(kFull, stop);
+    if (lane == 0) reinterpret_cast<uint32_t*>(ctl->expand)[c] = ~m;
   }
+  __syncwarp();
 }
 
-// End of a level (one thread): profile, convergence, and the set-up of the
-// next level (counter reset, direction, expand mask).
+// End of a level (one warp, all lanes call): profile, convergence, and the
+// set-up of the next level (counter reset, direction, expand mask).
 template <int W>
-__device__ void level_end(GroupDev& g) {
+__device__ __forceinline__ void level_end(const GroupDev& g, int lane) {
   LevelCtl* ctl = g.ctl;
   if (ctl->done) return;
   const int l = ctl->level;
   const int par = l & 1;
-  const unsigned long long nextc = ctl->count[par ^ 1];
-  if (g.prof != nullptr && l < ctl->profile_cap) {
-    LevelProfile p;
-    p.level = l;
-    p.dir = ctl->dir;
-    p.frontier = ctl->count[par];
-    p.edges = ctl->edges[par];
-    p.next = nextc;
-    p.active0 = ctl->active[par ^ 1][0];
-    p.new_pairs = ctl->lc.new_pairs;
-    p.pull_vertices = ctl->lc.pull_vertices;
-    p.pull_edges = ctl->lc.pull_edges;
-    p.sssp_pairs = ctl->lc.sssp_pairs;
-    p.sssp_active = ctl->lc.sssp_active;
-    p.improved = ctl->lc.improved;
-    p.spull_vertices = ctl->lc.spull_vertices;
-    p.spull_edges = ctl->lc.spull_edges;
-    p.sdir = ctl->sdir;
-    p.reserved = 0;
-    g.prof[l] = p;
+  const unsigned long long count = ctl->count[par], edges = ctl->edges[par];
+  const unsigned long long nextc = ctl->count[par ^ 1], nexte = ctl->edges[par ^ 1];
+  __syncwarp();
+  if (lane < W) ctl->active[par][lane] = 0;
+  if (lane == 0) {
+    const LevelCounters lc = ctl->lc;
+    if (g.prof != nullptr && l < ctl->profile_cap) {
+      LevelProfile p;
+      p.level = l;
+      p.dir = ctl->dir;
+      p.frontier = count;
+      p.edges = edges;
+      p.next = nextc;
+      p.active0 = ctl->active[par ^ 1][0];
+      p.new_pairs = lc.new_pairs;
+      p.pull_vertices = lc.pull_vertices;
+      p.pull_edges = lc.pull_edges;
+      p.sssp_pairs = lc.sssp_pairs;
+      p.sssp_active = lc.sssp_active;
+      p.improved = lc.improved;
+      p.spull_vertices = lc.spull_vertices;
+      p.spull_edges = lc.spull_edges;
+      p.sdir = ctl->sdir;
+      p.reserved = 0;
+      g.prof[l] = p;
+    }
+    LevelCounters t = ctl->total;
+    t.new_pairs += lc.new_pairs;
+    t.pull_vertices += lc.pull_vertices;
+    t.pull_edges += lc.pull_edges;
+    t.sssp_pairs += lc.sssp_pairs;
+    t.sssp_active += lc.sssp_active;
+    t.improved += lc.improved;
+    t.spull_vertices += lc.spull_vertices;
+    t.spull_edges += lc.spull_edges;
+    ctl->total = t;
+    ctl->prev_improved = lc.improved;
+    ctl->prev_pull_edges = lc.pull_edges;
+    ctl->prev_dir = ctl->dir;
+    ctl->lc = LevelCounters{};
+    ctl->dense_count = 0;
+    ctl->hq_packed = 0;
+    ctl->total_frontier += count;
+    ctl->total_edges += edges;
+    if (ctl->dir == kDirPush) ctl->push_levels++;
+    else ctl->pull_levels++;
+    ctl->level = l + 1;
+    // Set up level l+1 even when it is empty, so that a serving loop can add
+    // sources to it and resume.
+    ctl->prev_count = count;
+    ctl->count[par] = 0;
+    ctl->edges[par] = 0;
   }
-  ctl->total.new_pairs += ctl->lc.new_pairs;
-  ctl->total.pull_vertices += ctl->lc.pull_vertices;
-  ctl->total.pull_edges += ctl->lc.pull_edges;
-  ctl->total.sssp_pairs += ctl->lc.sssp_pairs;
-  ctl->total.sssp_active += ctl->lc.sssp_active;
-  ctl->total.improved += ctl->lc.improved;
-  ctl->prev_improved = ctl->lc.improved;
-  ctl->prev_pull_edges = ctl->lc.pull_edges;
-  ctl->prev_dir = ctl->dir;
-  ctl->total.spull_vertices += ctl->lc.spull_vertices;
-  ctl->total.spull_edges += ctl->lc.spull_edges;
-  ctl->lc = LevelCounters{};
-  ctl->dense_count = 0;
-  ctl->hq_packed = 0;
-  ctl->total_frontier += ctl->count[par];
-  ctl->total_edges += ctl->edges[par];
-  if (ctl->dir == kDirPush) ctl->push_levels++;
-  else ctl->pull_levels++;
-  ctl->level = l + 1;
-  // Set up level l+1 even when it is empty, so that a serving loop can add
-  // sources to it and resume.
-  ctl->prev_count = ctl->count[par];
-  ctl->count[par] = 0;
-  ctl->edges[par] = 0;
-  for (int i = 0; i < W; ++i) ctl->active[par][i] = 0;
-  compute_expand<W>(ctl, g.slots, g.Qg, l + 1);
-  ctl->dir = decide_dir(ctl, nextc, ctl->edges[par ^ 1], any_bits<W>(ctl->bfs_bits));
-  split_sssp_slots<W>(ctl, decide_sdir<W>(ctl, nextc, ctl->edges[par ^ 1]));
+  __syncwarp();
+  compute_expand<W>(ctl, g.slots, g.Qg, l + 1, lane);
+  const int32_t dir = decide_dir(ctl, nextc, nexte, any_bits<W>(ctl->bfs_bits));
+  split_sssp_slots<W>(ctl, decide_sdir<W>(ctl, nextc, nexte), lane);
+  if (lane != 0) return;
+  ctl->dir = dir;
   if (nextc == 0 || (ctl->max_iterations > 0 && l + 1 >= ctl->max_iterations)) {
     ctl->done = 1;
     return;
@@ -2717,7 +2738,7 @@ __device__ void level_end(GroupDev& g) {
 
 template <int W>
 __global__ void k_level_end(GroupDev g) {
-  if (threadIdx.x == 0) level_end<W>(g);
+  level_end<W>(g, static_cast<int>(threadIdx.x));
 }
 
 // Per 32-slot chunk, the out-edges of the next frontier's vertices that carry
@@ -2776,8 +2797,8 @@ __global__ void __launch_bounds__(kBlock) k_chunk_census(GroupDev g, DevGraph G)
 // kStatusLevelCap instead of looping on.
 template <int W>
 __global__ void k_level_end_loop(GroupDev g, cudaGraphConditionalHandle loop, int32_t level_cap) {
+  level_end<W>(g, static_cast<int>(threadIdx.x));
   if (threadIdx.x != 0) return;
-  level_end<W>(g);
   LevelCtl* ctl = g.ctl;
   if (ctl->done == 0 && ctl->level >= level_cap) {
     ctl->status |= kStatusLevelCap;
@@ -2817,12 +2838,15 @@ __global__ void k_seed(GroupDev g, DevGraph G) {
   flush_union<W>(uni, ctl->active[0], lane);
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) {
-    compute_expand<W>(ctl, g.slots, g.Qg, 0);
-    ctl->dir = decide_dir(ctl, ctl->count[0], ctl->edges[0], any_bits<W>(ctl->bfs_bits));
+  if (threadIdx.x < 32) {
+    compute_expand<W>(ctl, g.slots, g.Qg, 0, lane);
+    const int32_t dir = decide_dir(ctl, ctl->count[0], ctl->edges[0], any_bits<W>(ctl->bfs_bits));
     // the sources' level: every slot starts with the group's direction
-    split_sssp_slots<W>(ctl, decide_sdir<W>(ctl, ctl->count[0], ctl->edges[0]));
-    if (ctl->count[0] == 0) ctl->done = 1;
+    split_sssp_slots<W>(ctl, decide_sdir<W>(ctl, ctl->count[0], ctl->edges[0]), lane);
+    if (lane == 0) {
+      ctl->dir = dir;
+      if (ctl->count[0] == 0) ctl->done = 1;
+    }
   }
 }
 

@@ -1,0 +1,8 @@
+// Level kernels of groups with 4 mask words (256 slots), 32-bit offsets.
+#include "levels.cuh"
+
+namespace cgp {
+
+template Dispatch pick_depth<4, int32_t>(int depth, int wk);
+
+}  // namespace cgp

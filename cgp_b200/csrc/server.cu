@@ -105,14 +105,17 @@ __global__ void k_admit(GroupDev g, DevGraph G, const AdmitReq* reqs, int n) {
   }
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0 && ctl->count[par] > 0) {
-    ctl->done = 0;
-    ctl->dir = decide_dir(ctl, ctl->count[par], ctl->edges[par], any_bits<W>(ctl->bfs_bits));
-    if (ctl->chunk_dir) {
+  if (threadIdx.x < 32 && ctl->count[par] > 0) {
+    const int32_t dir = decide_dir(ctl, ctl->count[par], ctl->edges[par], any_bits<W>(ctl->bfs_bits));
+    if (!ctl->chunk_dir) {
+      split_sssp_slots<W>(ctl, decide_sdir<W>(ctl, ctl->count[par], ctl->edges[par]), lane);
+    } else if (lane == 0) {
       ctl->sdir = any_bits<W>(ctl->gsel) ? kDirPull : kDirPush;
       ctl->sscatter = any_bits<W>(ctl->ssel) ? 1 : 0;
-    } else {
-      split_sssp_slots<W>(ctl, decide_sdir<W>(ctl, ctl->count[par], ctl->edges[par]));
+    }
+    if (lane == 0) {
+      ctl->done = 0;
+      ctl->dir = dir;
     }
   }
 }
