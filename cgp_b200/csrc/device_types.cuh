@@ -27,6 +27,7 @@ enum : uint32_t {
   kStatusPlanesExhausted = 1u,  // depth planes too few for the level reached
   kStatusLevelCap = 2u,         // a device-looped traversal reached its level cap
   kStatusQueueOverflow = 4u,    // the heavy frontier queue was full (entry dropped)
+  kStatusBarrier = 8u,          // a grid barrier gave up waiting (the traversal is incomplete)
 };
 
 struct LevelProfile {
@@ -108,6 +109,9 @@ struct LevelCtl {
   unsigned long long prev_pull_edges; // in-edges the previous BFS pull level read
   int32_t prev_dir;                 // BFS direction of the previous level
   int32_t bfs_chunked;              // the BFS pull may run in CTA chunks (chunk table built)
+  uint32_t bar_arrived;             // grid barrier of the fused level loop: blocks arrived,
+  uint32_t bar_release;             // barriers passed,
+  uint32_t bar_abort;               // and nonzero once a wait has given up
   LevelCounters lc;                // counters of the current level
   LevelCounters total;             // sums over all levels
 };

@@ -536,13 +536,9 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
 
 namespace {
 
-// Enqueues `levels` levels either as a replayed CUDA graph or as plain
-// launches; levels < 0: the whole traversal as one device-looped graph (a
-// WHILE conditional node around one level, the condition set by the level's
-// last kernel from the done flag).
-int enqueue_levels(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp_options& o,
-                   cudaStream_t s, int levels, KernelTimer* kt) {
-  Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
+// What one level of the group launches under options o.
+LevelLaunch level_launch(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp_options& o,
+                         const Dispatch& d) {
   LevelLaunch L;
   L.g = group_dev(ws, spec, o.profile_iterations != 0);
   L.G = g->dev_graph(heavy_threshold(o));
@@ -564,6 +560,55 @@ int enqueue_levels(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp
   }
   L.dense_unroll = o.dense_unroll == 2 ? 2 : 1;
   L.chunk_dir = L.spull && sssp_chunk_dir(spec, o);
+  L.kt = nullptr;
+  return L;
+}
+
+// Edges x mask words up to which SSSP levels run fused.
+constexpr int64_t kFusedWork = 1 << 24;
+
+// Whether the group's levels run as the fused loop: the automatic loop form,
+// with the kernel variants the loop holds (the default ones).
+bool fused_loop(const GroupSpec& spec, const cgp_options& o, const LevelLaunch& L) {
+  if (o.level_loop != CGP_LOOP_AUTO || !o.use_cuda_graph || o.bfs_pull_form != 0) return false;
+  if (spec.W > 4 || (spec.has_sssp && L.G.E * spec.W > kFusedWork)) return false;
+  // serving groups on streams of their own: launched levels of different
+  // groups overlap on the device, cooperative launches take all of it in turn
+  if (spec.serving && (o.serve_groups > 1 || o.serve_admission == 2)) return false;
+  if (spec.has_sssp && (L.dense_unroll == 2 || (L.spull && !(L.gvec && L.lchunks)))) return false;
+  return true;
+}
+
+// Levels per launch of the fused loop: enough that the launches between are
+// nothing, few enough that a traversal that cannot converge (negative
+// weights) keeps coming back to the host.
+constexpr int kFusedLevels = 256;
+
+// Enqueues up to `levels` levels as one cooperative launch.
+int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelLaunch& L,
+                  cudaStream_t s, int levels) {
+  const TraverseKernel k = d.traverse(spec.has_bfs, spec.has_sssp);
+  if (k.fn == nullptr || k.per_sm < 1) return 0;
+  const int most = k.per_sm * g->num_sms;
+  const int blocks = static_cast<int>(std::max<int64_t>(
+      1, std::min<int64_t>(most, (g->E + g->V) / 512)));
+  void* args[] = {&L.g, &L.G, &levels};
+  ck(cudaLaunchCooperativeKernel(k.fn, dim3(blocks), dim3(kBlock), args, 0, s), "fused level loop");
+  return 1;
+}
+
+// Enqueues `levels` levels as one launch of the fused loop, as a replayed
+// CUDA graph or as plain launches; levels < 0: the whole traversal as one
+// device-looped graph (a WHILE conditional node around one level, the
+// condition set by the level's last kernel from the done flag).
+int enqueue_levels(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp_options& o,
+                   cudaStream_t s, int levels, KernelTimer* kt) {
+  Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
+  LevelLaunch L = level_launch(g, ws, spec, o, d);
+  if (kt == nullptr && levels > 0 && fused_loop(spec, o, L)) {
+    const int n = enqueue_fused(g, spec, d, L, s, levels);
+    if (n > 0) return n;
+  }
   L.kt = kt;
   if (!o.use_cuda_graph || kt != nullptr) {
     int n = 0;
@@ -635,7 +680,13 @@ int enqueue_levels(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp
 
 void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options& o,
                  cudaStream_t s, GroupRun* out, int max_levels, KernelTimer* kt) {
-  const int per_chunk = kt ? 1 : (o.levels_per_sync > 0 ? o.levels_per_sync : 8);
+  bool fused = false;
+  if (kt == nullptr) {
+    const Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
+    fused = fused_loop(spec, o, level_launch(g, ws, spec, o, d));
+  }
+  const int per_chunk = kt ? 1 : (o.levels_per_sync > 0 ? o.levels_per_sync
+                                                        : (fused ? kFusedLevels : 8));
   int enqueued = 0;
   int chunk = 0;
   LevelCtl* snap = ws->hctl;
@@ -676,6 +727,11 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
       ck(cudaEventSynchronize(ws->ev[chunk & 1]), "sync level");
       out->level_ms.push_back(static_cast<float>(level_sum(kt) - before));
       stop = snap[chunk & 1].done != 0;
+    } else if (fused) {
+      // one launch is a whole traversal as a rule: nothing is kept in flight
+      ck(cudaEventSynchronize(ws->ev[chunk & 1]), "sync levels");
+      const LevelCtl& c = snap[chunk & 1];
+      stop = c.done != 0 || (c.status & kStatusBarrier) != 0;
     } else if (chunk > 0) {
       ck(cudaEventSynchronize(ws->ev[(chunk - 1) & 1]), "sync chunk");
       const LevelCtl& c = snap[(chunk - 1) & 1];
@@ -687,6 +743,8 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
   ck(cudaStreamSynchronize(s), "level loop");
   LevelCtl c;
   ck(cudaMemcpy(&c, ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost), "read ctl");
+  if (c.status & kStatusBarrier)
+    throw ApiError{CGP_ERR_DEVICE, "grid barrier timed out at level " + std::to_string(c.level)};
   if (c.status & kStatusLevelCap)
     throw ApiError{CGP_ERR_DEVICE, "traversal did not converge within " +
                                        std::to_string(c.level) + " levels"};

@@ -357,8 +357,19 @@ struct WarpAppender {
 // Push level, non-heavy frontier vertices: one warp per tile of 32 list
 // entries; vertices with degree > 32 are expanded by the whole warp one at a
 // time, smaller ones edge-balanced across the warp through a warp scan.
+template <int W>
+struct PushSmem {
+  int64_t beg[kWarpsPerBlock][32];
+  int32_t inc[kWarpsPerBlock][32];
+  uint64_t f[kWarpsPerBlock][32][W];
+};
+
 template <int W, typename OT, int DEPTH>
-__global__ void __launch_bounds__(kBlock) k_bfs_push(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void bfs_push_tiles(const GroupDev& g, const DevGraph& G, unsigned bid,
+                                               unsigned nblk, PushSmem<W>& sm) {
+  int64_t (&s_beg)[kWarpsPerBlock][32] = sm.beg;
+  int32_t (&s_inc)[kWarpsPerBlock][32] = sm.inc;
+  uint64_t (&s_f)[kWarpsPerBlock][32][W] = sm.f;
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || ctl->dir != kDirPush) return;
   const LevelView lv = level_view(g);
@@ -370,13 +381,10 @@ __global__ void __launch_bounds__(kBlock) k_bfs_push(GroupDev g, DevGraph G) {
   for (int i = 0; i < W; ++i) sel[i] = ctl->bfs_bits[i] & ctl->expand[i];
   if (!mask_any<W>(sel)) return;
 
-  __shared__ int64_t s_beg[kWarpsPerBlock][32];
-  __shared__ int32_t s_inc[kWarpsPerBlock][32];
-  __shared__ uint64_t s_f[kWarpsPerBlock][32][W];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
-  const unsigned long long gw = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const unsigned long long nw = (static_cast<unsigned long long>(gridDim.x) * blockDim.x) >> 5;
+  const unsigned long long gw = (static_cast<unsigned long long>(bid) * blockDim.x + threadIdx.x) >> 5;
+  const unsigned long long nw = (static_cast<unsigned long long>(nblk) * blockDim.x) >> 5;
   uint64_t uni[W];
 #pragma unroll
   for (int i = 0; i < W; ++i) uni[i] = 0;
@@ -463,6 +471,12 @@ __global__ void __launch_bounds__(kBlock) k_bfs_push(GroupDev g, DevGraph G) {
   warp_add(pairs, &g.ctl->lc.new_pairs, lane);
 }
 
+template <int W, typename OT, int DEPTH>
+__global__ void __launch_bounds__(kBlock) k_bfs_push(GroupDev g, DevGraph G) {
+  __shared__ PushSmem<W> sm;
+  bfs_push_tiles<W, OT, DEPTH>(g, G, blockIdx.x, gridDim.x, sm);
+}
+
 // Heavy frontier queue.  At the start of a push level the frontier list is
 // scanned once and every vertex of degree > heavy_degree is queued with its
 // range of kHeavyChunk-edge chunks; one 64-bit atomicAdd hands out both the
@@ -473,14 +487,15 @@ __global__ void __launch_bounds__(kBlock) k_bfs_push(GroupDev g, DevGraph G) {
 constexpr int kQueueShift = 40;
 
 template <typename OT>
-__global__ void __launch_bounds__(kBlock) k_heavy_queue(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void heavy_queue_scan(const GroupDev& g, const DevGraph& G,
+                                                 unsigned bid, unsigned nblk) {
   LevelCtl* ctl = g.ctl;
   if (ctl->done || (ctl->dir != kDirPush && !ctl->sscatter)) return;
   const LevelView lv = level_view(g);
   const unsigned long long n = ctl->count[lv.par];
   const int64_t light = push_light_limit(g, G, n, ctl->edges[lv.par]);
-  for (unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-       i < n; i += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
+  for (unsigned long long i = static_cast<unsigned long long>(bid) * blockDim.x + threadIdx.x;
+       i < n; i += static_cast<unsigned long long>(nblk) * blockDim.x) {
     const int32_t u = lv.list[i];
     const int64_t deg = row_at<OT>(G.row, static_cast<int64_t>(u) + 1) - row_at<OT>(G.row, u);
     if (deg <= light) continue;
@@ -496,6 +511,11 @@ __global__ void __launch_bounds__(kBlock) k_heavy_queue(GroupDev g, DevGraph G) 
   }
 }
 
+template <typename OT>
+__global__ void __launch_bounds__(kBlock) k_heavy_queue(GroupDev g, DevGraph G) {
+  heavy_queue_scan<OT>(g, G, blockIdx.x, gridDim.x);
+}
+
 // Queue slot of chunk c (the last slot whose first chunk is <= c).
 __device__ __forceinline__ int heavy_queue_slot(const GroupDev& g, int nq, int64_t c) {
   int lo = 0, hi = nq - 1;
@@ -509,8 +529,14 @@ __device__ __forceinline__ int heavy_queue_slot(const GroupDev& g, int nq, int64
 
 // Push level, heavy frontier vertices: the static heavy list is cut into
 // kHeavyChunk-edge work items spread over all CTAs.
+struct HeavySlotSmem {
+  int32_t h;
+};
+
 template <int W, typename OT, int DEPTH>
-__global__ void __launch_bounds__(kBlock) k_bfs_push_heavy(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void bfs_push_chunks(const GroupDev& g, const DevGraph& G, unsigned bid,
+                                                unsigned nblk, HeavySlotSmem& sm) {
+  int32_t& s_h = sm.h;
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || ctl->dir != kDirPush) return;
   const unsigned long long hq = ctl->hq_packed;
@@ -520,13 +546,12 @@ __global__ void __launch_bounds__(kBlock) k_bfs_push_heavy(GroupDev g, DevGraph 
   if (nq == 0) return;
   const LevelView lv = level_view(g);
   WarpAppender ap;
-  __shared__ int32_t s_h;
   const int lane = threadIdx.x & 31;
   uint64_t uni[W];
 #pragma unroll
   for (int i = 0; i < W; ++i) uni[i] = 0;
   unsigned long long pairs = 0;
-  for (int64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+  for (int64_t c = bid; c < nchunks; c += nblk) {
     if (threadIdx.x == 0) s_h = heavy_queue_slot(g, nq, c);
     __syncthreads();
     const int h = s_h;
@@ -557,6 +582,12 @@ __global__ void __launch_bounds__(kBlock) k_bfs_push_heavy(GroupDev g, DevGraph 
   warp_add(pairs, &g.ctl->lc.new_pairs, lane);
 }
 
+template <int W, typename OT, int DEPTH>
+__global__ void __launch_bounds__(kBlock) k_bfs_push_heavy(GroupDev g, DevGraph G) {
+  __shared__ HeavySlotSmem sm;
+  bfs_push_chunks<W, OT, DEPTH>(g, G, blockIdx.x, gridDim.x, sm);
+}
+
 // Which light-vertex pull form a BFS pull level uses.  The chunked form
 // (k_bfs_pull_chunked) keeps 32 in-edges in flight per warp but checks early
 // exit once per 32-edge batch; the lane-per-vertex form (k_bfs_pull) stops a
@@ -573,7 +604,8 @@ __device__ __forceinline__ bool bfs_pull_chunked_level(const LevelCtl* ctl, int6
 // (exactly the vertices of that frontier's list).  Push levels only: a pull
 // level rewrites every vertex's next mask.
 template <int W>
-__global__ void __launch_bounds__(kBlock) k_clear_next(GroupDev g, int64_t E) {
+__device__ __forceinline__ void clear_next(const GroupDev& g, int64_t E, unsigned bid,
+                                           unsigned nblk) {
   const LevelCtl* ctl = g.ctl;
   if (ctl->done) return;
   // a lane-per-vertex pull level in vertex order rewrites every vertex's next
@@ -583,13 +615,18 @@ __global__ void __launch_bounds__(kBlock) k_clear_next(GroupDev g, int64_t E) {
   const LevelView lv = level_view(g);
   const unsigned long long n = ctl->prev_count;
   const int32_t* plist = lv.nlist;  // list of the previous frontier
-  for (unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-       i < n; i += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
+  for (unsigned long long i = static_cast<unsigned long long>(bid) * blockDim.x + threadIdx.x;
+       i < n; i += static_cast<unsigned long long>(nblk) * blockDim.x) {
     uint64_t z[W];
 #pragma unroll
     for (int k = 0; k < W; ++k) z[k] = 0;
     store_mask<W>(lv.fnext + static_cast<size_t>(plist[i]) * W, z);
   }
+}
+
+template <int W>
+__global__ void __launch_bounds__(kBlock) k_clear_next(GroupDev g, int64_t E) {
+  clear_next<W>(g, E, blockIdx.x, gridDim.x);
 }
 
 // --------------------------------------------------------------- BFS pull
@@ -634,7 +671,8 @@ __device__ __forceinline__ bool bfs_pull_uses_summary(const GroupDev& g, const L
 // lanes of a warp walk lists of about the same length (the next masks of the
 // vertices left out are zeroed by k_clear_next).
 template <int W, typename OT, int DEPTH>
-__global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 1)) k_bfs_pull(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void bfs_pull_tiles(const GroupDev& g, const DevGraph& G, unsigned bid,
+                                               unsigned nblk) {
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || ctl->dir != kDirPull) return;
   if (G.n_plight_chunks > 0 && bfs_pull_chunked_level(ctl, G.E)) return;
@@ -644,8 +682,8 @@ __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 1)) k_bfs_pull(GroupDev 
   for (int i = 0; i < W; ++i)
     act[i] = ctl->active[lv.par][i] & ctl->bfs_bits[i] & ctl->expand[i];
   const int lane = threadIdx.x & 31;
-  const unsigned long long gw = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const unsigned long long nwarps = (static_cast<unsigned long long>(gridDim.x) * blockDim.x) >> 5;
+  const unsigned long long gw = (static_cast<unsigned long long>(bid) * blockDim.x + threadIdx.x) >> 5;
+  const unsigned long long nwarps = (static_cast<unsigned long long>(nblk) * blockDim.x) >> 5;
   const unsigned long long V = static_cast<unsigned long long>(G.V);
   const bool use_sum = bfs_pull_uses_summary(g, ctl, lv, G.V);
   uint64_t uni[W];
@@ -763,6 +801,11 @@ __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 1)) k_bfs_pull(GroupDev 
   warp_add(pairs, &g.ctl->lc.new_pairs, lane);
   warp_add(pverts, &g.ctl->lc.pull_vertices, lane);
   warp_add(pedges, &g.ctl->lc.pull_edges, lane);
+}
+
+template <int W, typename OT, int DEPTH>
+__global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 1)) k_bfs_pull(GroupDev g, DevGraph G) {
+  bfs_pull_tiles<W, OT, DEPTH>(g, G, blockIdx.x, gridDim.x);
 }
 
 // Pull level (bottom-up), light vertices in CTA chunks of the pull CSR's light
@@ -921,7 +964,8 @@ __global__ void __launch_bounds__(kBlock) k_bfs_pull_chunked(GroupDev g, DevGrap
 // their own.  Every listed vertex's next mask is written (zero when nothing
 // is new), as the tile kernel does for its vertices.
 template <int W, typename OT, int DEPTH>
-__global__ void __launch_bounds__(kBlock, 3) k_bfs_pull_mid(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void bfs_pull_mid(const GroupDev& g, const DevGraph& G, unsigned bid,
+                                             unsigned nblk) {
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || ctl->dir != kDirPull || G.n_pmid == 0) return;
   if (G.n_plight_chunks > 0 && bfs_pull_chunked_level(ctl, G.E)) return;
@@ -932,8 +976,8 @@ __global__ void __launch_bounds__(kBlock, 3) k_bfs_pull_mid(GroupDev g, DevGraph
     act[i] = ctl->active[lv.par][i] & ctl->bfs_bits[i] & ctl->expand[i];
   const bool use_sum = bfs_pull_uses_summary(g, ctl, lv, G.V);
   const int lane = threadIdx.x & 31;
-  const long long gw = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+  const long long gw = (static_cast<long long>(bid) * blockDim.x + threadIdx.x) >> 5;
+  const long long nwarps = (static_cast<long long>(nblk) * blockDim.x) >> 5;
   WarpAppender ap;
   uint64_t uni[W];
 #pragma unroll
@@ -1000,18 +1044,30 @@ __global__ void __launch_bounds__(kBlock, 3) k_bfs_pull_mid(GroupDev g, DevGraph
   warp_add(pedges, &g.ctl->lc.pull_edges, lane);
 }
 
+template <int W, typename OT, int DEPTH>
+__global__ void __launch_bounds__(kBlock, 3) k_bfs_pull_mid(GroupDev g, DevGraph G) {
+  bfs_pull_mid<W, OT, DEPTH>(g, G, blockIdx.x, gridDim.x);
+}
+
 // Pull level, heavy vertices: chunks of their in-edges spread over CTAs; each
 // CTA ORs its chunk into hacc[h] (skipping chunks once hacc covers the need).
+template <int W>
+struct PullHeavySmem {
+  int skip;
+  uint64_t red[kWarpsPerBlock][W];
+};
+
 template <int W, typename OT>
-__global__ void __launch_bounds__(kBlock) k_bfs_pull_heavy(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void bfs_pull_chunks(const GroupDev& g, const DevGraph& G, unsigned bid,
+                                                unsigned nblk, PullHeavySmem<W>& sm) {
+  int& s_skip = sm.skip;
+  uint64_t (&s_red)[kWarpsPerBlock][W] = sm.red;
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || ctl->dir != kDirPull || G.n_pheavy == 0) return;
   const LevelView lv = level_view(g);
-  __shared__ int s_skip;
-  __shared__ uint64_t s_red[kWarpsPerBlock][W];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
-  for (int64_t c = blockIdx.x; c < G.pheavy_chunks; c += gridDim.x) {
+  for (int64_t c = bid; c < G.pheavy_chunks; c += nblk) {
     __syncthreads();  // the previous chunk's s_skip is read
     const int h = G.pheavy_ch[c];
     const int32_t v = G.pheavy[h];
@@ -1063,9 +1119,16 @@ __global__ void __launch_bounds__(kBlock) k_bfs_pull_heavy(GroupDev g, DevGraph 
   }
 }
 
+template <int W, typename OT>
+__global__ void __launch_bounds__(kBlock) k_bfs_pull_heavy(GroupDev g, DevGraph G) {
+  __shared__ PullHeavySmem<W> sm;
+  bfs_pull_chunks<W, OT>(g, G, blockIdx.x, gridDim.x, sm);
+}
+
 // Commits the heavy vertices of a pull level and resets their accumulators.
 template <int W, typename OT, int DEPTH>
-__global__ void __launch_bounds__(kBlock) k_bfs_pull_heavy_commit(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void bfs_pull_heavy_commit(const GroupDev& g, const DevGraph& G,
+                                                      unsigned bid, unsigned nblk) {
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || ctl->dir != kDirPull || G.n_pheavy == 0) return;
   const LevelView lv = level_view(g);
@@ -1074,8 +1137,8 @@ __global__ void __launch_bounds__(kBlock) k_bfs_pull_heavy_commit(GroupDev g, De
 #pragma unroll
   for (int i = 0; i < W; ++i) uni[i] = 0;
   unsigned long long pairs = 0, pverts = 0;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31);
+  const int64_t stride = static_cast<int64_t>(nblk) * blockDim.x;
+  for (int64_t base = static_cast<int64_t>(bid) * blockDim.x + (threadIdx.x & ~31);
        base < G.n_pheavy; base += stride) {
     const int64_t h = base + lane;
     bool app = false;
@@ -1106,6 +1169,11 @@ __global__ void __launch_bounds__(kBlock) k_bfs_pull_heavy_commit(GroupDev g, De
   flush_union<W>(uni, lv.nactive, lane);
   warp_add(pairs, &g.ctl->lc.new_pairs, lane);
   warp_add(pverts, &g.ctl->lc.pull_vertices, lane);
+}
+
+template <int W, typename OT, int DEPTH>
+__global__ void __launch_bounds__(kBlock) k_bfs_pull_heavy_commit(GroupDev g, DevGraph G) {
+  bfs_pull_heavy_commit<W, OT, DEPTH>(g, G, blockIdx.x, gridDim.x);
 }
 
 // -------------------------------------------------------------- SSSP push
@@ -1285,15 +1353,16 @@ __device__ __forceinline__ void sssp_dense_edges(const GroupDev& g, const DevGra
 // Dense SSSP vertices of a level, one warp per vertex (the tile kernel
 // queued them), so that this loop gets a register budget of its own.
 template <int W, typename OT, int WK, int U>
-__global__ void __launch_bounds__(kBlock, (U == 1 ? 4 : 3)) k_sssp_dense(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void sssp_dense_vertices(const GroupDev& g, const DevGraph& G,
+                                                    unsigned bid, unsigned nblk) {
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || !ctl->sscatter) return;
   const LevelView lv = level_view(g);
   WarpAppender ap;
   const unsigned long long n = ctl->dense_count;
   const int lane = threadIdx.x & 31;
-  const unsigned long long gw = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const unsigned long long nwarps = (static_cast<unsigned long long>(gridDim.x) * blockDim.x) >> 5;
+  const unsigned long long gw = (static_cast<unsigned long long>(bid) * blockDim.x + threadIdx.x) >> 5;
+  const unsigned long long nwarps = (static_cast<unsigned long long>(nblk) * blockDim.x) >> 5;
   uint64_t uni[W];
 #pragma unroll
   for (int i = 0; i < W; ++i) uni[i] = 0;
@@ -1313,11 +1382,31 @@ __global__ void __launch_bounds__(kBlock, (U == 1 ? 4 : 3)) k_sssp_dense(GroupDe
   warp_add(improved, &g.ctl->lc.improved, lane);
 }
 
+template <int W, typename OT, int WK, int U>
+__global__ void __launch_bounds__(kBlock, (U == 1 ? 4 : 3)) k_sssp_dense(GroupDev g, DevGraph G) {
+  sssp_dense_vertices<W, OT, WK, U>(g, G, blockIdx.x, gridDim.x);
+}
+
 // SSSP push over the frontier list: the (edge, active query) pairs of a tile
 // of 32 vertices are flattened and spread evenly over the warp's lanes, so a
 // vertex with k active queries and degree d costs k*d/32 warp steps.
+template <int W>
+struct SsspPushSmem {
+  int64_t beg[kWarpsPerBlock][32];
+  long long inc[kWarpsPerBlock][32];
+  int32_t k[kWarpsPerBlock][32];
+  int32_t u[kWarpsPerBlock][32];
+  uint64_t b[kWarpsPerBlock][32][W];
+};
+
 template <int W, typename OT, int WK>
-__global__ void __launch_bounds__(kBlock) k_sssp_push(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void sssp_push_tiles(const GroupDev& g, const DevGraph& G, unsigned bid,
+                                                unsigned nblk, SsspPushSmem<W>& sm) {
+  int64_t (&s_beg)[kWarpsPerBlock][32] = sm.beg;
+  long long (&s_inc)[kWarpsPerBlock][32] = sm.inc;
+  int32_t (&s_k)[kWarpsPerBlock][32] = sm.k;
+  int32_t (&s_u)[kWarpsPerBlock][32] = sm.u;
+  uint64_t (&s_b)[kWarpsPerBlock][32][W] = sm.b;
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || !ctl->sscatter) return;
   const LevelView lv = level_view(g);
@@ -1328,15 +1417,10 @@ __global__ void __launch_bounds__(kBlock) k_sssp_push(GroupDev g, DevGraph G) {
 #pragma unroll
   for (int i = 0; i < W; ++i) sel[i] = ctl->ssel[i];
   if (!mask_any<W>(sel)) return;
-  __shared__ int64_t s_beg[kWarpsPerBlock][32];
-  __shared__ long long s_inc[kWarpsPerBlock][32];
-  __shared__ int32_t s_k[kWarpsPerBlock][32];
-  __shared__ int32_t s_u[kWarpsPerBlock][32];
-  __shared__ uint64_t s_b[kWarpsPerBlock][32][W];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
-  const unsigned long long gw = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const unsigned long long nwarps = (static_cast<unsigned long long>(gridDim.x) * blockDim.x) >> 5;
+  const unsigned long long gw = (static_cast<unsigned long long>(bid) * blockDim.x + threadIdx.x) >> 5;
+  const unsigned long long nwarps = (static_cast<unsigned long long>(nblk) * blockDim.x) >> 5;
   uint64_t uni[W];
 #pragma unroll
   for (int i = 0; i < W; ++i) uni[i] = 0;
@@ -1440,10 +1524,30 @@ __global__ void __launch_bounds__(kBlock) k_sssp_push(GroupDev g, DevGraph G) {
   warp_add(sactive, &g.ctl->lc.sssp_active, lane);
 }
 
+template <int W, typename OT, int WK>
+__global__ void __launch_bounds__(kBlock) k_sssp_push(GroupDev g, DevGraph G) {
+  __shared__ SsspPushSmem<W> sm;
+  sssp_push_tiles<W, OT, WK>(g, G, blockIdx.x, gridDim.x, sm);
+}
+
 // SSSP push for heavy frontier vertices: per chunk of kHeavyChunk edges the
 // CTA lists the active query ids once and walks (edge, query) pairs.
+template <int W>
+struct SsspHeavySmem {
+  int32_t h;
+  int32_t k;
+  int16_t q[kMaxW * 64];
+  int32_t wpre[W + 1];
+};
+
 template <int W, typename OT, int WK>
-__global__ void __launch_bounds__(kBlock) k_sssp_push_heavy(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void sssp_push_chunks(const GroupDev& g, const DevGraph& G,
+                                                 unsigned bid, unsigned nblk,
+                                                 SsspHeavySmem<W>& sm) {
+  int32_t& s_h = sm.h;
+  int32_t& s_k = sm.k;
+  int16_t (&s_q)[kMaxW * 64] = sm.q;
+  int32_t (&s_wpre)[W + 1] = sm.wpre;
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || !ctl->sscatter) return;
   const unsigned long long hq = ctl->hq_packed;
@@ -1453,16 +1557,12 @@ __global__ void __launch_bounds__(kBlock) k_sssp_push_heavy(GroupDev g, DevGraph
   if (nq == 0) return;
   const LevelView lv = level_view(g);
   WarpAppender ap;
-  __shared__ int32_t s_h;
-  __shared__ int32_t s_k;
-  __shared__ int16_t s_q[kMaxW * 64];
-  __shared__ int32_t s_wpre[W + 1];
   const int lane = threadIdx.x & 31;
   uint64_t uni[W];
 #pragma unroll
   for (int i = 0; i < W; ++i) uni[i] = 0;
   unsigned long long improved = 0;
-  for (int64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+  for (int64_t c = bid; c < nchunks; c += nblk) {
     if (threadIdx.x == 0) s_h = heavy_queue_slot(g, nq, c);
     __syncthreads();
     const int h = s_h;
@@ -1552,6 +1652,12 @@ __global__ void __launch_bounds__(kBlock) k_sssp_push_heavy(GroupDev g, DevGraph
   ap.flush<OT>(G, lv, lane);
   flush_union<W>(uni, lv.nactive, lane);
   warp_add(improved, &g.ctl->lc.improved, lane);
+}
+
+template <int W, typename OT, int WK>
+__global__ void __launch_bounds__(kBlock) k_sssp_push_heavy(GroupDev g, DevGraph G) {
+  __shared__ SsspHeavySmem<W> sm;
+  sssp_push_chunks<W, OT, WK>(g, G, blockIdx.x, gridDim.x, sm);
 }
 
 
@@ -1938,7 +2044,8 @@ __device__ __forceinline__ int gather_screen_qs(const GroupDev& g, const LevelCt
 // (out-degree x gathering chunks with a frontier bit).  Words of vertices
 // outside the frontier keep an older level's stamp and read as empty.
 template <int W, typename OT>
-__global__ void __launch_bounds__(kBlock) k_frontier_summary(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void frontier_summary(const GroupDev& g, const DevGraph& G,
+                                                 unsigned bid, unsigned nblk) {
   LevelCtl* ctl = g.ctl;
   if (ctl->done) return;
   const LevelView lv = level_view(g);
@@ -1949,8 +2056,8 @@ __global__ void __launch_bounds__(kBlock) k_frontier_summary(GroupDev g, DevGrap
   const uint32_t gch = gather_chunks<W>(ctl);
   const int lane = threadIdx.x & 31;
   unsigned long long live = 0;
-  const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
-  for (unsigned long long i0 = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31);
+  const unsigned long long stride = static_cast<unsigned long long>(nblk) * blockDim.x;
+  for (unsigned long long i0 = static_cast<unsigned long long>(bid) * blockDim.x + (threadIdx.x & ~31);
        i0 < n; i0 += stride) {
     const unsigned long long i = i0 + lane;
     if (i < n) {
@@ -1963,6 +2070,11 @@ __global__ void __launch_bounds__(kBlock) k_frontier_summary(GroupDev g, DevGrap
     }
   }
   if (sssp) warp_add(live, &ctl->lc.live_chunks, lane);
+}
+
+template <int W, typename OT>
+__global__ void __launch_bounds__(kBlock) k_frontier_summary(GroupDev g, DevGraph G) {
+  frontier_summary<W, OT>(g, G, blockIdx.x, gridDim.x);
 }
 
 // Whether the lane reads part r of a source row whose 32-slot chunk bits are
@@ -2218,8 +2330,19 @@ __device__ __forceinline__ int chunk_edge_owner(int my_pre, int f0, int lane) {
 // are gathered in slices of W words: blockIdx.y is the slice, each CTA owns
 // its vertices' slice of the row, and the frontier append is claimed with an
 // atomic on the stamp (the slices of a vertex commit in different CTAs).
-template <int W, typename OT, int WK, int WF = W>
-__global__ void __launch_bounds__(kBlock, 3) k_sssp_pull_chunked(GroupDev g, DevGraph G) {
+template <int W>
+struct GatherChunkSmem {
+  alignas(16) uint32_t best[kLightChunkVerts * 64 * W];
+  int4 stage[kWarpsPerBlock][32];
+  int32_t v[kLightChunkVerts];
+  int64_t beg[kLightChunkVerts];
+  int32_t pre[kLightChunkVerts + 1];
+};
+
+template <int W, typename OT, int WK, int WF>
+__device__ __forceinline__ void sssp_pull_light_chunks(const GroupDev& g, const DevGraph& G,
+                                                       unsigned bid, unsigned nblk, int sl,
+                                                       GatherChunkSmem<W>& sm) {
   static_assert(W <= 4, "chunked gather holds 32 rows of at most 256 slots");
   static_assert(WF % W == 0, "a group is a whole number of slices");
   using GV = GatherVec<W>;
@@ -2230,15 +2353,14 @@ __global__ void __launch_bounds__(kBlock, 3) k_sssp_pull_chunked(GroupDev g, Dev
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || ctl->sdir != kDirPull || G.n_plight_chunks == 0) return;
   const LevelView lv = level_view(g);
-  __shared__ __align__(16) uint32_t s_best[kLightChunkVerts * R];
-  __shared__ int4 s_stage[kWarpsPerBlock][32];
-  __shared__ int32_t s_v[kLightChunkVerts];
-  __shared__ int64_t s_beg[kLightChunkVerts];
-  __shared__ int32_t s_pre[kLightChunkVerts + 1];
+  uint32_t (&s_best)[kLightChunkVerts * 64 * W] = sm.best;
+  int4 (&s_stage)[kWarpsPerBlock][32] = sm.stage;
+  int32_t (&s_v)[kLightChunkVerts] = sm.v;
+  int64_t (&s_beg)[kLightChunkVerts] = sm.beg;
+  int32_t (&s_pre)[kLightChunkVerts + 1] = sm.pre;
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
-  const int sl = WF > W ? static_cast<int>(blockIdx.y) : 0;  // slice of W words
-  const int s0 = sl * 64 * W;                                  // its first slot
+  const int s0 = sl * 64 * W;  // first slot of the slice of W words
   const uint64_t* sb = ctl->gsel + sl * W;
   uint32_t pmask, smask;
   gather_vec_masks<W>(sb, g.Qg - s0, lane, &pmask, &smask);
@@ -2257,7 +2379,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_sssp_pull_chunked(GroupDev g, Dev
   uint32_t uacc = 0;
   unsigned long long improved = 0, pairs = 0;
   unsigned scanned = 0, verts = 0;
-  for (int c = blockIdx.x; c < G.n_plight_chunks; c += gridDim.x) {
+  for (int c = bid; c < G.n_plight_chunks; c += nblk) {
     const int cs = G.plight_chunk_start[c];
     const int nv = G.plight_chunk_start[c + 1] - cs;
     if (wib == 0) {
@@ -2456,23 +2578,39 @@ __global__ void __launch_bounds__(kBlock, 3) k_sssp_pull_chunked(GroupDev g, Dev
   warp_add(verts, &g.ctl->lc.spull_vertices, lane);
 }
 
+template <int W, typename OT, int WK, int WF = W>
+__global__ void __launch_bounds__(kBlock, 3) k_sssp_pull_chunked(GroupDev g, DevGraph G) {
+  __shared__ GatherChunkSmem<W> sm;
+  sssp_pull_light_chunks<W, OT, WK, WF>(g, G, blockIdx.x, gridDim.x,
+                                        WF > W ? static_cast<int>(blockIdx.y) : 0, sm);
+}
+
 // Gather level (vectorised), heavy vertices: CTA per 2048-edge chunk, warps
 // min-reduce their slices into shared memory, one atomicMin per slot.
 // kMode 0: every gather level, whole source rows; 1: only levels that read
 // whole rows (dense entries); 2: only screened levels (sparse entries), with
-// the source rows' 32-slot chunks without frontier bits skipped.  Modes 1 and 2
+// the source rows' 32-slot chunks without frontier bits skipped; 3: every
+// gather level, skipping as 2 does on screened ones.  Modes 1 and 2
 // are launched together (groups of <= 256 slots) so that each level runs the
 // variant whose register budget suits it.
+template <int W>
+struct GatherHeavySmem {
+  alignas(16) uint32_t best[64 * W];
+  int4 stage[kWarpsPerBlock][32];
+};
+
 template <int W, typename OT, int WK, int kMode>
-__global__ void __launch_bounds__(kBlock) k_sssp_pull_heavy_vec(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void sssp_pull_heavy_chunks(const GroupDev& g, const DevGraph& G,
+                                                       unsigned bid, unsigned nblk,
+                                                       GatherHeavySmem<W>& sm) {
+  uint32_t (&s_best)[64 * W] = sm.best;
+  int4 (&s_stage)[kWarpsPerBlock][32] = sm.stage;
   using GV = GatherVec<W>;
   constexpr int E = GV::kElem;
   constexpr int C = 2 * W;
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || ctl->sdir != kDirPull || G.n_pheavy == 0) return;
   const LevelView lv = level_view(g);
-  __shared__ uint32_t s_best[C * 32];
-  __shared__ int4 s_stage[kWarpsPerBlock][32];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const uint64_t* sb = ctl->gsel;
@@ -2489,9 +2627,9 @@ __global__ void __launch_bounds__(kBlock) k_sssp_pull_heavy_vec(GroupDev g, DevG
   unsigned long long improved = 0, pairs = 0;
   unsigned scanned = 0;
   // every heavy vertex is gathered once per launch (all its chunks)
-  if (blockIdx.x == 0 && threadIdx.x == 0)
+  if (bid == 0 && threadIdx.x == 0)
     atomicAdd(&g.ctl->lc.spull_vertices, static_cast<unsigned long long>(G.n_pheavy));
-  for (int64_t ch = blockIdx.x; ch < G.pheavy_chunks; ch += gridDim.x) {
+  for (int64_t ch = bid; ch < G.pheavy_chunks; ch += nblk) {
     // the chunk's vertex and edge range: independent loads, no search
     const int32_t v = G.pheavy[G.pheavy_ch[ch]];
     const int64_t cb = G.pheavy_cb[ch];
@@ -2504,7 +2642,7 @@ __global__ void __launch_bounds__(kBlock) k_sssp_pull_heavy_vec(GroupDev g, DevG
     uint32_t best[GV::kSlots];
 #pragma unroll
     for (int j = 0; j < GV::kSlots; ++j) best[j] = 0xffffffffu;
-    gather_edges_vec<W, WK, kMode == 2>(g, G, lv, sb, pmask, wb, we, lane, s_stage[wib], best,
+    gather_edges_vec<W, WK, (kMode >= 2)>(g, G, lv, sb, pmask, wb, we, lane, s_stage[wib], best,
                                         pairs, scanned, screen_qs, gch);
 #pragma unroll
     for (int j = 0; j < GV::kSlots; ++j) {
@@ -2543,6 +2681,12 @@ __global__ void __launch_bounds__(kBlock) k_sssp_pull_heavy_vec(GroupDev g, DevG
   warp_add(improved, &g.ctl->lc.improved, lane);
   warp_add(pairs, &g.ctl->lc.sssp_pairs, lane);
   warp_add(scanned, &g.ctl->lc.spull_edges, lane);
+}
+
+template <int W, typename OT, int WK, int kMode>
+__global__ void __launch_bounds__(kBlock) k_sssp_pull_heavy_vec(GroupDev g, DevGraph G) {
+  __shared__ GatherHeavySmem<W> sm;
+  sssp_pull_heavy_chunks<W, OT, WK, kMode>(g, G, blockIdx.x, gridDim.x, sm);
 }
 
 // --------------------------------------------------------- level control
@@ -2746,7 +2890,8 @@ __global__ void k_level_end(GroupDev g) {
 // after the level's kernels, before its level end: each lane takes a vertex
 // of the next frontier list, the warp sums its chunks, lane 0 adds them.
 template <int W, typename OT>
-__global__ void __launch_bounds__(kBlock) k_chunk_census(GroupDev g, DevGraph G) {
+__device__ __forceinline__ void chunk_census(const GroupDev& g, const DevGraph& G, unsigned bid,
+                                             unsigned nblk) {
   LevelCtl* ctl = g.ctl;
   if (ctl->done || !ctl->chunk_dir) return;
   const LevelView lv = level_view(g);
@@ -2755,8 +2900,8 @@ __global__ void __launch_bounds__(kBlock) k_chunk_census(GroupDev g, DevGraph G)
   unsigned long long acc[2 * W], pacc[2 * W];
 #pragma unroll
   for (int c = 0; c < 2 * W; ++c) acc[c] = pacc[c] = 0;
-  const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
-  for (unsigned long long i0 = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31);
+  const unsigned long long stride = static_cast<unsigned long long>(nblk) * blockDim.x;
+  for (unsigned long long i0 = static_cast<unsigned long long>(bid) * blockDim.x + (threadIdx.x & ~31);
        i0 < n; i0 += stride) {
     const unsigned long long i = i0 + lane;
     if (i < n) {
@@ -2790,6 +2935,11 @@ __global__ void __launch_bounds__(kBlock) k_chunk_census(GroupDev g, DevGraph G)
   }
 }
 
+template <int W, typename OT>
+__global__ void __launch_bounds__(kBlock) k_chunk_census(GroupDev g, DevGraph G) {
+  chunk_census<W, OT>(g, G, blockIdx.x, gridDim.x);
+}
+
 // Level end inside a device-looped CUDA graph (a WHILE conditional node whose
 // body is one level): sets the loop condition from the done flag, so the
 // whole traversal runs without the host.  A traversal that is still running
@@ -2805,6 +2955,193 @@ __global__ void k_level_end_loop(GroupDev g, cudaGraphConditionalHandle loop, in
     ctl->done = 3;
   }
   cudaGraphSetConditional(loop, ctl->done == 0 ? 1u : 0u);
+}
+
+// ------------------------------------------------------- fused level loop
+// Barrier over all blocks of a cooperative launch.  The last block to arrive
+// runs `last(lane)` with its first warp before it lets the others go, so the
+// end of a level costs no barrier of its own.  A wait gives up after
+// kBarrierLimitNs (the other blocks are co-resident, so this means the device
+// is not running them), raises kStatusBarrier and tells every block to leave:
+// wait() then returns false in all of them.
+constexpr unsigned long long kBarrierLimitNs = 20ULL * 1000 * 1000 * 1000;
+
+__device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void store_release(unsigned* p, unsigned v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+struct GridBarrier {
+  LevelCtl* ctl;
+  unsigned nblk;
+  unsigned epoch;  // barriers passed
+
+  // Every block reads the epoch before it first arrives, so none can miss a
+  // release of this launch.
+  __device__ __forceinline__ GridBarrier(LevelCtl* c, unsigned n)
+      : ctl(c), nblk(n), epoch(load_acquire(&c->bar_release)) {}
+
+  template <typename F>
+  __device__ __forceinline__ bool wait(F&& last) {
+    __shared__ int s_ok;
+    ++epoch;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const int lane = static_cast<int>(threadIdx.x);
+      unsigned before = 0;
+      if (lane == 0) {
+        __threadfence();
+        before = atomicAdd(&ctl->bar_arrived, 1u);
+      }
+      before = __shfl_sync(kFull, before, 0);
+      bool ok = true;
+      if (before == nblk - 1) {
+        __threadfence();  // every lane: the other blocks' writes of the phase
+        last(lane);
+        if (lane == 0) ctl->bar_arrived = 0;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) store_release(&ctl->bar_release, epoch);
+      } else if (lane == 0) {
+        unsigned long long t0 = 0;
+        for (unsigned spins = 0; load_acquire(&ctl->bar_release) != epoch; ++spins) {
+          if ((spins & 255u) != 255u) continue;
+          if (load_acquire(&ctl->bar_abort) != 0) {
+            ok = false;
+            break;
+          }
+          const unsigned long long t = global_ns();
+          if (t0 == 0) t0 = t;
+          if (t - t0 > kBarrierLimitNs) {
+            atomicOr(&ctl->status, kStatusBarrier);
+            __threadfence();
+            store_release(&ctl->bar_abort, 1u);
+            ok = false;
+            break;
+          }
+        }
+      }
+      if (lane == 0) s_ok = ok ? 1 : 0;
+      __threadfence();
+    }
+    __syncthreads();
+    return s_ok != 0;
+  }
+
+  __device__ __forceinline__ bool wait() {
+    return wait([](int) {});
+  }
+};
+
+template <int W, bool kBfs, bool kSssp>
+union TraverseSmem {
+  PushSmem<kBfs ? W : 1> push;
+  HeavySlotSmem slot;
+  PullHeavySmem<kBfs ? W : 1> pull_heavy;
+  SsspPushSmem<kSssp ? W : 1> sssp_push;
+  SsspHeavySmem<kSssp ? W : 1> sssp_heavy;
+  GatherHeavySmem<kSssp ? W : 1> gather_heavy;
+  GatherChunkSmem<kSssp ? (W < 4 ? W : 4) : 1> gather_light;
+};
+
+// Up to `levels` whole levels in one cooperative launch: the phases that are
+// kernels of their own in the launched form (see enqueue_level_t) run one
+// after another with a grid barrier wherever one reads what another wrote,
+// and the level end runs in the last block to reach the level's last barrier.
+// A launched level is 10 to 16 dependent kernels, most of which find nothing
+// to do; with small graphs and in the first and last levels of deep ones
+// their launches are the level's whole time.
+template <int W, typename OT, int DEPTH, int WK, bool kBfs, bool kSssp>
+__global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev g, DevGraph G,
+                                                                      int levels) {
+  __shared__ TraverseSmem<W, kBfs, kSssp> sm;
+  const unsigned bid = blockIdx.x, nblk = gridDim.x;
+  LevelCtl* ctl = g.ctl;
+  GridBarrier bar(ctl, nblk);
+  for (int l = 0; l < levels; ++l) {
+    if (ctl->done) return;
+    const bool bfs_pull = kBfs && ctl->dir == kDirPull;
+    const bool gather = kSssp && ctl->sdir == kDirPull;
+    const bool scatter = kSssp && ctl->sscatter != 0;
+    bool summary = gather;
+    if constexpr (kBfs) summary |= bfs_pull_uses_summary(g, ctl, level_view(g), G.V);
+    // what the level's phases read or add to: a pull over whole masks alone
+    // rewrites every next mask and needs nothing prepared
+    if (!bfs_pull || summary || scatter) {
+      clear_next<W>(g, G.E, bid, nblk);
+      if (summary) frontier_summary<W, OT>(g, G, bid, nblk);
+      if (g.hq_vertex != nullptr) heavy_queue_scan<OT>(g, G, bid, nblk);
+      if (!bar.wait()) return;
+    }
+    if constexpr (kBfs) {
+      if (!bfs_pull) {
+        bfs_push_tiles<W, OT, DEPTH>(g, G, bid, nblk, sm.push);
+        if (g.hq_vertex != nullptr) {
+          __syncthreads();
+          bfs_push_chunks<W, OT, DEPTH>(g, G, nblk - 1 - bid, nblk, sm.slot);
+        }
+      } else {
+        bfs_pull_tiles<W, OT, DEPTH>(g, G, bid, nblk);
+        bfs_pull_mid<W, OT, DEPTH>(g, G, bid, nblk);
+        if (G.n_pheavy > 0) {
+          bfs_pull_chunks<W, OT>(g, G, bid, nblk, sm.pull_heavy);
+          if (!bar.wait()) return;
+          bfs_pull_heavy_commit<W, OT, DEPTH>(g, G, bid, nblk);
+        }
+        // the pull stores whole next masks: SSSP bits are added afterwards
+        if (kSssp && (scatter || gather) && !bar.wait()) return;
+      }
+      __syncthreads();
+    }
+    if constexpr (kSssp) {
+      if (scatter) {
+        sssp_push_tiles<W, OT, WK>(g, G, bid, nblk, sm.sssp_push);
+        if (g.hq_vertex != nullptr) {
+          __syncthreads();
+          sssp_push_chunks<W, OT, WK>(g, G, nblk - 1 - bid, nblk, sm.sssp_heavy);
+        }
+        if (!bar.wait()) return;  // the list of dense vertices is complete
+        sssp_dense_vertices<W, OT, WK, 1>(g, G, bid, nblk);
+        // a gather stores whole vectors of a row
+        if (gather && !bar.wait()) return;
+      }
+      if (gather) {
+        // heavy vertices first: the light ones read their lowered distances
+        if (G.n_pheavy > 0) {
+          sssp_pull_heavy_chunks<W, OT, WK, (W <= 4 ? 3 : 0)>(g, G, bid, nblk, sm.gather_heavy);
+          if (!bar.wait()) return;
+        }
+        constexpr int WS = W < 4 ? W : 4;  // words per slice
+        constexpr unsigned kSlices = W / WS;
+        const unsigned per = nblk / kSlices;
+        if (per == 0) {
+          for (unsigned sl = 0; sl < kSlices; ++sl) {
+            sssp_pull_light_chunks<WS, OT, WK, W>(g, G, bid, nblk, static_cast<int>(sl), sm.gather_light);
+            __syncthreads();
+          }
+        } else if (bid < per * kSlices) {
+          sssp_pull_light_chunks<WS, OT, WK, W>(g, G, bid / kSlices, per,
+                                                static_cast<int>(bid % kSlices), sm.gather_light);
+        }
+      }
+      if (ctl->chunk_dir) {
+        if (!bar.wait()) return;
+        chunk_census<W, OT>(g, G, bid, nblk);
+      }
+    }
+    if (!bar.wait([&](int lane) { level_end<W>(g, lane); })) return;
+  }
 }
 
 // Seeds the sources of every slot (one block).  Level 0 starts afterwards.

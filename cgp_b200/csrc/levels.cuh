@@ -179,12 +179,45 @@ void seed_t(const GroupDev& g, const DevGraph& G, cudaStream_t s) {
   k_seed<W, OT><<<1, kBlock, 0, s>>>(g, G);
 }
 
+template <int W, typename OT, int DEPTH, int WK, bool kBfs, bool kSssp>
+TraverseKernel traverse_kernel() {
+  auto* fn = k_traverse<W, OT, DEPTH, WK, kBfs, kSssp>;
+  static const int per_sm = [&] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kBlock, 0) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    return n;
+  }();
+  return {reinterpret_cast<const void*>(fn), per_sm};
+}
+
+template <int W, typename OT, int DEPTH, int WK>
+TraverseKernel traverse_t(bool has_bfs, bool has_sssp) {
+  // wider groups: a level's work outweighs its launches (see fused_loop)
+  if constexpr (W > 4) return {nullptr, 0};
+  else if (!has_sssp) return traverse_kernel<W, OT, DEPTH, kWeightNone, true, false>();
+  else if constexpr (DEPTH == kDepthPlanes) {
+    return {nullptr, 0};  // planes hold BFS depths only
+  } else {
+    return has_bfs ? traverse_kernel<W, OT, DEPTH, WK, true, true>()
+                   : traverse_kernel<W, OT, DEPTH, WK, false, true>();
+  }
+}
+
+template <int W, typename OT, int DEPTH, int WK>
+Dispatch dispatch_of() {
+  return {enqueue_level_t<W, OT, DEPTH, WK>, grids_t<W, OT, DEPTH, WK>, seed_t<W, OT>,
+          traverse_t<W, OT, DEPTH, WK>};
+}
+
 template <int W, typename OT, int DEPTH>
 Dispatch pick_wk(int wk) {
   switch (wk) {
-    case kWeightU32: return {enqueue_level_t<W, OT, DEPTH, kWeightU32>, grids_t<W, OT, DEPTH, kWeightU32>, seed_t<W, OT>};
-    case kWeightF32: return {enqueue_level_t<W, OT, DEPTH, kWeightF32>, grids_t<W, OT, DEPTH, kWeightF32>, seed_t<W, OT>};
-    default: return {enqueue_level_t<W, OT, DEPTH, kWeightNone>, grids_t<W, OT, DEPTH, kWeightNone>, seed_t<W, OT>};
+    case kWeightU32: return dispatch_of<W, OT, DEPTH, kWeightU32>();
+    case kWeightF32: return dispatch_of<W, OT, DEPTH, kWeightF32>();
+    default: return dispatch_of<W, OT, DEPTH, kWeightNone>();
   }
 }
 

@@ -50,10 +50,20 @@ using EnqueueFn = int (*)(const LevelLaunch&, cudaStream_t);
 using GridsFn = Grids (*)(int);
 using SeedFn = void (*)(const GroupDev&, const DevGraph&, cudaStream_t);
 
+
+// The fused level loop for a group's kinds, and how many of its blocks an SM
+// holds (0: not available).
+struct TraverseKernel {
+  const void* fn;
+  int per_sm;
+};
+using TraverseFn = TraverseKernel (*)(bool has_bfs, bool has_sssp);
+
 struct Dispatch {
   EnqueueFn enqueue;
   GridsFn grids;
   SeedFn seed;
+  TraverseFn traverse;
 };
 
 // Entry points for mask width W (1, 2, 4, 8, 16), offset type OT (int32_t or

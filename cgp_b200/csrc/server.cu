@@ -639,6 +639,7 @@ void cgp_server::loop() {
         const LevelCtl& c = gr.ws->hctl[0];
         if (c.status & kStatusQueueOverflow)
           throw ApiError{CGP_ERR_DEVICE, "heavy frontier queue overflow"};
+        if (c.status & kStatusBarrier) throw ApiError{CGP_ERR_DEVICE, "grid barrier timed out"};
         gr.level = c.level;
         gr.levels_done = c.level;
         gr.sssp_chunk_levels = static_cast<int64_t>(c.sssp_chunk_levels);
