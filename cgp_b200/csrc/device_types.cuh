@@ -109,6 +109,12 @@ struct LevelCtl {
   unsigned long long prev_pull_edges; // in-edges the previous BFS pull level read
   int32_t prev_dir;                 // BFS direction of the previous level
   int32_t bfs_chunked;              // the BFS pull may run in CTA chunks (chunk table built)
+  int32_t bnd_avail;                // bounds arrays exist and the gather kernels read them
+  int32_t bnd_on;                   // this gather level screens row chunks by bounds
+  int32_t bnd_good;                 // the last level that did skipped at least half of them
+  int32_t bnd_wait;                 // gather levels left before bounds are tried again
+  int32_t bnd_fail;                 // tries in a row that skipped too few
+  int32_t gathers;                  // gather levels so far
   uint32_t bar_arrived;             // grid barrier of the fused level loop: blocks arrived,
   uint32_t bar_release;             // barriers passed,
   uint32_t bar_abort;               // and nonzero once a wait has given up
@@ -150,6 +156,7 @@ struct DevGraph {
   const int64_t* plight_beg;         // first pull-CSR in-edge of plight[i]
   const int32_t* plight_pre;         // in-edges of plight[i]'s chunk up to and including it
   int32_t n_plight_chunks;
+  int32_t hub;                       // a vertex of largest in-degree (reference row of the bounds)
   int32_t n_pmid;                    // plight[0 .. n_pmid) have in-degree > 32 (BFS pull mid kernel)
 };
 
@@ -166,6 +173,8 @@ struct GroupDev {
   uint64_t* fsum;      // [V] frontier summary: (level + 1) << 32 | 32-slot chunks with a
                        // frontier bit, written for the frontier's vertices on levels that
                        // screen sources by it (nullptr: not kept)
+  uint32_t* blo;       // [V][2W] per 32-slot chunk: lower bound of (frontier slot - hub's slot),
+  uint32_t* bhi;       // [V][2W] and upper bound of (gathering slot - hub's slot); nullptr: none
   int32_t* dense_list; // [V] SSSP frontier vertices with many active bits
   int32_t* hq_vertex;  // [n_heavy] heavy vertices of the current frontier
   int64_t* hq_start;   // [n_heavy] their first chunk in the level's chunk space

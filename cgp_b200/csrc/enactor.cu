@@ -54,6 +54,7 @@ cgp_status cgp_enactor_create(cgp_graph* graph, const cgp_query* queries, int32_
     e->ws = std::make_unique<Workspace>(g->device);
     e->stream = e->opts.stream ? static_cast<cudaStream_t>(e->opts.stream) : e->ws->stream;
     e->spec = make_group(queries, nq, choose_words(nq, e->opts.mask_words), e->opts.depth_mode);
+    if (e->spec.has_sssp) pad_rows(e->spec);
     for (int i = 0; i < nq; ++i)
       if (queries[i].kind == CGP_KIND_WCC) e->wcc_slots.push_back(i);
     *out = e;
@@ -215,7 +216,7 @@ cgp_status cgp_enactor_read_values(cgp_enactor* e, void* out, int32_t out_layout
   if (!e->prepared) return set_error(CGP_ERR_INVALID_ARG, "prepare_frontier was not called");
   try {
     const int64_t V = e->g->V;
-    const int nq = e->spec.Qg;
+    const int nq = e->spec.n;
     const bool qmajor = out_layout == CGP_LAYOUT_QUERY_MAJOR;
     uint32_t* dout = static_cast<uint32_t*>(out);
     if (!on_device) {

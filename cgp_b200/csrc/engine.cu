@@ -60,6 +60,26 @@ bool DevBuf::ensure(size_t need) {
   return true;
 }
 
+bool DevBuf::offer(size_t need, bool* moved) {
+  if (need <= bytes && p) return true;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || need > free_b / 8) {
+    cudaGetLastError();
+    return false;
+  }
+  if (p) cudaFree(p);
+  p = nullptr;
+  bytes = 0;
+  *moved = true;  // the old block is gone either way
+  if (cudaMalloc(&p, need) != cudaSuccess) {
+    cudaGetLastError();
+    p = nullptr;
+    return false;
+  }
+  bytes = need;
+  return true;
+}
+
 Workspace::Workspace(int dev) : device(dev) {
   ck(cudaHostAlloc(reinterpret_cast<void**>(&hctl), 2 * sizeof(LevelCtl), cudaHostAllocDefault),
      "cudaHostAlloc(ctl)");
@@ -161,6 +181,7 @@ DevGraph GraphImpl::dev_graph(int64_t h) {
   d.n_plight_chunks = hp.plight.chunks;
   d.n_pmid = hp.plight.n_mid;
   d.heavy_degree = h;
+  d.hub = hub;
   return d;
 }
 
@@ -343,6 +364,7 @@ int choose_words(int n, int requested) {
 GroupSpec make_group(const cgp_query* q, int n, int W, int depth_mode) {
   GroupSpec g;
   g.W = W;
+  g.n = n;
   g.Qg = n;
   g.slots.resize(n);
   for (int i = 0; i < n; ++i) {
@@ -357,6 +379,11 @@ GroupSpec make_group(const cgp_query* q, int n, int W, int depth_mode) {
   else if (depth_mode == CGP_DEPTH_DIRECT || g.has_sssp) g.depth_mode = kDepthDirect;
   else g.depth_mode = (n >= 16) ? kDepthPlanes : kDepthDirect;  // auto
   return g;
+}
+
+void pad_rows(GroupSpec& g) {
+  g.Qg = (g.n + 3) & ~3;
+  g.slots.resize(g.Qg, dev::SlotDev{-1, -1, 0, 0});
 }
 
 static constexpr int kInitialPlanes = 8;
@@ -400,6 +427,10 @@ GroupDev group_dev(Workspace* ws, const GroupSpec& spec, bool profiles) {
                  : (spec.external_values ? spec.external_values : ws->values.as<uint32_t>());
   g.hacc = ws->hacc.as<uint64_t>();
   g.fsum = ws->fsum.as<uint64_t>();
+  if (spec.bounds) {
+    g.blo = ws->bounds.as<uint32_t>();
+    g.bhi = g.blo + ws->bounds.bytes / 8;
+  }
   g.dense_list = ws->dense.as<int32_t>();
   g.hq_vertex = ws->hq_vertex.as<int32_t>();
   g.hq_start = ws->hq_start.as<int64_t>();
@@ -425,6 +456,13 @@ bool sssp_gather_on(const GraphImpl* g, const cgp_options& o) {
 bool sssp_chunk_dir(const GroupSpec& spec, const cgp_options& o) {
   if (!spec.has_sssp || o.traversal_mode != CGP_MODE_HYBRID) return false;
   return o.sssp_chunk_direction > 0 || (o.sssp_chunk_direction == 0 && spec.serving);
+}
+
+// Rows the vectorised gather can read: whole kElem-slot vectors, aligned.
+bool vector_rows(const GroupSpec& spec, const uint32_t* values) {
+  const int elem = spec.W == 1 ? 2 : 4;
+  return values != nullptr && spec.Qg % elem == 0 &&
+         reinterpret_cast<uintptr_t>(values) % (4 * elem) == 0;
 }
 
 }  // namespace
@@ -458,6 +496,13 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
       moved |= ws->values.ensure(static_cast<size_t>(V) * spec.Qg * 4);
     }
     if (o.profile_iterations) moved |= ws->prof.ensure(kProfileCap * sizeof(LevelProfile));
+    // Bounds for the default gather kernels.  A serving group decides gather
+    // or scatter per 32-slot chunk and its slots are in every phase at once.
+    spec.bounds = spec.has_sssp && !spec.serving && sssp_gather_on(g, o) &&
+                  !sssp_chunk_dir(spec, o) && o.light_chunks >= 0 &&
+                  vector_rows(spec, spec.external_values ? spec.external_values
+                                                         : ws->values.as<uint32_t>()) &&
+                  ws->bounds.offer(static_cast<size_t>(V) * W * 16, &moved);
   } catch (...) {
     // a failed ensure() has already freed its old block: graphs captured with
     // the old pointers must never be replayed
@@ -510,6 +555,7 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
   c.chunk_dir = sssp_chunk_dir(spec, o) ? 1 : 0;
   c.bfs_chunked = (spec.has_bfs && (o.bfs_pull_form == 1 || o.bfs_pull_form == 2) &&
                    hp.plight.chunks > 0) ? o.bfs_pull_form : 0;
+  c.bnd_avail = spec.bounds ? 1 : 0;
   c.prev_dir = kDirPush;
   c.sssp_pull_edge_threshold = static_cast<unsigned long long>(
       std::max(1.0, o.sssp_pull_edge_ratio * static_cast<double>(g->E)));
@@ -551,13 +597,9 @@ LevelLaunch level_launch(GraphImpl* g, Workspace* ws, const GroupSpec& spec, con
   L.heavy_push = L.G.n_heavy > 0 || g->max_degree > 32;
   L.bfs_chunked = L.pull && spec.has_bfs && L.G.n_plight_chunks > 0 && o.bfs_pull_form == 1;
   L.spull = spec.has_sssp && sssp_gather_on(g, o);
-  {
-    // vector gather: kElem-slot vectors must stay inside rows and be aligned
-    const int elem = spec.W == 1 ? 2 : 4;
-    L.gvec = L.g.values != nullptr && spec.Qg % elem == 0 &&
-             reinterpret_cast<uintptr_t>(L.g.values) % (4 * elem) == 0;
-    L.lchunks = o.light_chunks >= 0;
-  }
+  L.gvec = vector_rows(spec, L.g.values);
+  L.lchunks = o.light_chunks >= 0;
+  L.bounds = spec.bounds;
   L.dense_unroll = o.dense_unroll == 2 ? 2 : 1;
   L.chunk_dir = L.spull && sssp_chunk_dir(spec, o);
   L.kt = nullptr;
@@ -622,7 +664,8 @@ int enqueue_levels(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp
                              (spec.has_bfs ? 1 : 0) | (spec.has_sssp ? 2 : 0) | (L.pull ? 4 : 0) |
                                  (o.profile_iterations ? 8 : 0) | (L.dense_unroll == 2 ? 16 : 0) |
                                  (L.spull ? 32 : 0) | (L.lchunks ? 64 : 0) | (loop ? 128 : 0) |
-                                 (L.chunk_dir ? 256 : 0) | (L.bfs_chunked ? 512 : 0),
+                                 (L.chunk_dir ? 256 : 0) | (L.bfs_chunked ? 512 : 0) |
+                                 (L.bounds ? 1024 : 0),
                              levels, spec.Qg, static_cast<int>(L.G.heavy_degree), ws->generation,
                              reinterpret_cast<uint64_t>(L.g.values));
   auto it = ws->graphs.find(key);
@@ -796,19 +839,19 @@ void group_enqueue_levels(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cg
 void group_write_output(GraphImpl* g, Workspace* ws, GroupSpec& spec, OutMap om,
                         int query_major, cudaStream_t s) {
   spec.launches++;
-  const dim3 grid(g->num_sms * 8, query_major ? std::min(spec.Qg, 65535) : 1);
+  const dim3 grid(g->num_sms * 8, query_major ? std::min(spec.n, 65535) : 1);
   if (spec.depth_mode == kDepthPlanes) {
     LevelCtl c;
     ck(cudaMemcpyAsync(&c, ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost, s), "read ctl");
     ck(cudaStreamSynchronize(s), "read ctl");
     switch (spec.W) {
-#define CGP_MAT(WW) case WW: k_materialize_planes<WW><<<grid, kBlock, 0, s>>>(ws->visited.as<uint64_t>(), ws->planes.as<uint64_t>(), c.num_planes, g->V, spec.Qg, om, query_major); break;
+#define CGP_MAT(WW) case WW: k_materialize_planes<WW><<<grid, kBlock, 0, s>>>(ws->visited.as<uint64_t>(), ws->planes.as<uint64_t>(), c.num_planes, g->V, spec.n, om, query_major); break;
       CGP_MAT(1) CGP_MAT(2) CGP_MAT(4) CGP_MAT(8) CGP_MAT(16)
 #undef CGP_MAT
     }
   } else {
     k_copy_values<<<grid, kBlock, 0, s>>>(group_dev(ws, spec, false).values, ws->slots.as<SlotDev>(),
-                                          g->V, spec.Qg, om, query_major);
+                                          g->V, spec.n, spec.Qg, om, query_major);
   }
   ck(cudaGetLastError(), "write output");
 }
@@ -967,6 +1010,11 @@ cgp_status cgp_graph_create(const void* row_offsets, int32_t offset_bytes,
             ck(cudaMemcpy(G.tw.p, tw.data(), num_edges * 4, cudaMemcpyHostToDevice), "upload t-weights");
         }
       }
+    }
+    {
+      const std::vector<int64_t>& in = trow.empty() ? hrow : trow;
+      for (int64_t v = 1; v < num_vertices; ++v)
+        if (in[v + 1] - in[v] > in[G.hub + 1] - in[G.hub]) G.hub = static_cast<int32_t>(v);
     }
     {
       std::lock_guard<std::mutex> lk(g_host_mu);
@@ -1153,8 +1201,24 @@ cgp_status cgp_batch_run(cgp_graph* graph, const cgp_query* queries, int32_t nq,
       GroupSpec spec = make_group(gq.data(), n, gp.W, o.depth_mode);
       // A device vertex-major output holding exactly this group's columns is
       // used directly as the working value matrix (no copy at the end).
-      const bool in_place = out_on_device && !qmajor && single && wcc_idx.empty() &&
-                            spec.depth_mode != kDepthPlanes;
+      bool in_place = out_on_device && !qmajor && single && wcc_idx.empty() &&
+                      spec.depth_mode != kDepthPlanes;
+      // SSSP rows of a slot count that is no multiple of 4 are padded to one in
+      // a matrix of the engine's own: the gather then reads 16-byte vectors
+      // (499 slots on Chung-Lu, 300K vertices: see GroupSpec::Qg).  An output
+      // that could be used in place is left for that only where the matrix is
+      // small beside the free memory.
+      if (spec.has_sssp && n % 4 != 0 && sssp_gather_on(g, o)) {
+        const size_t need = static_cast<size_t>(V) * ((n + 3) & ~3) * 4;
+        if (in_place && ws->values.bytes < need) {
+          size_t free_b = 0, total_b = 0;
+          ck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+          if (need <= free_b / 4) in_place = false;
+        } else {
+          in_place = false;
+        }
+        if (!in_place) pad_rows(spec);
+      }
       if (in_place) spec.external_values = dout;
       if (kt) kt->mark(kClassInit, s);
       group_prepare(g, ws.get(), spec, o, s);

@@ -38,6 +38,9 @@ struct DevBuf {
   ~DevBuf();
   // Returns true when a new block was allocated (pointers changed).
   bool ensure(size_t need);
+  // As ensure, for a block the caller can do without: false (and no block)
+  // when it would take more than 1/8 of the free device memory.
+  bool offer(size_t need, bool* moved);
   template <typename T>
   T* as() const { return static_cast<T*>(p); }
 };
@@ -123,6 +126,7 @@ struct Workspace {
   int device = 0;
   DevBuf visited, fbuf0, fbuf1, list0, list1, stamp, planes, values, hacc, dense, hq_vertex, hq_start;
   DevBuf fsum;  // frontier summary words (uint64 per vertex)
+  DevBuf bounds;  // gather bounds: two uint32 per vertex and 32-slot chunk
   DevBuf ctl, prof, slots, stage, wcc, qmap;
   LevelCtl* hctl = nullptr;  // pinned, 2 snapshots
   dev::SlotDev* hslots = nullptr;  // pinned, kMaxWords*64 entries
@@ -144,6 +148,7 @@ struct GraphImpl {
   int num_sms = 148;
   int64_t V = 0, E = 0;
   int64_t max_degree = 0;  // largest out-degree of the traversal CSR
+  int32_t hub = 0;         // a vertex of largest in-degree
   int64_t n_deg32 = 0;     // vertices of out-degree > 32 (heavy-queue capacity)
   int offset_bytes = 4;
   int weight_kind = CGP_WEIGHT_NONE;
@@ -176,13 +181,15 @@ struct GraphImpl {
 // A traversal group: up to 64*W slots sharing one set of vertex masks.
 struct GroupSpec {
   int W = 1;
-  int Qg = 0;
+  int n = 0;   // queries (slots 0 .. n-1)
+  int Qg = 0;  // slots per value row: n, or n rounded up to 4 (pad_rows)
   std::vector<dev::SlotDev> slots;
   int depth_mode = dev::kDepthDirect;
   bool has_bfs = false;
   bool has_sssp = false;
   uint32_t* external_values = nullptr;  // caller's device buffer used as working values
   uint32_t uniform_inf = 0;             // nonzero: fill every value with it (serving)
+  bool bounds = false;                  // gather levels may screen by bounds
   bool serving = false;                 // the group belongs to a serving loop
   uint64_t launches = 0;                // kernels enqueued for this group
 };
@@ -201,6 +208,9 @@ struct GroupRun {
 
 // Engine entry points (engine.cu).
 GroupSpec make_group(const cgp_query* q, int n, int W, int depth_mode);
+// Rounds the value rows up to a multiple of 4 slots; the added slots belong to
+// no query (kind and source -1: never seeded, never written out).
+void pad_rows(GroupSpec& g);
 void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options& o,
                    cudaStream_t s);
 // Runs levels until convergence (done != 0) or, with max_levels > 0, that

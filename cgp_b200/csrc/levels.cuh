@@ -35,6 +35,10 @@ int enqueue_level_t(const LevelLaunch& L, cudaStream_t s) {
     k_frontier_summary<W, OT><<<c, kBlock, 0, s>>>(L.g, L.G);
     ++n;
   }
+  if (L.bounds) {
+    k_gather_bounds<W, OT, WK><<<t, kBlock, 0, s>>>(L.g, L.G);
+    ++n;
+  }
   if (L.heavy_push) {
     k_heavy_queue<OT><<<c, kBlock, 0, s>>>(L.g, L.G);
     ++n;

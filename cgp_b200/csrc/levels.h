@@ -33,6 +33,7 @@ struct LevelLaunch {
   bool has_bfs;
   bool has_sssp;
   bool pull;
+  bool bounds = false;  // gather levels may screen by bounds
   bool spull;        // SSSP gather kernels are part of the level
   bool gvec;         // rows allow the vectorised gather (alignment, width)
   bool lchunks;      // light vertices gathered in CTA chunks (in 4-word slices above W = 4)

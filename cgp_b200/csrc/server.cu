@@ -750,6 +750,7 @@ cgp_status cgp_server_create(cgp_graph* graph, int32_t slots, const cgp_options*
       gr.ws = std::make_unique<Workspace>(g->device);
       gr.stream = gr.ws->stream;
       gr.spec.W = gr.W;
+      gr.spec.n = gr.S;
       gr.spec.Qg = gr.S;
       gr.spec.slots.assign(gr.S, SlotDev{-1, -1, 0, 0});
       gr.spec.depth_mode = kDepthDirect;
