@@ -17,6 +17,7 @@ constexpr int kMaxW = 16;
 constexpr int kMaxPlanes = 24;
 constexpr int kLightChunkVerts = 32;    // light vertices per chunked-gather CTA item
 constexpr int kLightChunkEdges = 2048;  // and their in-edges
+constexpr int kGatherHeavy = 256;       // in-edges one warp of the row gather takes at most
 
 enum : int32_t { kDirPush = 0, kDirPull = 1 };
 enum : int32_t { kDepthNone = 0, kDepthDirect = 1, kDepthPlanes = 2 };
@@ -154,8 +155,16 @@ struct DevGraph {
   const int32_t* plight;             // light vertices of the pull CSR (chunked gathers)
   const int32_t* plight_chunk_start; // [n_plight_chunks + 1]
   const int64_t* plight_beg;         // first pull-CSR in-edge of plight[i]
-  const int32_t* plight_pre;         // in-edges of plight[i]'s chunk up to and including it
   int32_t n_plight_chunks;
+  const int32_t* gitem_start;        // [n_gitems + 1] row gather items: runs of plight entries
+  const int32_t* gitem_pre;          // in-edges of plight[i]'s item up to and including it
+  int32_t n_gitems;
+  const int32_t* sheavy;             // the vector gather's heavy vertices: above kGatherHeavy
+  const int32_t* sheavy_ch;          // in-edges beside the row gather, else the pheavy table
+  const int64_t* sheavy_cb;
+  const int64_t* sheavy_ce;
+  int32_t n_sheavy;
+  int64_t sheavy_chunks;
   int32_t hub;                       // a vertex of largest in-degree (reference row of the bounds)
   int32_t n_pmid;                    // plight[0 .. n_pmid) have in-degree > 32 (BFS pull mid kernel)
 };

@@ -152,7 +152,7 @@ void KernelTimer::flush() {
 }
 
 // --------------------------------------------------------------- graph
-DevGraph GraphImpl::dev_graph(int64_t h) {
+DevGraph GraphImpl::dev_graph(int64_t h, bool light_items) {
   const HeavyPair& hp = heavy_for(h);
   DevGraph d;
   d.row = row.p;
@@ -177,9 +177,18 @@ DevGraph GraphImpl::dev_graph(int64_t h) {
   d.plight = hp.plight.vertices.as<int32_t>();
   d.plight_chunk_start = hp.plight.chunk_start.as<int32_t>();
   d.plight_beg = hp.plight.beg.as<int64_t>();
-  d.plight_pre = hp.plight.pre.as<int32_t>();
   d.n_plight_chunks = hp.plight.chunks;
   d.n_pmid = hp.plight.n_mid;
+  d.gitem_start = hp.plight.item_start.as<int32_t>();
+  d.gitem_pre = hp.plight.item_pre.as<int32_t>();
+  d.n_gitems = hp.plight.items;
+  const HeavyTable& sh = light_items ? hp.gheavy : hp.pheavy;
+  d.sheavy = sh.vertices.as<int32_t>();
+  d.sheavy_ch = sh.chunk_h.as<int32_t>();
+  d.sheavy_cb = sh.chunk_beg.as<int64_t>();
+  d.sheavy_ce = sh.chunk_end.as<int64_t>();
+  d.n_sheavy = sh.n;
+  d.sheavy_chunks = sh.chunks;
   d.heavy_degree = h;
   d.hub = hub;
   return d;
@@ -241,14 +250,18 @@ void build_light_chunks(const std::vector<int64_t>& row, int64_t V, int64_t h, L
   // light vertices by in-degree, largest first (ties by id): CTAs take chunks
   // roughly in this order, so within a gather level the better-connected
   // vertices settle first and the rest read their lowered distances
-  std::vector<int32_t> order;
+  // (a counting sort by in-degree)
+  std::vector<int64_t> at(static_cast<size_t>(h) + 2, 0);
   for (int64_t v = 0; v < V; ++v) {
     const int64_t d = row[v + 1] - row[v];
-    if (d > 0 && d <= h) order.push_back(static_cast<int32_t>(v));
+    if (d > 0 && d <= h) ++at[h - d + 1];
   }
-  std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
-    return row[a + 1] - row[a] > row[b + 1] - row[b];
-  });
+  for (int64_t i = 0; i <= h; ++i) at[i + 1] += at[i];
+  std::vector<int32_t> order(static_cast<size_t>(at[h + 1]));
+  for (int64_t v = 0; v < V; ++v) {
+    const int64_t d = row[v + 1] - row[v];
+    if (d > 0 && d <= h) order[at[h - d]++] = static_cast<int32_t>(v);
+  }
   std::vector<int32_t> vs;
   std::vector<int32_t> cs{0};
   int cur_v = 0;
@@ -269,33 +282,43 @@ void build_light_chunks(const std::vector<int64_t>& row, int64_t V, int64_t h, L
   t.chunks = static_cast<int32_t>(cs.size()) - 1;
   t.n_mid = 0;
   while (t.n_mid < t.n && row[vs[t.n_mid] + 1] - row[vs[t.n_mid]] > 32) ++t.n_mid;
-  // per entry: its first in-edge and the chunk's in-edges up to and including
-  // it, so that a chunk's header is three independent loads
+  // per entry: its first in-edge; and the row gather's items with their
+  // in-edge prefixes, so that an item's header is three independent loads
   std::vector<int64_t> beg(vs.size());
-  std::vector<int32_t> pre(vs.size());
-  for (size_t c = 0; c + 1 < cs.size(); ++c) {
-    int32_t acc = 0;
-    for (int32_t i = cs[c]; i < cs[c + 1]; ++i) {
-      const int32_t v = vs[i];
-      beg[i] = row[v];
-      acc += static_cast<int32_t>(row[v + 1] - row[v]);
-      pre[i] = acc;
+  std::vector<int32_t> pre(vs.size()), is;
+  int32_t run = 0, acc = 0;
+  for (size_t i = 0; i < vs.size(); ++i) {
+    beg[i] = row[vs[i]];
+    const int64_t d = row[vs[i] + 1] - row[vs[i]];
+    if (d > dev::kGatherHeavy) continue;
+    if (is.empty() || run == 32 || acc + d > dev::kGatherHeavy) {
+      is.push_back(static_cast<int32_t>(i));
+      run = 0;
+      acc = 0;
     }
+    ++run;
+    acc += static_cast<int32_t>(d);
+    pre[i] = acc;
   }
+  t.items = static_cast<int32_t>(is.size());
+  is.push_back(static_cast<int32_t>(vs.size()));
   t.vertices.ensure(std::max<size_t>(vs.size(), 1) * sizeof(int32_t));
   t.chunk_start.ensure(cs.size() * sizeof(int32_t));
   t.beg.ensure(std::max<size_t>(vs.size(), 1) * sizeof(int64_t));
-  t.pre.ensure(std::max<size_t>(vs.size(), 1) * sizeof(int32_t));
+  t.item_start.ensure(is.size() * sizeof(int32_t));
+  t.item_pre.ensure(std::max<size_t>(vs.size(), 1) * sizeof(int32_t));
   if (!vs.empty()) {
     ck(cudaMemcpy(t.vertices.p, vs.data(), vs.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
        "upload light vertices");
     ck(cudaMemcpy(t.beg.p, beg.data(), beg.size() * sizeof(int64_t), cudaMemcpyHostToDevice),
        "upload light offsets");
-    ck(cudaMemcpy(t.pre.p, pre.data(), pre.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
+    ck(cudaMemcpy(t.item_pre.p, pre.data(), pre.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
        "upload light prefixes");
   }
   ck(cudaMemcpy(t.chunk_start.p, cs.data(), cs.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
      "upload light chunks");
+  ck(cudaMemcpy(t.item_start.p, is.data(), is.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
+     "upload gather items");
 }
 
 }  // namespace
@@ -310,6 +333,8 @@ const HeavyPair& GraphImpl::heavy_for(int64_t h) {
     HostCsr& hc = g_host[this];
     build_heavy(hc.row, V, h, hp->heavy);
     build_heavy(hc.trow.empty() ? hc.row : hc.trow, V, h, hp->pheavy);
+    build_heavy(hc.trow.empty() ? hc.row : hc.trow, V, std::min<int64_t>(h, dev::kGatherHeavy),
+                hp->gheavy);
     build_light_chunks(hc.trow.empty() ? hc.row : hc.trow, V, h, hp->plight);
   }
   return *heavy_cache.emplace(h, std::move(hp)).first->second;
@@ -587,7 +612,7 @@ LevelLaunch level_launch(GraphImpl* g, Workspace* ws, const GroupSpec& spec, con
                          const Dispatch& d) {
   LevelLaunch L;
   L.g = group_dev(ws, spec, o.profile_iterations != 0);
-  L.G = g->dev_graph(heavy_threshold(o));
+  L.G = g->dev_graph(heavy_threshold(o), o.light_chunks >= 0);
   L.gr = d.grids(g->num_sms);
   L.has_bfs = spec.has_bfs;
   L.has_sssp = spec.has_sssp;
@@ -611,12 +636,14 @@ constexpr int64_t kFusedWork = 1 << 24;
 
 // Whether the group's levels run as the fused loop: the automatic loop form,
 // with the kernel variants the loop holds (the default ones).
-bool fused_loop(const GroupSpec& spec, const cgp_options& o, const LevelLaunch& L) {
-  if (o.level_loop != CGP_LOOP_AUTO || !o.use_cuda_graph || o.bfs_pull_form != 0) return false;
+bool fused_loop(const GroupSpec& spec, const cgp_options& o, const Dispatch& d,
+                const LevelLaunch& L) {
   if (spec.W > 4 || (spec.has_sssp && L.G.E * spec.W > kFusedWork)) return false;
+  if (o.level_loop != CGP_LOOP_AUTO || !o.use_cuda_graph || o.bfs_pull_form != 0) return false;
   // serving groups on streams of their own: launched levels of different
   // groups overlap on the device, cooperative launches take all of it in turn
   if (spec.serving && (o.serve_groups > 1 || o.serve_admission == 2)) return false;
+  if (d.traverse(spec.has_bfs, spec.has_sssp).per_sm < 1) return false;
   if (spec.has_sssp && (L.dense_unroll == 2 || (L.spull && !(L.gvec && L.lchunks)))) return false;
   return true;
 }
@@ -630,7 +657,6 @@ constexpr int kFusedLevels = 256;
 int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelLaunch& L,
                   cudaStream_t s, int levels) {
   const TraverseKernel k = d.traverse(spec.has_bfs, spec.has_sssp);
-  if (k.fn == nullptr || k.per_sm < 1) return 0;
   const int most = k.per_sm * g->num_sms;
   const int blocks = static_cast<int>(std::max<int64_t>(
       1, std::min<int64_t>(most, (g->E + g->V) / 512)));
@@ -647,10 +673,8 @@ int enqueue_levels(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp
                    cudaStream_t s, int levels, KernelTimer* kt) {
   Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
   LevelLaunch L = level_launch(g, ws, spec, o, d);
-  if (kt == nullptr && levels > 0 && fused_loop(spec, o, L)) {
-    const int n = enqueue_fused(g, spec, d, L, s, levels);
-    if (n > 0) return n;
-  }
+  if (kt == nullptr && levels > 0 && fused_loop(spec, o, d, L))
+    return enqueue_fused(g, spec, d, L, s, levels);
   L.kt = kt;
   if (!o.use_cuda_graph || kt != nullptr) {
     int n = 0;
@@ -726,7 +750,7 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
   bool fused = false;
   if (kt == nullptr) {
     const Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
-    fused = fused_loop(spec, o, level_launch(g, ws, spec, o, d));
+    fused = fused_loop(spec, o, d, level_launch(g, ws, spec, o, d));
   }
   const int per_chunk = kt ? 1 : (o.levels_per_sync > 0 ? o.levels_per_sync
                                                         : (fused ? kFusedLevels : 8));

@@ -64,14 +64,19 @@ struct LightChunks {
   DevBuf vertices;     // int32 [n] light vertices, largest in-degree first
   DevBuf chunk_start;  // int32 [chunks + 1] positions in `vertices`
   DevBuf beg;          // int64 [n] first in-edge of each vertex in the pull CSR
-  DevBuf pre;          // int32 [n] in-edges of the chunk up to and including the vertex
+  DevBuf item_start;   // int32 [items + 1] positions in `vertices` of the row gather's items:
+                       // runs of at most 32 vertices and kGatherHeavy in-edges, over the
+                       // vertices of at most kGatherHeavy in-edges
+  DevBuf item_pre;     // int32 [n] in-edges of the item up to and including the vertex
   int32_t n = 0;
   int32_t chunks = 0;
+  int32_t items = 0;
   int32_t n_mid = 0;   // the first n_mid have in-degree > 32
 };
 
 struct HeavyPair {
   HeavyTable heavy, pheavy;
+  HeavyTable gheavy;   // vertices of more than kGatherHeavy in-edges (beside the items)
   LightChunks plight;
 };
 
@@ -173,7 +178,8 @@ struct GraphImpl {
   bool can_gather() const { return pull_row() != nullptr; }
   // Heavy tables for threshold h (built on first use, then kept).
   const HeavyPair& heavy_for(int64_t h);
-  dev::DevGraph dev_graph(int64_t h);
+  // light_items: the vector gather's light vertices go by items (row gather).
+  dev::DevGraph dev_graph(int64_t h, bool light_items = true);
   std::unique_ptr<Workspace> acquire();
   void release(std::unique_ptr<Workspace> ws);
 };

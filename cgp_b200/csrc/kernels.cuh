@@ -66,6 +66,13 @@ __device__ __forceinline__ bool mask_any(const uint64_t (&m)[W]) {
   return a != 0;
 }
 
+template <int W>
+__device__ __forceinline__ bool any_bits(const uint64_t* m) {
+  uint64_t a = 0;
+  for (int i = 0; i < W; ++i) a |= m[i];
+  return a != 0;
+}
+
 __device__ __forceinline__ uint64_t atomic_or64(uint64_t* p, uint64_t v) {
   return static_cast<uint64_t>(atomicOr(reinterpret_cast<unsigned long long*>(p),
                                         static_cast<unsigned long long>(v)));
@@ -2522,193 +2529,264 @@ __device__ __forceinline__ int chunk_edge_owner(int my_pre, int f0, int lane) {
   return k0 + __popc(starts & upto);
 }
 
-// Gather level (vectorised), light vertices in CTA chunks.  A chunk is a
-// run of up to kLightChunkVerts light vertices with at most kLightChunkEdges
-// in-edges in total (static table of the pull CSR).  The CTA's warps split
-// the chunk's in-edges evenly, across vertex boundaries, so every warp keeps
-// several source rows in flight all the time instead of stalling on each
-// small vertex's chain of dependent loads; a warp min-reduces its run of one
-// vertex into that vertex's row in shared memory, and after a barrier each
-// vertex is committed once (compare, store, frontier words, append: no
-// atomics, the chunk owns its vertices).  W <= 4 (a row of 64W slots fits
-// 32 times in 32 KB of shared memory).  Wider groups (WF = 8 or 16 words)
-// are gathered in slices of W words: blockIdx.y is the slice, each CTA owns
-// its vertices' slice of the row, and the frontier append is claimed with an
-// atomic on the stamp (the slices of a vertex commit in different CTAs).
+// ORs each 32-slot chunk's improved bits over the lanes that own its slots and
+// hands every chunk's word to one lane: `bits` holds the lane's kSlots bits
+// (slot r*kElem + k at bit r*kElem + k); the lane that receives a chunk gets
+// its index in *chunk (else -1).  With two parts the halves of the lanes swap
+// the part they do not keep, so both are reduced in log2(lanes per chunk)
+// shuffles together.
 template <int W>
-struct GatherChunkSmem {
-  alignas(16) uint32_t best[kLightChunkVerts * 64 * W];
-  int4 stage[kWarpsPerBlock][32];
-  int32_t v[kLightChunkVerts];
-  int64_t beg[kLightChunkVerts];
-  int32_t pre[kLightChunkVerts + 1];
-  alignas(16) uint32_t hi[kLightChunkVerts][2 * W];
+__device__ __forceinline__ uint32_t chunk_word(uint32_t bits, int lane, int* chunk) {
+  using GV = GatherVec<W>;
+  constexpr int E = GV::kElem;
+  constexpr int L = GV::kLanesPerHalf;
+  constexpr uint32_t kMask = (1u << E) - 1u;
+  const int sh = E * (lane % L);
+  uint32_t h;
+  if constexpr (GV::kParts == 2) {
+    const uint32_t h0 = (bits & kMask) << sh, h1 = ((bits >> E) & kMask) << sh;
+    const bool odd = lane & 1;
+    h = (odd ? h1 : h0) | __shfl_xor_sync(kFull, odd ? h0 : h1, 1);
+#pragma unroll
+    for (int o = L / 2; o > 1; o >>= 1) h |= __shfl_xor_sync(kFull, h, o);
+    *chunk = lane % L < 2 ? (32 / L) * (lane & 1) + lane / L : -1;
+  } else {
+    static_assert(GV::kParts == 1, "one or two parts per row slice");
+    h = (bits & kMask) << sh;
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) h |= __shfl_xor_sync(kFull, h, o);
+    *chunk = lane % L == 0 ? lane / L : -1;
+  }
+  return h;
+}
+
+// Gather level (vectorised), vertices of at most kGatherHeavy in-edges: a warp
+// takes an item, a run of up to 32 vertices of about the same in-degree with at
+// most kGatherHeavy in-edges in all, and walks the item's in-edges 32 at a
+// time.  Each lane screens one in-edge (by the bounds, or by the source's
+// frontier chunks); what is left goes to the warp's staging list with one
+// entry for the vertex's own row before its first live in-edge, and the rows
+// are read kSteps at a time, relaxed in registers and committed when the next
+// vertex's own row comes up.  A vertex none of whose in-edges is live costs
+// its screening only.  The warp owns its vertices' rows (no distance atomics),
+// and the next 32 in-edges and the next item's header are in flight while the
+// current ones are worked on.  Groups of more than 256 slots are taken in
+// slices of 4 words, slice by slice over all items.
+//
+// What bounds it: reading rows from L2 (a loop that only reads and relaxes
+// 1 KB rows in R-MAT 20's order reaches 16.7 TB/s).  The form before it, a CTA
+// per 32 vertices with row minima merged in shared memory, spent most of its
+// time outside that: 8.4 TB/s when every row is read, and 1.4 ms for a level
+// that reads 1% of them.
+constexpr int kRowStage = 64;  // 32 in-edges and as many own rows
+
+struct GatherRowSmem {
+  int4 stage[kWarpsPerBlock][kRowStage];
+  alignas(16) uint32_t hi[kWarpsPerBlock][32][8];
 };
 
 template <int W, typename OT, int WK, int WF>
-__device__ __forceinline__ void sssp_pull_light_chunks(const GroupDev& g, const DevGraph& G,
-                                                       unsigned bid, unsigned nblk, int sl,
-                                                       GatherChunkSmem<W>& sm) {
-  static_assert(W <= 4, "chunked gather holds 32 rows of at most 256 slots");
+__device__ __forceinline__ void sssp_pull_light_rows(const GroupDev& g, const DevGraph& G,
+                                                     unsigned bid, unsigned nblk,
+                                                     GatherRowSmem& sm) {
+  static_assert(W <= 4, "a slice is at most 256 slots");
   static_assert(WF % W == 0, "a group is a whole number of slices");
   using GV = GatherVec<W>;
   constexpr int E = GV::kElem;
   constexpr int P = GV::kParts;
-  constexpr int S = GV::kSteps < 4 ? GV::kSteps : 4;
-  constexpr int R = 64 * W;
+  constexpr int S = W == 4 ? 4 : 8;
   const LevelCtl* ctl = g.ctl;
-  if (ctl->done || ctl->sdir != kDirPull || G.n_plight_chunks == 0) return;
+  if (ctl->done || ctl->sdir != kDirPull || G.n_gitems == 0) return;
   const LevelView lv = level_view(g);
-  uint32_t (&s_best)[kLightChunkVerts * 64 * W] = sm.best;
-  int4 (&s_stage)[kWarpsPerBlock][32] = sm.stage;
-  int32_t (&s_v)[kLightChunkVerts] = sm.v;
-  int64_t (&s_beg)[kLightChunkVerts] = sm.beg;
-  int32_t (&s_pre)[kLightChunkVerts + 1] = sm.pre;
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
-  const int s0 = sl * 64 * W;  // first slot of the slice of W words
-  const uint64_t* sb = ctl->gsel + sl * W;
-  uint32_t pmask, smask;
-  gather_vec_masks<W>(sb, g.Qg - s0, lane, &pmask, &smask);
-  const uint32_t gch = gather_chunks<W>(sb);
-  if (gch == 0) return;  // no gathering slot in this slice (uniform over the CTA)
-  // screen or read whole rows: one decision for the whole group
-  int screen_qs = gather_screen_qs<WF>(g, ctl, lv, G.E);
-  if (screen_qs >= 0) {
-    screen_qs = 0;
-#pragma unroll
-    for (int i = 0; i < W; ++i) screen_qs += __popcll(sb[i]);
-  }
+  const unsigned below = (1u << lane) - 1u;
+  int4* stage = sm.stage[wib];
+  uint32_t(*s_hi)[8] = sm.hi[wib];
   const bool bounds = ctl->bnd_on != 0;
+  const bool screened = gather_screen_qs<WF>(g, ctl, lv, G.E) < 0;
+  // only this kernel adds bits to its vertices' next masks: plain stores
+  const bool plain = !ctl->sscatter && !any_bits<WF>(ctl->bfs_bits);
   const size_t Qg = static_cast<size_t>(g.Qg);
-  const uint32_t* lanebase = g.values + s0 + lane * E;
-  WarpAppender ap;
-  uint32_t uacc = 0;
+  const long long n_items = G.n_gitems;
+  const long long total_items = n_items * (WF / W);
+  const long long gw = (static_cast<long long>(bid) * blockDim.x + threadIdx.x) >> 5;
+  const long long nwarps = (static_cast<long long>(nblk) * blockDim.x) >> 5;
+
+  int sl = -1;             // current slice
+  uint32_t pmask = 0, smask = 0, gch = 0;
+  int qs = 0;              // gathering slots of the slice
+  uint32_t uacc = 0;       // union of the slice's improved bits
   unsigned long long improved = 0, pairs = 0;
   unsigned scanned = 0, verts = 0;
-  for (int c = bid; c < G.n_plight_chunks; c += nblk) {
-    const int cs = G.plight_chunk_start[c];
-    const int nv = G.plight_chunk_start[c + 1] - cs;
-    if (wib == 0) {
-      // vertex, first in-edge and in-edge prefix come from the table: three
-      // independent loads (no chain through the offsets)
-      if (lane < nv) {
-        s_v[lane] = G.plight[cs + lane];
-        s_beg[lane] = G.plight_beg[cs + lane];
-        s_pre[lane + 1] = G.plight_pre[cs + lane];
-        if (bounds) {
-          constexpr int N = 2 * W < 4 ? 2 : 4;
-          const uint32_t* hi = g.bhi + static_cast<size_t>(s_v[lane]) * (2 * WF) + sl * 2 * W;
+  int32_t pend_v = 0;      // lane i: i-th vertex waiting to be appended
+  int pend_n = 0;          // uniform
+
+  auto flush_union_bits = [&]() {
+    int c;
+    const uint32_t w = chunk_word<W>(uacc, lane, &c);
+    if (c >= 0 && w) {
+      const int at = sl * 2 * W + c;  // 32-bit halves of the active words
+      atomic_or64(lv.nactive + (at >> 1), static_cast<uint64_t>(w) << (32 * (at & 1)));
+    }
+    uacc = 0;
+  };
+  auto flush_pending = [&]() {
+    bool fresh = false;
+    if (lane < pend_n) fresh = atomicMax(g.stamp + pend_v, lv.level + 1) < lv.level + 1;
+    warp_append(fresh, pend_v, fresh ? degree_of<OT>(G.row, pend_v) : 0, lv.nlist, lv.ncount,
+                lv.nedges, lane);
+    pend_n = 0;
+  };
+
+  // header of the next item: lane k holds its k-th vertex
+  int32_t hv = 0, hpre = 0;
+  int64_t hbeg = 0;
+  int hnv = 0;
+  auto load_header = [&](long long it) {
+    const long long i = WF > W ? it % n_items : it;
+    const int cs = G.gitem_start[i];
+    hnv = G.gitem_start[i + 1] - cs;
+    if (lane < hnv) {
+      hv = G.plight[cs + lane];
+      hbeg = G.plight_beg[cs + lane];
+      hpre = G.gitem_pre[cs + lane];
+    }
+  };
+  if (gw < total_items) load_header(gw);
+  for (long long it = gw; it < total_items; it += nwarps) {
+    const int nsl = WF > W ? static_cast<int>(it / n_items) : 0;
+    if (nsl != sl) {
+      if (sl >= 0) flush_union_bits();
+      sl = nsl;
+      const uint64_t* sb = ctl->gsel + sl * W;
+      gather_vec_masks<W>(sb, g.Qg - sl * 64 * W, lane, &pmask, &smask);
+      gch = gather_chunks<W>(sb);
+      qs = 0;
 #pragma unroll
-          for (int i = 0; i < 2 * W; i += N) {
-            uint32_t x[N];
-            load_vec<N>(hi + i, x);
-            store_vec<N>(&sm.hi[lane][i], x);
-          }
+      for (int i = 0; i < W; ++i) qs += __popcll(sb[i]);
+    }
+    const int nv = hnv;
+    const int32_t v = hv;
+    const int total = __shfl_sync(kFull, hpre, nv - 1);
+    int start = __shfl_up_sync(kFull, hpre, 1);
+    if (lane == 0) start = 0;
+    const int64_t base = hbeg - start;  // in-edge f of the item: base + f
+    if (lane >= nv) start = 0x7fffffff;
+    if (it + nwarps < total_items) load_header(it + nwarps);
+    if (gch == 0) continue;  // no gathering slot in this slice
+    const size_t hoff = static_cast<size_t>(sl) * 2 * W;  // the slice's chunks in the bounds
+    if (bounds) {
+      constexpr int N = 2 * W < 4 ? 2 : 4;
+      if (lane < nv) {
+        const uint32_t* hi = g.bhi + static_cast<size_t>(v) * (2 * WF) + hoff;
+#pragma unroll
+        for (int i = 0; i < 2 * W; i += N) {
+          uint32_t x[N];
+          load_vec<N>(hi + i, x);
+          store_vec<N>(&s_hi[lane][i], x);
         }
       }
-      if (lane == 0) s_pre[0] = 0;
+      __syncwarp();
     }
-    for (int i = threadIdx.x; i < nv * R; i += blockDim.x) s_best[i] = 0xffffffffu;
-    __syncthreads();
-    // the rows the commit reads: the 2W lines of 128 bytes of each vertex's
-    // slice move to L2 while the chunk gathers
-    {
-      const int k = static_cast<int>(threadIdx.x >> 3), ln = static_cast<int>(threadIdx.x & 7);
-      if (k < nv && ln < 2 * W && s0 + ln * 32 < g.Qg)
-        prefetch_l2(g.values + static_cast<size_t>(s_v[k]) * Qg + s0 + ln * 32);
+    if (sl == 0) {
+      verts += lane == 0 ? nv : 0;
+      for (int f = lane; f < total; f += 32) ++scanned;
     }
-    const int total = s_pre[nv];
-    const int seg = (total + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    const int fa = min(total, wib * seg);
-    const int fb = min(total, fa + seg);
-    uint32_t best[GV::kSlots];
+    const uint32_t* lanebase = g.values + sl * 64 * W + lane * E;
+    uint32_t best[GV::kSlots], own[GV::kSlots];
+    int cur_k = -1;     // vertex in work (uniform)
+    int32_t cur_v = 0;
+    auto commit = [&]() {
+      uint32_t imp = 0;
 #pragma unroll
-    for (int j = 0; j < GV::kSlots; ++j) best[j] = 0xffffffffu;
-    int cur_k = -1;
-    // adds this warp's run of vertex cur_k into its shared row
-    auto flush_row = [&]() {
-      uint32_t* row = s_best + cur_k * R;
+      for (int r = 0; r < P; ++r) {
+        uint32_t b = 0;
 #pragma unroll
-      for (int j = 0; j < GV::kSlots; ++j) {
-        if (best[j] != 0xffffffffu) atomicMin(row + (32 * (j / E) + lane) * E + (j % E), best[j]);
-        best[j] = 0xffffffffu;
+        for (int q = 0; q < E; ++q) {
+          const int j = r * E + q;
+          const bool up = ((smask >> j) & 1u) && best[j] < own[j];
+          best[j] = up ? best[j] : own[j];
+          b |= static_cast<uint32_t>(up) << q;
+        }
+        if (b) store_vec<E>(const_cast<uint32_t*>(lanebase) + static_cast<size_t>(cur_v) * Qg + 32 * E * r, &best[r * E]);
+        imp |= b << (r * E);
+      }
+      if (!__any_sync(kFull, imp != 0)) return;
+      improved += __popc(imp);
+      uacc |= imp;
+      int c;
+      const uint32_t w = chunk_word<W>(imp, lane, &c);
+      if (c >= 0 && w) {
+        uint32_t* fw = reinterpret_cast<uint32_t*>(lv.fnext + static_cast<size_t>(cur_v) * WF) + hoff + c;
+        if (plain) *fw = w;
+        else atomicOr(fw, w);
+      }
+      if (lane == pend_n) pend_v = cur_v;
+      if (++pend_n == 32) flush_pending();
+    };
+
+    // in-edges f0 .. f0 + 31, lane by lane (the next batch is loaded ahead)
+    int nk = 0;
+    int32_t nu = 0;
+    uint32_t nw = 0;
+    auto load_batch = [&](int f0) {
+      nk = chunk_edge_owner(start, f0, lane);
+      const int64_t e = __shfl_sync(kFull, base, nk) + f0 + lane;
+      if (f0 + lane < total) {
+        nu = G.pcol[e];
+        nw = weight_bits<WK>(G.pw, e);
       }
     };
-    int4* stage = s_stage[wib];
-    for (int f0 = fa; f0 < fb; f0 += 32) {
-      const int f = f0 + lane;
-      int cnt = 0;
-      int32_t u = 0;
-      uint32_t wb = 0;
-      uint32_t cm = 0xffffffffu;  // 32-slot chunks of the source row to read
-      const int k = chunk_edge_owner(lane < nv ? s_pre[lane] : 0x7fffffff, f0, lane);
-      if (f < fb) {
-        const int64_t e = s_beg[k] + (f - s_pre[k]);
-        u = G.pcol[e];
-        wb = weight_bits<WK>(G.pw, e);
-        if (bounds) {
-          cm = bound_chunks<W, WK>(g.blo + static_cast<size_t>(u) * (2 * WF) + sl * 2 * W, sm.hi[k],
-                                   wb) & gch;
-          cnt = __popc(cm) << 5;
-        } else if (screen_qs < 0 && g.fsum != nullptr) {
-          cm = (summary_chunks(g.fsum, lv.level, u) >> (2 * W * sl)) & gch;
-          cnt = __popc(cm) << 5;
-        } else if (screen_qs < 0) {
+    load_batch(0);
+    for (int f0 = 0; f0 < total; f0 += 32) {
+      const int k = nk;
+      const int32_t u = nu;
+      const uint32_t wb = nw;
+      uint32_t cm = 0;
+      if (f0 + lane < total) {
+        if (bounds)
+          cm = bound_chunks<W, WK>(g.blo + static_cast<size_t>(u) * (2 * WF) + hoff, s_hi[k], wb) & gch;
+        else if (!screened)
+          cm = gch;
+        else if (g.fsum != nullptr)
+          cm = (summary_chunks(g.fsum, lv.level, u) >> hoff) & gch;
+        else {
           uint64_t m[W];
           load_mask<W>(lv.fcur + static_cast<size_t>(u) * WF + sl * W, m);
-          // the next batch's source masks move to L2 while this batch's rows load
-          const int fn = f + 32;
-          if (fn < fb) {
-            int a = k, b = nv - 1;  // owner of fn: last k' >= k with s_pre[k'] <= fn
-            while (a < b) {
-              const int mid = (a + b + 1) >> 1;
-              if (s_pre[mid] <= fn) a = mid;
-              else b = mid - 1;
-            }
-            prefetch_l2(lv.fcur + static_cast<size_t>(G.pcol[s_beg[a] + (fn - s_pre[a])]) * WF + sl * W);
-          }
 #pragma unroll
-          for (int i = 0; i < W; ++i) {
-            m[i] &= sb[i];
-            cnt += __popcll(m[i]);
-          }
+          for (int i = 0; i < W; ++i) m[i] &= ctl->gsel[sl * W + i];
           cm = chunk_bits<W>(m);
-        } else {
-          cnt = screen_qs;
-        }
-        if (sl == 0) ++scanned;  // in-edges counted once per group
-        if (cnt > 0 && fb - fa <= 32) {
-          // a warp whose whole share is one batch (chunks of low in-degree
-          // vertices, where the gather waits on latency): the source row's
-          // live 128-byte chunks move to L2 now, so that the staged row loads
-          // below wait on L2 rather than on DRAM (on longer shares the extra
-          // requests slowed the bandwidth-bound dense levels)
-          const uint32_t* rb = g.values + static_cast<size_t>(u) * Qg + s0;
-          uint32_t lines = cm & gch;
-          while (lines) {
-            prefetch_l2(rb + 32 * (__ffs(lines) - 1));
-            lines &= lines - 1;
-          }
         }
       }
-      pairs += static_cast<unsigned long long>(cnt);
-      const unsigned lm = __ballot_sync(kFull, cnt > 0);
-      if (cnt > 0)
-        stage[__popc(lm & ((1u << lane) - 1u))] = make_int4(u, static_cast<int>(wb), k, static_cast<int>(cm));
+      if (f0 + 32 < total) load_batch(f0 + 32);
+      const bool live = cm != 0;
+      const unsigned lm = __ballot_sync(kFull, live);
+      if (lm == 0) continue;
+      pairs += (bounds || screened) ? static_cast<unsigned long long>(__popc(cm)) << 5
+                                    : (live ? static_cast<unsigned long long>(qs) : 0ULL);
+      // the vertex's own row goes before its first live in-edge
+      const unsigned lb = lm & below;
+      const int kp = __shfl_sync(kFull, k, lb ? 31 - __clz(lb) : lane);
+      const bool first = live && k != (lb ? kp : cur_k);
+      const unsigned fm = __ballot_sync(kFull, first);
+      const int pos = __popc(lb) + __popc(fm & (below | (1u << lane)));
+      const int32_t vk = __shfl_sync(kFull, v, k);
+      if (live) stage[pos] = make_int4(u, static_cast<int>(wb), k, static_cast<int>(cm));
+      if (first) stage[pos - 1] = make_int4(vk, 0, ~k, static_cast<int>(gch));
       __syncwarp();
-      const int n = __popc(lm);
+      const int n = __popc(lm) + __popc(fm);
       for (int i = 0; i < n; i += S) {
         int4 ed[S];
-#pragma unroll
-        for (int t = 0; t < S; ++t) ed[t] = stage[i + t < n ? i + t : i];
         uint32_t cur[S][GV::kSlots];
 #pragma unroll
         for (int t = 0; t < S; ++t) {
+          ed[t] = stage[i + t < n ? i + t : i];
           const uint32_t* row = lanebase + static_cast<size_t>(ed[t].x) * Qg;
 #pragma unroll
           for (int r = 0; r < P; ++r) {
-            if (i + t < n && ((pmask >> r) & 1u) && chunk_live<W>(static_cast<uint32_t>(ed[t].w), r, lane)) {
+            if (i + t < n && ((pmask >> r) & 1u) &&
+                chunk_live<W>(static_cast<uint32_t>(ed[t].w), r, lane)) {
               load_vec_cg<E>(row + 32 * E * r, &cur[t][r * E]);
             } else {
 #pragma unroll
@@ -2719,80 +2797,23 @@ __device__ __forceinline__ void sssp_pull_light_chunks(const GroupDev& g, const 
 #pragma unroll
         for (int t = 0; t < S; ++t) {
           if (i + t >= n) break;  // uniform
-          if (ed[t].z != cur_k) {  // uniform: a new vertex starts
-            if (cur_k >= 0) flush_row();
-            cur_k = ed[t].z;
+          if (ed[t].z < 0) {      // uniform: a new vertex starts
+            if (cur_k >= 0) commit();
+            cur_k = ~ed[t].z;
+            cur_v = ed[t].x;
+#pragma unroll
+            for (int j = 0; j < GV::kSlots; ++j) own[j] = best[j] = cur[t][j];
+          } else {
+            relax_min_row<WK>(best, cur[t], static_cast<uint32_t>(ed[t].y));
           }
-          relax_min_row<WK>(best, cur[t], static_cast<uint32_t>(ed[t].y));
         }
       }
       __syncwarp();
     }
-    if (cur_k >= 0) flush_row();
-    __syncthreads();
-    // commit: warp wib takes vertices wib, wib + 8, ...
-    for (int k = wib; k < nv; k += kWarpsPerBlock) {
-      const int32_t v = s_v[k];
-      uint32_t* row = g.values + static_cast<size_t>(v) * Qg + s0 + lane * E;
-      const uint32_t* srow = s_best + k * R + lane * E;
-      uint32_t imp = 0;
-#pragma unroll
-      for (int r = 0; r < P; ++r) {
-        if (!((pmask >> r) & 1u)) continue;
-        uint32_t o[E], b[E], nvv[E];
-        load_vec<E>(row + 32 * E * r, o);
-        if constexpr (E == 4) {
-          const uint4 x = *reinterpret_cast<const uint4*>(srow + 32 * E * r);
-          b[0] = x.x; b[1] = x.y; b[2] = x.z; b[3] = x.w;
-        } else {
-          const uint2 x = *reinterpret_cast<const uint2*>(srow + 32 * E * r);
-          b[0] = x.x; b[1] = x.y;
-        }
-        uint32_t bits = 0;
-#pragma unroll
-        for (int q = 0; q < E; ++q) {
-          const bool up = ((smask >> (r * E + q)) & 1u) && b[q] < o[q];
-          nvv[q] = up ? b[q] : o[q];
-          bits |= static_cast<uint32_t>(up) << q;
-        }
-        if (bits) store_vec<E>(row + 32 * E * r, nvv);
-        imp |= bits << (r * E);
-      }
-      if (lane == 0 && sl == 0) ++verts;
-      if (!__any_sync(kFull, imp != 0)) continue;
-      improved += __popc(imp);
-      uacc |= imp;
-      uint64_t words[P];
-      gather_vec_words<W>(imp, lane, words);
-#pragma unroll
-      for (int r = 0; r < P; ++r) {
-        if (words[r]) {
-          const int wi = ((32 * r + lane) * E) >> 6;
-          lv.fnext[static_cast<size_t>(v) * WF + sl * W + wi] |= words[r];
-        }
-      }
-      bool fresh;
-      if constexpr (WF > W) {
-        int old = 0;
-        if (lane == 0) old = atomicMax(g.stamp + v, lv.level + 1);
-        fresh = __shfl_sync(kFull, old, 0) < lv.level + 1;
-      } else {
-        fresh = g.stamp[v] < lv.level + 1;  // uniform
-        __syncwarp();
-        if (fresh && lane == 0) g.stamp[v] = lv.level + 1;
-      }
-      ap.add<OT>(fresh && lane == 0, v, G, lv, lane);
-    }
-    __syncthreads();
+    if (cur_k >= 0) commit();
   }
-  ap.flush<OT>(G, lv, lane);
-  {
-    uint64_t words[P];
-    gather_vec_words<W>(uacc, lane, words);
-#pragma unroll
-    for (int r = 0; r < P; ++r)
-      if (words[r]) atomic_or64(lv.nactive + sl * W + (((32 * r + lane) * E) >> 6), words[r]);
-  }
+  if (pend_n > 0) flush_pending();
+  if (sl >= 0) flush_union_bits();
   warp_add(improved, &g.ctl->lc.improved, lane);
   warp_add(pairs, &g.ctl->lc.sssp_pairs, lane);
   warp_add(scanned, &g.ctl->lc.spull_edges, lane);
@@ -2800,10 +2821,9 @@ __device__ __forceinline__ void sssp_pull_light_chunks(const GroupDev& g, const 
 }
 
 template <int W, typename OT, int WK, int WF = W>
-__global__ void __launch_bounds__(kBlock, 3) k_sssp_pull_chunked(GroupDev g, DevGraph G) {
-  __shared__ GatherChunkSmem<W> sm;
-  sssp_pull_light_chunks<W, OT, WK, WF>(g, G, blockIdx.x, gridDim.x,
-                                        WF > W ? static_cast<int>(blockIdx.y) : 0, sm);
+__global__ void __launch_bounds__(kBlock, 3) k_sssp_pull_rows(GroupDev g, DevGraph G) {
+  __shared__ GatherRowSmem sm;
+  sssp_pull_light_rows<W, OT, WK, WF>(g, G, blockIdx.x, gridDim.x, sm);
 }
 
 // Gather level (vectorised), heavy vertices: CTA per 2048-edge chunk, warps
@@ -2831,7 +2851,7 @@ __device__ __forceinline__ void sssp_pull_heavy_chunks(const GroupDev& g, const 
   constexpr int E = GV::kElem;
   constexpr int C = 2 * W;
   const LevelCtl* ctl = g.ctl;
-  if (ctl->done || ctl->sdir != kDirPull || G.n_pheavy == 0) return;
+  if (ctl->done || ctl->sdir != kDirPull || G.n_sheavy == 0) return;
   const LevelView lv = level_view(g);
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
@@ -2852,12 +2872,12 @@ __device__ __forceinline__ void sssp_pull_heavy_chunks(const GroupDev& g, const 
   unsigned scanned = 0;
   // every heavy vertex is gathered once per launch (all its chunks)
   if (bid == 0 && threadIdx.x == 0)
-    atomicAdd(&g.ctl->lc.spull_vertices, static_cast<unsigned long long>(G.n_pheavy));
-  for (int64_t ch = bid; ch < G.pheavy_chunks; ch += nblk) {
+    atomicAdd(&g.ctl->lc.spull_vertices, static_cast<unsigned long long>(G.n_sheavy));
+  for (int64_t ch = bid; ch < G.sheavy_chunks; ch += nblk) {
     // the chunk's vertex and edge range: independent loads, no search
-    const int32_t v = G.pheavy[G.pheavy_ch[ch]];
-    const int64_t cb = G.pheavy_cb[ch];
-    const int64_t ce = G.pheavy_ce[ch];
+    const int32_t v = G.sheavy[G.sheavy_ch[ch]];
+    const int64_t cb = G.sheavy_cb[ch];
+    const int64_t ce = G.sheavy_ce[ch];
     for (int i = threadIdx.x; i < C * 32; i += blockDim.x) s_best[i] = 0xffffffffu;
     if (bounds && threadIdx.x < C) sm.hi[threadIdx.x] = g.bhi[static_cast<size_t>(v) * C + threadIdx.x];
     __syncthreads();
@@ -2923,15 +2943,6 @@ __device__ __forceinline__ int32_t decide_dir(const LevelCtl* ctl, unsigned long
   if (ctl->mode == 1) return kDirPull;   // CGP_MODE_PULL
   return (edges >= ctl->pull_edge_threshold || count >= ctl->pull_vertex_threshold)
              ? kDirPull : kDirPush;
-}
-
-// SSSP direction of the next level: gather once the frontier's edges reach
-// the threshold (dense levels), scatter otherwise.
-template <int W>
-__device__ __forceinline__ bool any_bits(const uint64_t* m) {
-  uint64_t a = 0;
-  for (int i = 0; i < W; ++i) a |= m[i];
-  return a != 0;
 }
 
 // Group-wide SSSP direction of a level whose frontier has `count` vertices
@@ -3299,7 +3310,7 @@ union TraverseSmem {
   SsspPushSmem<kSssp ? W : 1> sssp_push;
   SsspHeavySmem<kSssp ? W : 1> sssp_heavy;
   GatherHeavySmem<kSssp ? W : 1> gather_heavy;
-  GatherChunkSmem<kSssp ? (W < 4 ? W : 4) : 1> gather_light;
+  GatherRowSmem gather_light;
 };
 
 // Up to `levels` whole levels in one cooperative launch: the phases that are
@@ -3366,22 +3377,11 @@ __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev 
       }
       if (gather) {
         // heavy vertices first: the light ones read their lowered distances
-        if (G.n_pheavy > 0) {
+        if (G.n_sheavy > 0) {
           sssp_pull_heavy_chunks<W, OT, WK, (W <= 4 ? 3 : 0)>(g, G, bid, nblk, sm.gather_heavy);
           if (!bar.wait()) return;
         }
-        constexpr int WS = W < 4 ? W : 4;  // words per slice
-        constexpr unsigned kSlices = W / WS;
-        const unsigned per = nblk / kSlices;
-        if (per == 0) {
-          for (unsigned sl = 0; sl < kSlices; ++sl) {
-            sssp_pull_light_chunks<WS, OT, WK, W>(g, G, bid, nblk, static_cast<int>(sl), sm.gather_light);
-            __syncthreads();
-          }
-        } else if (bid < per * kSlices) {
-          sssp_pull_light_chunks<WS, OT, WK, W>(g, G, bid / kSlices, per,
-                                                static_cast<int>(bid % kSlices), sm.gather_light);
-        }
+        sssp_pull_light_rows<(W < 4 ? W : 4), OT, WK, W>(g, G, bid, nblk, sm.gather_light);
       }
       if (ctl->chunk_dir) {
         if (!bar.wait()) return;

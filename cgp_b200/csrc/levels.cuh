@@ -88,7 +88,7 @@ int enqueue_level_t(const LevelLaunch& L, cudaStream_t s) {
       if (kt) kt->mark(kClassSsspPull, s);
       // heavy vertices first: the light vertices' gathers of the same level
       // then read the hubs' lowered distances (the level is Gauss-Seidel)
-      if (L.G.n_pheavy) {
+      if (L.gvec ? L.G.n_sheavy : L.G.n_pheavy) {
         if (L.gvec && W <= 4) {
           // whole-row and chunk-skipping variants; each returns at once on the
           // other's levels
@@ -104,14 +104,14 @@ int enqueue_level_t(const LevelLaunch& L, cudaStream_t s) {
       }
       if constexpr (W <= 4) {
         if (L.gvec && L.lchunks) {
-          k_sssp_pull_chunked<W, OT, WK><<<L.gr.gather_chunked, kBlock, 0, s>>>(L.g, L.G);
+          k_sssp_pull_rows<W, OT, WK><<<L.gr.gather_rows, kBlock, 0, s>>>(L.g, L.G);
         } else if (L.gvec) {
           k_sssp_pull_vec<W, OT, WK><<<L.gr.gather_vec, kBlock, 0, s>>>(L.g, L.G);
         } else {
           k_sssp_pull<W, OT, WK><<<L.gr.gather, kBlock, 0, s>>>(L.g, L.G);
         }
       } else if (L.gvec && L.lchunks) {
-        k_sssp_pull_chunked<4, OT, WK, W><<<dim3(L.gr.gather_chunked, W / 4), kBlock, 0, s>>>(L.g, L.G);
+        k_sssp_pull_rows<4, OT, WK, W><<<L.gr.gather_rows, kBlock, 0, s>>>(L.g, L.G);
       } else if (L.gvec) {
         k_sssp_pull_vec<W, OT, WK><<<L.gr.gather_vec, kBlock, 0, s>>>(L.g, L.G);
       } else {
@@ -136,17 +136,12 @@ int enqueue_level_t(const LevelLaunch& L, cudaStream_t s) {
 template <int W, typename OT, int DEPTH, int WK>
 Grids grids_t(int sms) {
   static int tile = 0, heavy = 0, dense = 0, dense2 = 0, gather = 0, gather_heavy = 0;
-  static int gather_vec = 0, gather_heavy_vec = 0, gather_chunked = 0, gather_heavy_vec2 = 0;
+  static int gather_vec = 0, gather_heavy_vec = 0, gather_rows = 0, gather_heavy_vec2 = 0;
   static int bfs_chunked = 0, bfs_mid = 0;
   if (tile == 0) {
     bfs_chunked = occupancy_grid(k_bfs_pull_chunked<W, OT, DEPTH>, sms);
     bfs_mid = occupancy_grid(k_bfs_pull_mid<W, OT, DEPTH>, sms);
-    if constexpr (W <= 4) {
-      gather_chunked = occupancy_grid(k_sssp_pull_chunked<W, OT, WK>, sms);
-    } else {
-      // slices of 4 words, all resident at once: x blocks per slice
-      gather_chunked = std::max(1, occupancy_grid(k_sssp_pull_chunked<4, OT, WK, W>, sms) / (W / 4));
-    }
+    gather_rows = occupancy_grid(k_sssp_pull_rows<(W < 4 ? W : 4), OT, WK, W>, sms);
     gather_vec = occupancy_grid(k_sssp_pull_vec<W, OT, WK>, sms);
     gather_heavy_vec = occupancy_grid(k_sssp_pull_heavy_vec<W, OT, WK, (W <= 4 ? 1 : 0)>, sms);
     gather_heavy_vec2 = occupancy_grid(k_sssp_pull_heavy_vec<W, OT, WK, 2>, sms);
@@ -171,7 +166,7 @@ Grids grids_t(int sms) {
   g.gather_heavy = gather_heavy;
   g.gather_vec = gather_vec;
   g.gather_heavy_vec = gather_heavy_vec;
-  g.gather_chunked = gather_chunked;
+  g.gather_rows = gather_rows;
   g.gather_heavy_vec2 = gather_heavy_vec2;
   g.bfs_chunked = bfs_chunked;
   g.bfs_mid = bfs_mid;

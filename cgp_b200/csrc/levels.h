@@ -20,7 +20,7 @@ struct Grids {
   int gather_heavy;
   int gather_vec;
   int gather_heavy_vec;
-  int gather_chunked;
+  int gather_rows;
   int gather_heavy_vec2;
   int bfs_chunked;
   int bfs_mid;
@@ -36,7 +36,7 @@ struct LevelLaunch {
   bool bounds = false;  // gather levels may screen by bounds
   bool spull;        // SSSP gather kernels are part of the level
   bool gvec;         // rows allow the vectorised gather (alignment, width)
-  bool lchunks;      // light vertices gathered in CTA chunks (in 4-word slices above W = 4)
+  bool lchunks;      // light vertices gathered by items (in 4-word slices above W = 4)
   int dense_unroll;  // edges per step of the dense SSSP kernel (1 or 2)
   KernelTimer* kt;   // per-class event timing (non-graph runs only)
   bool heavy_push = false;                // heavy-queue push kernels are part of a level

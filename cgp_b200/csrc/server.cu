@@ -481,6 +481,15 @@ int cgp_server::pick_slot(int* group, int32_t kind) {
       }
       if (gsel < 0 && !gr.cohort && gr.active == 0) gsel = gi;
     }
+    // While other groups run, a new cohort waits for a burst of arrivals to
+    // end (0.5 ms without one, 5 ms at most): requests of one burst that come
+    // a level apart would otherwise be split over two cohorts, and the second
+    // part waits for a whole cohort to finish.
+    if (gsel >= 0 && groups[gsel].nadmit == 0 && active > groups[gsel].active) {
+      const double t = now_ms();
+      if (t - reqs[pending.back()].t_submit < 0.5 && t - reqs[pending.front()].t_submit < 5.0)
+        gsel = -1;
+    }
     *group = gsel;
     if (gsel < 0) return -1;
     const ServeGroup& gr = groups[gsel];
