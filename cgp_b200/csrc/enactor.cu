@@ -236,7 +236,7 @@ cgp_status cgp_enactor_read_values(cgp_enactor* e, void* out, int32_t out_layout
     om.qmap_contiguous = 1;
     group_write_output(e->g, e->ws.get(), e->spec, om, qmajor, e->stream);
     if (!e->wcc_slots.empty()) {
-      e->ws->wcc.ensure(static_cast<size_t>(V) * 4);
+      e->ws->wcc.ensure(static_cast<size_t>(V + 1) * 4);
       wcc_labels(e->g, e->ws->wcc.as<uint32_t>(), e->stream);
       for (int i : e->wcc_slots) broadcast_labels(e->ws->wcc.as<uint32_t>(), V, om, i, e->stream);
     }

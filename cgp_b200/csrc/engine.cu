@@ -1176,10 +1176,10 @@ cgp_status cgp_batch_run(cgp_graph* graph, const cgp_query* queries, int32_t nq,
     t_level_ms.clear();
     if (!wcc_idx.empty()) {
       if (kt) kt->mark(kClassWcc, s);
-      ws->wcc.ensure(static_cast<size_t>(V) * 4);
+      ws->wcc.ensure(static_cast<size_t>(V + 1) * 4);
       wcc_labels(g, ws->wcc.as<uint32_t>(), s);
       for (int i : wcc_idx) broadcast_labels(ws->wcc.as<uint32_t>(), V, om, i, s);
-      launches += 3 + wcc_idx.size();
+      launches += 9 + (g->symmetric ? 0 : 1) + wcc_idx.size();
       if (kt) kt->mark(-1, s);
     }
     // Traversal groups of up to 64*W queries, in submission order.  A batch

@@ -231,7 +231,8 @@ void group_write_output(GraphImpl* g, Workspace* ws, GroupSpec& spec,
                         dev::OutMap om, int query_major, cudaStream_t s);
 int choose_words(int n, int requested);
 int64_t group_state_bytes(const GraphImpl* g, int W, int Qg, int depth_mode);
-// WCC: minimum vertex id of each weak component into `labels` (device).
+// WCC: minimum vertex id of each weak component into labels[0 .. V) (device,
+// V + 1 entries).
 void wcc_labels(GraphImpl* g, uint32_t* labels, cudaStream_t s);
 // Writes labels[v] into global column `col` of the output mapping.
 void broadcast_labels(const uint32_t* labels, int64_t V, dev::OutMap om, int col,

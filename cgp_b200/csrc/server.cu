@@ -358,7 +358,7 @@ void cgp_server::finish_wcc(std::vector<uint64_t>& tickets) {
   if (tickets.empty()) return;
   cudaStream_t s = wcc_ws->stream;
   if (!wcc_ready) {
-    wcc_ws->wcc.ensure(static_cast<size_t>(g->V) * 4);
+    wcc_ws->wcc.ensure(static_cast<size_t>(g->V + 1) * 4);
     wcc_labels(g, wcc_ws->wcc.as<uint32_t>(), s);
     wcc_ready = true;
   }
