@@ -200,8 +200,10 @@ struct OutMap {
   uint32_t* out;
   int64_t sv;
   int64_t sq;
-  const int32_t* qmap;
-  int32_t qmap_contiguous;  // qmap[q] == qmap[0] + q for every q
+  const int32_t* qmap;  // nullptr: global query q0 + q
+  int32_t q0;
+
+  __device__ __forceinline__ int64_t col(int q) const { return qmap != nullptr ? qmap[q] : q0 + q; }
 };
 
 template <typename OT>

@@ -223,17 +223,12 @@ cgp_status cgp_enactor_read_values(cgp_enactor* e, void* out, int32_t out_layout
       e->ws->stage.ensure(static_cast<size_t>(V) * nq * 4);
       dout = e->ws->stage.as<uint32_t>();
     }
-    std::vector<int32_t> qmap(nq);
-    for (int i = 0; i < nq; ++i) qmap[i] = i;
-    e->ws->qmap.ensure(static_cast<size_t>(nq) * 4);
-    ck(cudaMemcpyAsync(e->ws->qmap.p, qmap.data(), nq * 4, cudaMemcpyHostToDevice, e->stream),
-       "upload query map");
     OutMap om;
     om.out = dout;
     om.sv = qmajor ? 1 : nq;
     om.sq = qmajor ? V : 1;
-    om.qmap = e->ws->qmap.as<int32_t>();
-    om.qmap_contiguous = 1;
+    om.qmap = nullptr;
+    om.q0 = 0;
     group_write_output(e->g, e->ws.get(), e->spec, om, qmajor, e->stream);
     if (!e->wcc_slots.empty()) {
       e->ws->wcc.ensure(static_cast<size_t>(V + 1) * 4);

@@ -83,16 +83,18 @@ bool DevBuf::offer(size_t need, bool* moved) {
 Workspace::Workspace(int dev) : device(dev) {
   ck(cudaHostAlloc(reinterpret_cast<void**>(&hctl), 2 * sizeof(LevelCtl), cudaHostAllocDefault),
      "cudaHostAlloc(ctl)");
-  ck(cudaHostAlloc(reinterpret_cast<void**>(&hslots), kMaxWords * 64 * sizeof(SlotDev),
-                   cudaHostAllocDefault),
-     "cudaHostAlloc(slots)");
+  const size_t start_bytes = kSlotsOffset + kMaxWords * 64 * sizeof(SlotDev);
+  ck(cudaHostAlloc(reinterpret_cast<void**>(&hstart), start_bytes, cudaHostAllocDefault),
+     "cudaHostAlloc(start)");
+  ck(cudaEventCreateWithFlags(&uploaded, cudaEventDisableTiming), "cudaEventCreate");
+  ck(cudaEventCreate(&t0), "cudaEventCreate");
+  ck(cudaEventCreate(&t1), "cudaEventCreate");
   ck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
   ck(cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking), "cudaStreamCreate");
   ck(cudaStreamCreateWithFlags(&copy, cudaStreamNonBlocking), "cudaStreamCreate");
   ck(cudaEventCreateWithFlags(&out_ready, cudaEventDisableTiming), "cudaEventCreate");
   for (auto& e : ev) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-  ctl.ensure(sizeof(LevelCtl));
-  slots.ensure(kMaxWords * 64 * sizeof(SlotDev));
+  ctl.ensure(start_bytes);
 }
 
 void Workspace::clear_graphs() {
@@ -103,7 +105,10 @@ void Workspace::clear_graphs() {
 Workspace::~Workspace() {
   clear_graphs();
   if (hctl) cudaFreeHost(hctl);
-  if (hslots) cudaFreeHost(hslots);
+  if (hstart) cudaFreeHost(hstart);
+  if (uploaded) cudaEventDestroy(uploaded);
+  if (t0) cudaEventDestroy(t0);
+  if (t1) cudaEventDestroy(t1);
   if (stream) cudaStreamDestroy(stream);
   if (capture) cudaStreamDestroy(capture);
   if (copy) cudaStreamDestroy(copy);
@@ -399,6 +404,7 @@ GroupSpec make_group(const cgp_query* q, int n, int W, int depth_mode) {
     g.slots[i].base = 0;
     if (q[i].kind == CGP_KIND_SSSP) g.has_sssp = true;
     if (q[i].kind == CGP_KIND_BFS || q[i].kind == CGP_KIND_KHOP) g.has_bfs = true;
+    if (q[i].kind == CGP_KIND_WCC) g.has_wcc = true;
   }
   if (depth_mode == CGP_DEPTH_PLANES && !g.has_sssp) g.depth_mode = kDepthPlanes;
   else if (depth_mode == CGP_DEPTH_DIRECT || g.has_sssp) g.depth_mode = kDepthDirect;
@@ -411,7 +417,8 @@ void pad_rows(GroupSpec& g) {
   g.slots.resize(g.Qg, dev::SlotDev{-1, -1, 0, 0});
 }
 
-static constexpr int kInitialPlanes = 8;
+static constexpr int kInitialPlanes = 8;  // depth planes allocated at first
+static constexpr int kStartPlanes = 4;    // ... and zeroed: depths up to 15
 
 int64_t group_state_bytes(const GraphImpl* g, int W, int Qg, int depth_mode) {
   const int64_t V = g->V;
@@ -462,7 +469,7 @@ GroupDev group_dev(Workspace* ws, const GroupSpec& spec, bool profiles) {
   g.hq_cap = static_cast<int64_t>(ws->hq_start.bytes / sizeof(int64_t));
   g.ctl = ws->ctl.as<LevelCtl>();
   g.prof = profiles ? ws->prof.as<LevelProfile>() : nullptr;
-  g.slots = ws->slots.as<SlotDev>();
+  g.slots = ws->slots_dev();
   g.Qg = spec.Qg;
   return g;
 }
@@ -499,6 +506,7 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
   const int64_t hth = heavy_threshold(o);
   const HeavyPair& hp = g->heavy_for(hth);
   bool moved = false;
+  spec.depth_bits = 0;
   const size_t mask_bytes = static_cast<size_t>(V) * W * 8;
   try {
     moved |= ws->visited.ensure(mask_bytes);
@@ -539,24 +547,35 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
     ws->generation++;
     ws->clear_graphs();
   }
-  ck(cudaMemsetAsync(ws->visited.p, 0, mask_bytes, s), "memset visited");
-  ck(cudaMemsetAsync(ws->fbuf0.p, 0, mask_bytes, s), "memset frontier");
-  ck(cudaMemsetAsync(ws->fbuf1.p, 0, mask_bytes, s), "memset next frontier");
-  ck(cudaMemsetAsync(ws->stamp.p, 0xff, static_cast<size_t>(V) * 4, s), "memset stamp");
-  ck(cudaMemsetAsync(ws->hacc.p, 0, static_cast<size_t>(std::max(1, hp.pheavy.n)) * W * 8, s),
-     "memset hacc");
-  ck(cudaMemsetAsync(ws->fsum.p, 0, static_cast<size_t>(V) * 8, s), "memset fsum");
-  if (spec.depth_mode == kDepthPlanes)
-    ck(cudaMemsetAsync(ws->planes.p, 0, static_cast<size_t>(kInitialPlanes) * mask_bytes, s),
-       "memset planes");
+  const uint32_t sssp_inf = g->weight_kind == CGP_WEIGHT_F32 ? 0x7f800000u : 0xffffffffu;
+  uint32_t* values = group_dev(ws, spec, false).values;
+  // one marker for every slot: all of one kind, or the serving layout
+  const bool one_kind = !(spec.has_bfs && spec.has_sssp) && !spec.has_wcc;
+  uint32_t marker = spec.uniform_inf;
+  if (marker == 0 && one_kind) marker = spec.has_sssp ? sssp_inf : 0x7fffffffu;
+  // only 4 planes are zeroed: group_enact adds planes when a depth needs them
+  const size_t planes_bytes = static_cast<size_t>(kStartPlanes) * mask_bytes;
+  FillList fill;
+  bool fill_late = false;
+  fill.add(ws->visited.p, mask_bytes, 0);
+  fill.add(ws->fbuf0.p, mask_bytes, 0);
+  fill.add(ws->fbuf1.p, mask_bytes, 0);
+  fill.add(ws->stamp.p, static_cast<size_t>(V) * 4, 0xffffffffu);
+  fill.add(ws->hacc.p, static_cast<size_t>(std::max(1, hp.pheavy.n)) * W * 8, 0);
+  fill.add(ws->fsum.p, static_cast<size_t>(V) * 8, 0);
+  if (spec.depth_mode == kDepthPlanes) {
+    fill.add(ws->planes.p, planes_bytes, 0);
+  } else if (marker != 0 && reinterpret_cast<uintptr_t>(values) % 16 == 0) {
+    fill.add(values, static_cast<size_t>(V) * spec.Qg * 4, marker);
+  } else {
+    fill_late = true;
+  }
 
-  // slots and control block
-  ck(cudaStreamSynchronize(s), "sync before slot upload");  // hslots/hctl are reused
-  std::memcpy(ws->hslots, spec.slots.data(), spec.slots.size() * sizeof(SlotDev));
-  ck(cudaMemcpyAsync(ws->slots.p, ws->hslots, spec.slots.size() * sizeof(SlotDev),
-                     cudaMemcpyHostToDevice, s),
-     "upload slots");
-  LevelCtl& c = ws->hctl[0];
+  // slots and control block, one upload (the last one has left the buffer)
+  ck(cudaEventSynchronize(ws->uploaded), "slot upload");
+  std::memcpy(ws->hstart + Workspace::kSlotsOffset, spec.slots.data(),
+              spec.slots.size() * sizeof(SlotDev));
+  LevelCtl& c = *reinterpret_cast<LevelCtl*>(ws->hstart);
   std::memset(&c, 0, sizeof(c));
   for (int q = 0; q < spec.Qg; ++q) {
     const int k = spec.slots[q].kind;
@@ -570,7 +589,7 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
   int mode = o.traversal_mode;
   if (!g->can_gather()) mode = CGP_MODE_PUSH;
   c.mode = mode;
-  c.num_planes = spec.depth_mode == kDepthPlanes ? kInitialPlanes : 0;
+  c.num_planes = spec.depth_mode == kDepthPlanes ? kStartPlanes : 0;
   c.profile_cap = o.profile_iterations ? kProfileCap : 0;
   c.pull_vertex_threshold = static_cast<unsigned long long>(
       std::max(1.0, o.pull_frontier_ratio * static_cast<double>(V)));
@@ -588,17 +607,21 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
                               ? static_cast<unsigned long long>(
                                     std::max(1.0, o.sssp_pull_pair_ratio * static_cast<double>(g->E)))
                               : 0ULL;
-  ck(cudaMemcpyAsync(ws->ctl.p, &c, sizeof(LevelCtl), cudaMemcpyHostToDevice, s), "upload ctl");
-
-  const uint32_t sssp_inf = g->weight_kind == CGP_WEIGHT_F32 ? 0x7f800000u : 0xffffffffu;
-  if (spec.depth_mode != kDepthPlanes) {
-    int blocks = g->num_sms * 8;
-    k_fill_values<<<blocks, kBlock, 0, s>>>(group_dev(ws, spec, false).values,
-                                            ws->slots.as<SlotDev>(), spec.Qg, V, sssp_inf,
-                                            spec.uniform_inf);
-    ck(cudaGetLastError(), "fill values");
+  ck(cudaMemcpyAsync(ws->ctl.p, ws->hstart,
+                     Workspace::kSlotsOffset + spec.slots.size() * sizeof(SlotDev),
+                     cudaMemcpyHostToDevice, s), "upload ctl");
+  ck(cudaEventRecord(ws->uploaded, s), "event");
+  int64_t words = 0;
+  for (int i = 0; i < fill.n; ++i) words += fill.span[i].words;
+  const int blocks = static_cast<int>(std::min<int64_t>(g->num_sms * 8, words / (4 * kBlock) + 1));
+  k_fill_spans<<<blocks, kBlock, 0, s>>>(fill);
+  spec.launches++;
+  if (fill_late) {  // per-slot markers: reads the uploaded slots
+    k_fill_values<<<g->num_sms * 8, kBlock, 0, s>>>(values, ws->slots_dev(), spec.Qg, V, sssp_inf,
+                                                    spec.uniform_inf);
     spec.launches++;
   }
+  ck(cudaGetLastError(), "group start");
   Dispatch d = dispatch(W, g->offset_bytes, spec.depth_mode, g->weight_kind);
   d.seed(group_dev(ws, spec, o.profile_iterations != 0), g->dev_graph(hth), s);
   ck(cudaGetLastError(), "seed");
@@ -757,6 +780,7 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
   int enqueued = 0;
   int chunk = 0;
   LevelCtl* snap = ws->hctl;
+  int last = -1;  // snapshot of the last levels enqueued
   // A run to convergence without per-level timing is one device-looped graph:
   // the host waits once.  (The launch count of such a run is that of one
   // level; the per-level count is reported with the level count below.)
@@ -765,8 +789,9 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
   if (device_loop) {
     const int per_level = enqueue_levels(g, ws, spec, o, s, -1, nullptr);
     ck(cudaStreamSynchronize(s), "device level loop");
-    LevelCtl c;
-    ck(cudaMemcpy(&c, ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost), "read ctl");
+    ck(cudaMemcpy(&snap[0], ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost), "read ctl");
+    last = 0;
+    const LevelCtl& c = snap[0];
     spec.launches += static_cast<uint64_t>(per_level) * static_cast<uint64_t>(std::max(1, c.level));
   }
   for (;;) {
@@ -787,6 +812,7 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
     enqueued += n;
     ck(cudaMemcpyAsync(&snap[chunk & 1], ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost, s),
        "read ctl");
+    last = chunk & 1;
     ck(cudaEventRecord(ws->ev[chunk & 1], s), "event");
     bool stop = false;
     if (kt) {
@@ -807,38 +833,48 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
     if (stop) break;
     ++chunk;
   }
-  ck(cudaStreamSynchronize(s), "level loop");
-  LevelCtl c;
-  ck(cudaMemcpy(&c, ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost), "read ctl");
+  if (!fused || last < 0) ck(cudaStreamSynchronize(s), "level loop");
+  if (last < 0) {
+    ck(cudaMemcpy(&snap[0], ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost), "read ctl");
+    last = 0;
+  }
+  LevelCtl c = snap[last];
   if (c.status & kStatusBarrier)
     throw ApiError{CGP_ERR_DEVICE, "grid barrier timed out at level " + std::to_string(c.level)};
   if (c.status & kStatusLevelCap)
     throw ApiError{CGP_ERR_DEVICE, "traversal did not converge within " +
                                        std::to_string(c.level) + " levels"};
   if (c.done == 2 && (c.status & kStatusPlanesExhausted)) {
-    // Deeper than the depth planes can hold: grow them and resume.
+    // Deeper than the depth planes can hold: add planes and resume.
     const size_t mask_bytes = static_cast<size_t>(g->V) * spec.W * 8;
     const int K = c.num_planes;
-    const int K2 = std::min(kMaxPlanes, K + 8);
+    const int K2 = std::min(kMaxPlanes, K < kInitialPlanes ? kInitialPlanes : K + 8);
     if (K2 == K) throw ApiError{CGP_ERR_DEVICE, "BFS depth exceeds 2^24 levels"};
-    DevBuf bigger;
-    bigger.ensure(static_cast<size_t>(K2) * mask_bytes);
-    ck(cudaMemcpyAsync(bigger.p, ws->planes.p, static_cast<size_t>(K) * mask_bytes,
-                       cudaMemcpyDeviceToDevice, s), "grow planes");
-    ck(cudaMemsetAsync(static_cast<char*>(bigger.p) + static_cast<size_t>(K) * mask_bytes, 0,
+    if (static_cast<size_t>(K2) * mask_bytes > ws->planes.bytes) {
+      DevBuf bigger;
+      bigger.ensure(static_cast<size_t>(K2) * mask_bytes);
+      ck(cudaMemcpyAsync(bigger.p, ws->planes.p, static_cast<size_t>(K) * mask_bytes,
+                         cudaMemcpyDeviceToDevice, s), "grow planes");
+      ck(cudaStreamSynchronize(s), "grow planes");
+      std::swap(ws->planes.p, bigger.p);
+      std::swap(ws->planes.bytes, bigger.bytes);
+      ws->generation++;
+      ws->clear_graphs();
+    }
+    ck(cudaMemsetAsync(static_cast<char*>(ws->planes.p) + static_cast<size_t>(K) * mask_bytes, 0,
                        static_cast<size_t>(K2 - K) * mask_bytes, s), "zero planes");
-    std::swap(ws->planes.p, bigger.p);
-    std::swap(ws->planes.bytes, bigger.bytes);
-    ck(cudaStreamSynchronize(s), "grow planes");
-    ws->generation++;
-    ws->clear_graphs();
     c.num_planes = K2;
     c.status &= ~kStatusPlanesExhausted;
     c.done = 0;
-    ck(cudaMemcpy(ws->ctl.p, &c, sizeof(LevelCtl), cudaMemcpyHostToDevice), "resume");
-    group_enact(g, ws, spec, o, s, out, max_levels > 0 ? max_levels - enqueued : 0, kt);
-    return;
+    ck(cudaMemcpyAsync(ws->ctl.p, &c, sizeof(LevelCtl), cudaMemcpyHostToDevice, s), "resume");
+    ck(cudaStreamSynchronize(s), "resume");
+    if (max_levels <= 0 || enqueued < max_levels) {
+      group_enact(g, ws, spec, o, s, out, max_levels > 0 ? max_levels - enqueued : 0, kt);
+      return;
+    }
   }
+  spec.depth_bits = 0;  // depths written are at most c.level
+  while (spec.depth_bits < c.num_planes && (c.level >> spec.depth_bits) != 0) ++spec.depth_bits;
   out->iterations = c.level;
   out->push_levels = c.push_levels;
   out->pull_levels = c.pull_levels;
@@ -865,16 +901,13 @@ void group_write_output(GraphImpl* g, Workspace* ws, GroupSpec& spec, OutMap om,
   spec.launches++;
   const dim3 grid(g->num_sms * 8, query_major ? std::min(spec.n, 65535) : 1);
   if (spec.depth_mode == kDepthPlanes) {
-    LevelCtl c;
-    ck(cudaMemcpyAsync(&c, ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost, s), "read ctl");
-    ck(cudaStreamSynchronize(s), "read ctl");
     switch (spec.W) {
-#define CGP_MAT(WW) case WW: k_materialize_planes<WW><<<grid, kBlock, 0, s>>>(ws->visited.as<uint64_t>(), ws->planes.as<uint64_t>(), c.num_planes, g->V, spec.n, om, query_major); break;
+#define CGP_MAT(WW) case WW: k_materialize_planes<WW><<<grid, kBlock, 0, s>>>(ws->visited.as<uint64_t>(), ws->planes.as<uint64_t>(), spec.depth_bits, g->V, spec.n, om, query_major); break;
       CGP_MAT(1) CGP_MAT(2) CGP_MAT(4) CGP_MAT(8) CGP_MAT(16)
 #undef CGP_MAT
     }
   } else {
-    k_copy_values<<<grid, kBlock, 0, s>>>(group_dev(ws, spec, false).values, ws->slots.as<SlotDev>(),
+    k_copy_values<<<grid, kBlock, 0, s>>>(group_dev(ws, spec, false).values, ws->slots_dev(),
                                           g->V, spec.n, spec.Qg, om, query_major);
   }
   ck(cudaGetLastError(), "write output");
@@ -1147,9 +1180,7 @@ cgp_status cgp_batch_run(cgp_graph* graph, const cgp_query* queries, int32_t nq,
     if (o.profile_kernels) kt = std::make_unique<KernelTimer>();
     cudaStream_t s = o.stream ? static_cast<cudaStream_t>(o.stream) : ws->stream;
     auto wall0 = std::chrono::steady_clock::now();
-    cudaEvent_t t0, t1;
-    ck(cudaEventCreate(&t0), "event");
-    ck(cudaEventCreate(&t1), "event");
+    const cudaEvent_t t0 = ws->t0, t1 = ws->t1;
     ck(cudaEventRecord(t0, s), "event");
     const int64_t V = g->V;
     const bool qmajor = out_layout == CGP_LAYOUT_QUERY_MAJOR;
@@ -1164,7 +1195,7 @@ cgp_status cgp_batch_run(cgp_graph* graph, const cgp_query* queries, int32_t nq,
     om.sv = qmajor ? 1 : nq;
     om.sq = qmajor ? V : 1;
     om.qmap = nullptr;
-    om.qmap_contiguous = 0;
+    om.q0 = 0;
     // WCC queries: one union-find pass, labels broadcast to every WCC column
     std::vector<int> wcc_idx, trav_idx;
     for (int i = 0; i < nq; ++i) (queries[i].kind == CGP_KIND_WCC ? wcc_idx : trav_idx).push_back(i);
@@ -1253,16 +1284,21 @@ cgp_status cgp_batch_run(cgp_graph* graph, const cgp_query* queries, int32_t nq,
         if (kt) kt->mark(kClassOutput, s);
         std::vector<int32_t> qmap(n);
         for (int i = 0; i < n; ++i) qmap[i] = (*gp.cls)[gp.begin + i];
-        ws->qmap.ensure(static_cast<size_t>(n) * 4);
-        ck(cudaMemcpyAsync(ws->qmap.p, qmap.data(), static_cast<size_t>(n) * 4,
-                           cudaMemcpyHostToDevice, s), "upload query map");
+        bool run = true;  // consecutive columns
+        for (int i = 1; i < n; ++i) run = run && qmap[i] == qmap[0] + i;
         OutMap m = om;
-        m.qmap = ws->qmap.as<int32_t>();
-        m.qmap_contiguous = 1;
-        for (int i = 1; i < n; ++i) m.qmap_contiguous &= qmap[i] == qmap[0] + i ? 1 : 0;
+        m.q0 = qmap[0];
+        // sized with the group, so that a later batch in another order does
+        // not allocate between its traversal and its output
+        ws->qmap.ensure(static_cast<size_t>(n) * 4);
+        if (!run) {
+          ck(cudaMemcpyAsync(ws->qmap.p, qmap.data(), static_cast<size_t>(n) * 4,
+                             cudaMemcpyHostToDevice, s), "upload query map");
+          m.qmap = ws->qmap.as<int32_t>();
+        }
         group_write_output(g, ws.get(), spec, m, qmajor, s);
         if (kt) kt->mark(-1, s);
-        if (host_out && m.qmap_contiguous && wcc_idx.empty()) {
+        if (host_out && run && wcc_idx.empty()) {
           ck(cudaEventRecord(ws->out_ready, s), "event");
           ck(cudaStreamWaitEvent(ws->copy, ws->out_ready, 0), "wait");
           const size_t q0 = static_cast<size_t>(qmap[0]);
@@ -1311,8 +1347,6 @@ cgp_status cgp_batch_run(cgp_graph* graph, const cgp_query* queries, int32_t nq,
     if (host_out) ck(cudaStreamSynchronize(ws->copy), "copy out");
     float ms = 0;
     cudaEventElapsedTime(&ms, t0, t1);
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
     if (kt) {
       kt->flush();
       std::memset(&t_kernel_profile, 0, sizeof(t_kernel_profile));

@@ -132,9 +132,16 @@ struct Workspace {
   DevBuf visited, fbuf0, fbuf1, list0, list1, stamp, planes, values, hacc, dense, hq_vertex, hq_start;
   DevBuf fsum;  // frontier summary words (uint64 per vertex)
   DevBuf bounds;  // gather bounds: two uint32 per vertex and 32-slot chunk
-  DevBuf ctl, prof, slots, stage, wcc, qmap;
+  DevBuf ctl;   // LevelCtl, then at kSlotsOffset the slots (uploaded together)
+  DevBuf prof, stage, wcc, qmap;
+  static constexpr size_t kSlotsOffset = (sizeof(LevelCtl) + 255) / 256 * 256;
+  dev::SlotDev* slots_dev() const {
+    return reinterpret_cast<dev::SlotDev*>(static_cast<char*>(ctl.p) + kSlotsOffset);
+  }
   LevelCtl* hctl = nullptr;  // pinned, 2 snapshots
-  dev::SlotDev* hslots = nullptr;  // pinned, kMaxWords*64 entries
+  char* hstart = nullptr;    // pinned: control block and slots of a group's start, as in ctl
+  cudaEvent_t uploaded = nullptr;  // hstart's last upload is done
+  cudaEvent_t t0 = nullptr, t1 = nullptr;  // timing of a batch
   cudaStream_t stream = nullptr;
   cudaStream_t capture = nullptr;
   cudaStream_t copy = nullptr;     // device->host result copies overlapping later groups
@@ -193,10 +200,12 @@ struct GroupSpec {
   int depth_mode = dev::kDepthDirect;
   bool has_bfs = false;
   bool has_sssp = false;
+  bool has_wcc = false;                 // enactor slots answered by union-find
   uint32_t* external_values = nullptr;  // caller's device buffer used as working values
   uint32_t uniform_inf = 0;             // nonzero: fill every value with it (serving)
   bool bounds = false;                  // gather levels may screen by bounds
   bool serving = false;                 // the group belongs to a serving loop
+  int depth_bits = 0;                   // depth planes that hold bits, after group_enact
   uint64_t launches = 0;                // kernels enqueued for this group
 };
 

@@ -3436,6 +3436,37 @@ __global__ void k_seed(GroupDev g, DevGraph G) {
 }
 
 // --------------------------------------------------------------- output
+// The buffers a group starts from, each filled with one 32-bit word, in one
+// launch (a traversal of a small graph spent more time in seven memsets than
+// in a level).
+struct FillSpan {
+  uint32_t* p;    // 16-byte aligned
+  int64_t words;
+  uint32_t x;
+};
+struct FillList {
+  FillSpan span[9];
+  int n = 0;
+  void add(void* p, size_t bytes, uint32_t x) {
+    if (bytes == 0) return;
+    span[n].p = static_cast<uint32_t*>(p);
+    span[n].words = static_cast<int64_t>(bytes / 4);
+    span[n++].x = x;
+  }
+};
+
+static __global__ void __launch_bounds__(kBlock) k_fill_spans(FillList f) {
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int i = 0; i < f.n; ++i) {
+    const FillSpan s = f.span[i];
+    const uint4 x = make_uint4(s.x, s.x, s.x, s.x);
+    const int64_t vecs = s.words / 4;
+    for (int64_t k = t0; k < vecs; k += stride) reinterpret_cast<uint4*>(s.p)[k] = x;
+    if (t0 < s.words - 4 * vecs) s.p[4 * vecs + t0] = s.x;
+  }
+}
+
 // Fills the working values with each slot's "unreached" marker, or with
 // `uniform` everywhere when it is nonzero (the serving layout, where a slot
 // changes kind between requests).  Warp per vertex row, lanes over slots.
@@ -3478,7 +3509,7 @@ __global__ void k_materialize_planes(const uint64_t* visited, const uint64_t* pl
                                      int K, int64_t V, int Qg, OutMap om, int query_major) {
   if (query_major) {
     for (int q = blockIdx.y; q < Qg; q += gridDim.y) {
-      uint32_t* col = om.out + static_cast<int64_t>(om.qmap[q]) * om.sq;
+      uint32_t* col = om.out + om.col(q) * om.sq;
       for (int64_t v = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < V;
            v += static_cast<int64_t>(gridDim.x) * blockDim.x)
         col[v * om.sv] = plane_depth<W>(visited, planes, K, V, v, q);
@@ -3491,7 +3522,8 @@ __global__ void k_materialize_planes(const uint64_t* visited, const uint64_t* pl
   // depths (two 16-byte stores when the columns are contiguous and aligned).
   const int lane = threadIdx.x & 31;
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  const bool vec = om.qmap_contiguous && (om.sv % 4 == 0) && om.sq == 1 && (om.qmap[0] % 4 == 0);
+  const bool vec = om.qmap == nullptr && (om.sv % 4 == 0) && om.sq == 1 && (om.q0 % 4 == 0) &&
+                   (reinterpret_cast<uintptr_t>(om.out) & 15) == 0;
   for (int64_t v = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; v < V;
        v += warps) {
     uint32_t* row = om.out + v * om.sv;
@@ -3523,12 +3555,12 @@ __global__ void k_materialize_planes(const uint64_t* visited, const uint64_t* pl
       for (int j = 0; j < 8; ++j)
         if (!((vis >> j) & 1u)) d[j] = 0x7fffffffu;
       if (vec && q0 + 8 <= Qg) {
-        uint4* dst = reinterpret_cast<uint4*>(row + om.qmap[q0]);
+        uint4* dst = reinterpret_cast<uint4*>(row + om.col(q0));
         dst[0] = make_uint4(d[0], d[1], d[2], d[3]);
         dst[1] = make_uint4(d[4], d[5], d[6], d[7]);
       } else {
         for (int j = 0; j < 8 && q0 + j < Qg; ++j)
-          row[static_cast<int64_t>(om.qmap[q0 + j]) * om.sq] = d[j];
+          row[om.col(q0 + j) * om.sq] = d[j];
       }
     }
   }
@@ -3541,7 +3573,7 @@ static __global__ void k_copy_values(const uint32_t* values, const SlotDev* slot
   if (query_major) {
     for (int q = blockIdx.y; q < n; q += gridDim.y) {
       if (slots[q].kind == 2) continue;
-      uint32_t* col = om.out + static_cast<int64_t>(om.qmap[q]) * om.sq;
+      uint32_t* col = om.out + om.col(q) * om.sq;
       for (int64_t v = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < V;
            v += static_cast<int64_t>(gridDim.x) * blockDim.x)
         col[v * om.sv] = values[static_cast<size_t>(v) * Qg + q];
@@ -3556,7 +3588,7 @@ static __global__ void k_copy_values(const uint32_t* values, const SlotDev* slot
     const uint32_t* src = values + static_cast<size_t>(v) * Qg;
     uint32_t* row = om.out + v * om.sv;
     for (int q = lane; q < n; q += 32)
-      if (slots[q].kind != 2) row[static_cast<int64_t>(om.qmap[q]) * om.sq] = src[q];
+      if (slots[q].kind != 2) row[om.col(q) * om.sq] = src[q];
   }
 }
 

@@ -333,7 +333,7 @@ GroupDev server_dev(const ServeGroup& gr) {
   g.hq_start = nullptr;
   g.ctl = ws->ctl.as<LevelCtl>();
   g.prof = nullptr;
-  g.slots = ws->slots.as<SlotDev>();
+  g.slots = ws->slots_dev();
   g.Qg = gr.S;
   return g;
 }
