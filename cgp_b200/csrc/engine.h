@@ -14,6 +14,7 @@
 
 #include "cgp_b200_internal.h"
 #include "device_types.cuh"
+#include "host_copy.h"
 
 namespace cgp {
 
@@ -172,6 +173,7 @@ struct GraphImpl {
   std::mutex heavy_mu;
   std::map<int64_t, std::unique_ptr<HeavyPair>> heavy_cache;  // built once per threshold
   std::vector<std::unique_ptr<Workspace>> pool;  // idle workspaces
+  std::vector<std::unique_ptr<HostCopier>> copiers;  // idle copiers, one per copy at a time
 
   // Pull CSR: the CSR itself when it lists every vertex's in-edges in the
   // order of the transpose (symmetric, sorted), else the stored transpose.
@@ -189,6 +191,8 @@ struct GraphImpl {
   dev::DevGraph dev_graph(int64_t h, bool light_items = true);
   std::unique_ptr<Workspace> acquire();
   void release(std::unique_ptr<Workspace> ws);
+  // Copies segments into pageable memory through an idle (or new) copier.
+  void copy_out(const std::vector<HostSegment>& segs, cudaStream_t s);
 };
 
 // A traversal group: up to 64*W slots sharing one set of vertex masks.

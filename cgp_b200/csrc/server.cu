@@ -420,12 +420,17 @@ void cgp_server::retire(ServeGroup& gr, std::vector<int>& to_retire, bool forced
     rf(server_dev(gr), V, gr.retire_dev.as<RetireReq>(), n, staging.as<uint32_t>(),
        gr.clear_dev.as<uint64_t>(), forced ? 1 : 0, f32, g->num_sms * 4, gr.stream);
     ck(cudaGetLastError(), "retire");
+    std::vector<HostSegment> rows;  // results for pageable memory
     for (int i = 0; i < n; ++i) {
-      if (gr.h_retire[i].has_out && !outs[i].second)
-        ck(cudaMemcpyAsync(outs[i].first, staging.as<uint32_t>() + static_cast<size_t>(i) * V,
-                           static_cast<size_t>(V) * 4, cudaMemcpyDeviceToHost, gr.stream),
-           "result copy");
+      if (!gr.h_retire[i].has_out || outs[i].second) continue;
+      const uint32_t* row = staging.as<uint32_t>() + static_cast<size_t>(i) * V;
+      if (HostCopier::direct(outs[i].first))
+        ck(cudaMemcpyAsync(outs[i].first, row, static_cast<size_t>(V) * 4, cudaMemcpyDeviceToHost,
+                           gr.stream), "result copy");
+      else
+        rows.push_back({outs[i].first, row, static_cast<size_t>(V) * 4});
     }
+    if (!rows.empty()) g->copy_out(rows, gr.stream);
     ck(cudaStreamSynchronize(gr.stream), "retire");
     std::lock_guard<std::mutex> lk(mu);
     const double t = now_ms();
