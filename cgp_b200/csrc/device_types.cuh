@@ -110,6 +110,7 @@ struct LevelCtl {
   unsigned long long prev_pull_edges; // in-edges the previous BFS pull level read
   int32_t prev_dir;                 // BFS direction of the previous level
   int32_t bfs_chunked;              // the BFS pull may run in CTA chunks (chunk table built)
+  int32_t khop;                     // the group has held k-hop slots: expand is recomputed
   int32_t bnd_avail;                // bounds arrays exist and the gather kernels read them
   int32_t bnd_on;                   // this gather level screens row chunks by bounds
   int32_t bnd_good;                 // the last level that did skipped at least half of them

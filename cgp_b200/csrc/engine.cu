@@ -596,6 +596,7 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
     const int k = spec.slots[q].kind;
     if (k == CGP_KIND_BFS || k == CGP_KIND_KHOP) c.bfs_bits[q >> 6] |= 1ULL << (q & 63);
     if (k == CGP_KIND_SSSP) c.sssp_bits[q >> 6] |= 1ULL << (q & 63);
+    if (k == CGP_KIND_KHOP) c.khop = 1;
   }
   for (int i = 0; i < kMaxW; ++i) c.expand[i] = ~0ULL;
   c.forced_dir = -1;
@@ -698,7 +699,8 @@ int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelL
   const int most = k.per_sm * g->num_sms;
   const int blocks = static_cast<int>(std::max<int64_t>(
       1, std::min<int64_t>(most, (g->E + g->V) / 512)));
-  void* args[] = {&L.g, &L.G, &levels};
+  bool heavy = L.heavy_push;
+  void* args[] = {&L.g, &L.G, &levels, &heavy};
   ck(cudaLaunchCooperativeKernel(k.fn, dim3(blocks), dim3(kBlock), args, 0, s), "fused level loop");
   return 1;
 }

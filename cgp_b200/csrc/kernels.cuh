@@ -152,18 +152,6 @@ __device__ __forceinline__ int select_bit64(uint64_t x, int j) {
   return pos;
 }
 
-// j-th (0-based) set bit of a W-word mask.
-template <int W>
-__device__ __forceinline__ int jth_set_bit(const uint64_t* bits, int j) {
-#pragma unroll
-  for (int i = 0; i < W; ++i) {
-    const int c = __popcll(bits[i]);
-    if (j < c) return i * 64 + select_bit64(bits[i], j);
-    j -= c;
-  }
-  return -1;
-}
-
 // Bit c: 32-slot chunk c of the mask has a bit set.
 template <int W>
 __device__ __forceinline__ uint32_t chunk_bits(const uint64_t (&m)[W]) {
@@ -373,7 +361,8 @@ struct PushSmem {
 
 template <int W, typename OT, int DEPTH>
 __device__ __forceinline__ void bfs_push_tiles(const GroupDev& g, const DevGraph& G, unsigned bid,
-                                               unsigned nblk, PushSmem<W>& sm) {
+                                               unsigned nblk, PushSmem<W>& sm,
+                                               bool sweep = false) {
   int64_t (&s_beg)[kWarpsPerBlock][32] = sm.beg;
   int32_t (&s_inc)[kWarpsPerBlock][32] = sm.inc;
   uint64_t (&s_f)[kWarpsPerBlock][32][W] = sm.f;
@@ -411,6 +400,12 @@ __device__ __forceinline__ void bfs_push_tiles(const GroupDev& g, const DevGraph
       load_mask<W>(lv.fcur + static_cast<size_t>(u) * W, f);
 #pragma unroll
       for (int i = 0; i < W; ++i) f[i] &= sel[i];
+      if (sweep) {  // no one else reads the mask: the buffer is clean for level + 1
+        uint64_t z[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) z[i] = 0;
+        store_mask<W>(const_cast<uint64_t*>(lv.fcur) + static_cast<size_t>(u) * W, z);
+      }
     }
     const int64_t deg = end - beg;
     const bool work = valid && mask_any<W>(f) && deg > 0 && deg <= light;
@@ -1195,53 +1190,7 @@ __device__ __forceinline__ uint32_t relax(uint32_t du, const void* w, int64_t e)
   }
 }
 
-// One (edge, query) relaxation: values are compared as uint32, which orders
-// non-negative floats exactly like their values (+inf = 0x7f800000).
-template <int W, int WK>
-__device__ __forceinline__ bool sssp_relax(const GroupDev& g, const LevelView& lv,
-                                           int32_t u, int32_t n, int q,
-                                           const void* w, int64_t e,
-                                           uint64_t (&uni)[W],
-                                           unsigned long long& improved) {
-  const size_t Qg = static_cast<size_t>(g.Qg);
-  const uint32_t du = g.values[static_cast<size_t>(u) * Qg + q];
-  const uint32_t cand = relax<WK>(du, w, e);
-  uint32_t* dst = g.values + static_cast<size_t>(n) * Qg + q;
-  if (cand >= *dst) return false;
-  const uint32_t old = atomicMin(dst, cand);
-  if (cand >= old) return false;
-  const uint64_t bit = 1ULL << (q & 63);
-  // hub destinations receive many improvements per level: a plain read of
-  // the frontier word and of the stamp skips atomics that would change
-  // nothing (bits and stamps only grow within a level)
-  uint64_t* fw = lv.fnext + static_cast<size_t>(n) * W + (q >> 6);
-  if (!(*fw & bit)) atomic_or64(fw, bit);
-  uni[q >> 6] |= bit;
-  ++improved;
-  if (g.stamp[n] >= lv.level + 1) return false;
-  return atomicMax(g.stamp + n, lv.level + 1) < lv.level + 1;
-}
-
-// Second half of sssp_relax, for callers that loaded the destination value
-// themselves (cand < the value they read): the atomicMin and its frontier,
-// union and stamp updates.  True when n must be appended.
-template <int W>
-__device__ __forceinline__ bool sssp_commit(const GroupDev& g, const LevelView& lv, int32_t n,
-                                            int q, uint32_t cand, uint64_t (&uni)[W],
-                                            unsigned long long& improved) {
-  uint32_t* dst = g.values + static_cast<size_t>(n) * static_cast<size_t>(g.Qg) + q;
-  const uint32_t old = atomicMin(dst, cand);
-  if (cand >= old) return false;
-  const uint64_t bit = 1ULL << (q & 63);
-  uint64_t* fw = lv.fnext + static_cast<size_t>(n) * W + (q >> 6);
-  if (!(*fw & bit)) atomic_or64(fw, bit);
-  uni[q >> 6] |= bit;
-  ++improved;
-  if (g.stamp[n] >= lv.level + 1) return false;
-  return atomicMax(g.stamp + n, lv.level + 1) < lv.level + 1;
-}
-
-// Pairs handled per lane per step by the sparse scatter loops: their column,
+// Pairs handled per lane per step by the flattened scatter loops: their column,
 // source and destination loads are independent and issued together.
 constexpr int kPairSteps = 4;
 
@@ -1265,252 +1214,284 @@ __device__ __forceinline__ uint32_t weight_bits(const void* w, int64_t e) {
   }
 }
 
-// Vertices with more active SSSP bits than this take the dense path.
-constexpr int kDenseBits = 16;
+// Vertices with at most this many active SSSP bits are scattered as flattened
+// (edge, slot) pairs, those with more as slot lists.  A pair costs a search for
+// its vertex and a division (some 80 instructions for 32 pairs); a list step
+// (some 14) relaxes up to 32 slots over one edge, so it pays from about 6 on.
+constexpr int kListBits = 6;
 
-// Dense SSSP relaxation of edges [eb, ee) of vertex u by one warp (all lanes
-// call).  Lane j owns query 32c+j of every 32-bit chunk c of the vertex's
-// active mask: u's distances stay in registers, and per edge each active
-// chunk costs one coalesced 128-byte load of the neighbour's row, a compare,
-// and an atomicMin only where it improves; the improved bits of a chunk are
-// combined by a ballot into one atomicOr of the next-frontier word.
-template <int W, typename OT, int WK, int U>
-__device__ __forceinline__ void sssp_dense_edges(const GroupDev& g, const DevGraph& G,
-                                                 const LevelView& lv, int32_t u,
-                                                 const uint64_t (&bits)[W], int64_t eb,
-                                                 int64_t ee, int lane, uint64_t (&uni)[W],
-                                                 unsigned long long& improved,
-                                                 WarpAppender& ap) {
-  const size_t Qg = static_cast<size_t>(g.Qg);
-  uint32_t half[2 * W];
-  uint32_t du[2 * W];
-  bool act[2 * W];
+// Union of the slots improved by a block, one 32-bit word per 32 slots.
+template <int W>
+struct SlotUnion {
+  uint32_t word[2 * W];
+};
+
+template <int W>
+__device__ __forceinline__ void slot_union_clear(SlotUnion<W>& un) {
+  if (threadIdx.x < 2 * W) un.word[threadIdx.x] = 0;
+  __syncthreads();
+}
+
+// All threads call, after their last improvement.
+template <int W>
+__device__ __forceinline__ void slot_union_flush(const SlotUnion<W>& un, uint64_t* dst) {
+  __syncthreads();
+  if (threadIdx.x < 2 * W && un.word[threadIdx.x])
+    atomicOr(reinterpret_cast<uint32_t*>(dst) + threadIdx.x, un.word[threadIdx.x]);
+}
+
+// Lists the set bits of a vertex's active mask (32-bit half c in lane c, c <
+// 2W; 0 in the other lanes) into slots[], ascending; returns how many there
+// are.  All lanes call.
+__device__ __forceinline__ int list_slots(uint32_t half, int lane, uint16_t* slots) {
+  const int mine = __popc(half);
+  int inc = mine;
 #pragma unroll
-  for (int c = 0; c < 2 * W; ++c) {
-    half[c] = static_cast<uint32_t>(bits[c >> 1] >> (32 * (c & 1)));
-    act[c] = (half[c] >> lane) & 1u;
-    du[c] = act[c] ? g.values[static_cast<size_t>(u) * Qg + 32 * c + lane] : 0xffffffffu;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(kFull, inc, o);
+    if (lane >= o) inc += t;
   }
-  for (int64_t e0 = eb; e0 < ee; e0 += 32) {
-    const int64_t e = e0 + lane;
-    int32_t nl = 0;
-    uint32_t wl = 0;
-    if (e < ee) {
-      nl = G.col[e];
-      wl = weight_bits<WK>(G.w, e);
-    }
-    const int cnt = static_cast<int>(ee - e0 < 32 ? ee - e0 : 32);
-    // U edges per step (1 or 2): U x (active chunks) row loads in flight per warp
-    for (int i = 0; i < cnt; i += U) {
-      const bool two = U == 2 && i + 1 < cnt;
-      const int32_t nb0 = __shfl_sync(kFull, nl, i);
-      const uint32_t wt0 = __shfl_sync(kFull, wl, i);
-      const int32_t nb1 = __shfl_sync(kFull, nl, two ? i + 1 : i);
-      const uint32_t wt1 = __shfl_sync(kFull, wl, two ? i + 1 : i);
-      uint32_t* row0 = g.values + static_cast<size_t>(nb0) * Qg + lane;
-      uint32_t* row1 = g.values + static_cast<size_t>(nb1) * Qg + lane;
-      uint32_t cur0[2 * W], cur1[2 * W];
-#pragma unroll
-      for (int c = 0; c < 2 * W; ++c) {
-        cur0[c] = act[c] ? row0[32 * c] : 0u;
-        cur1[c] = (act[c] && two) ? row1[32 * c] : 0u;
+  int at = inc - mine;
+  while (half) {
+    slots[at++] = static_cast<uint16_t>(32 * lane + __ffs(half) - 1);
+    half &= half - 1;
+  }
+  __syncwarp();
+  return __shfl_sync(kFull, inc, 31);
+}
+
+// Scatters edges [eb, ee) of vertex u for the k slots in slots[] (one warp, all
+// lanes call): lane j takes the j-th slot of each run of 32, keeps u's distance
+// to it in a register and relaxes U edges per step.  Listed slots ascend, so a
+// run of neighbouring slots reads neighbouring words, and a vertex with every
+// slot active reads whole rows.
+template <int W, typename OT, int WK, int U>
+__device__ __forceinline__ void scatter_list(const GroupDev& g, const DevGraph& G,
+                                             const LevelView& lv, int32_t u,
+                                             const uint16_t* slots, int k, int64_t eb, int64_t ee,
+                                             int lane, SlotUnion<W>& un,
+                                             unsigned long long& improved, WarpAppender& ap) {
+  const size_t Qg = static_cast<size_t>(g.Qg);
+  for (int j0 = 0; j0 < k; j0 += 32) {
+    const bool on = j0 + lane < k;
+    const int q = on ? slots[j0 + lane] : 0;
+    const uint32_t du = on ? g.values[static_cast<size_t>(u) * Qg + q] : 0xffffffffu;
+    // 32 slots of one aligned chunk: the ballot of the improved lanes is its word
+    const int q0 = __shfl_sync(kFull, q, 0);
+    const bool chunk = __all_sync(kFull, on && (q0 & 31) == 0 && q == q0 + lane);
+    for (int64_t e0 = eb; e0 < ee; e0 += 32) {
+      int32_t nl = 0;
+      uint32_t wl = 0;
+      if (e0 + lane < ee) {
+        nl = G.col[e0 + lane];
+        wl = weight_bits<WK>(G.w, e0 + lane);
       }
-      bool better = false;
-#pragma unroll
-      for (int c = 0; c < 2 * W; ++c) {
-        better |= act[c] && relax_w<WK>(du[c], wt0) < cur0[c];
-        better |= act[c] && two && relax_w<WK>(du[c], wt1) < cur1[c];
-      }
-      // improvements are rare: atomics and ballots only when some lane of the
-      // warp has a better candidate for one of the two edges
-      if (!__any_sync(kFull, better)) continue;
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        if (t == 1 && !two) break;
-        const int32_t nb = t ? nb1 : nb0;
-        const uint32_t wt = t ? wt1 : wt0;
-        uint32_t* row = t ? row1 : row0;
+      const int cnt = static_cast<int>(ee - e0 < 32 ? ee - e0 : 32);
+      for (int i = 0; i < cnt; i += U) {
+        int32_t nb[U];
+        uint32_t cand[U], cur[U];
         bool any = false;
 #pragma unroll
-        for (int c = 0; c < 2 * W; ++c) {
-          if (half[c] == 0) continue;
-          const uint32_t cand = relax_w<WK>(du[c], wt);
-          bool imp = false;
-          if (act[c] && cand < (t ? cur1[c] : cur0[c])) imp = cand < atomicMin(row + 32 * c, cand);
-          const unsigned m = __ballot_sync(kFull, imp);
-          if (m) {
-            any = true;
-            if (lane == 0) {
-              const uint64_t bitsw = static_cast<uint64_t>(m) << (32 * (c & 1));
-              atomic_or64(lv.fnext + static_cast<size_t>(nb) * W + (c >> 1), bitsw);
-              uni[c >> 1] |= bitsw;
-              improved += __popc(m);
-            }
-          }
+        for (int t = 0; t < U; ++t) {
+          nb[t] = __shfl_sync(kFull, nl, i + t < cnt ? i + t : i);
+          const uint32_t w = __shfl_sync(kFull, wl, i + t < cnt ? i + t : i);
+          const bool go = on && i + t < cnt;
+          cand[t] = go ? relax_w<WK>(du, w) : 0xffffffffu;
+          cur[t] = go ? g.values[static_cast<size_t>(nb[t]) * Qg + q] : 0u;
         }
-        bool app = false;
-        if (any && lane == 0 && g.stamp[nb] < lv.level + 1)
-          app = atomicMax(g.stamp + nb, lv.level + 1) < lv.level + 1;
-        ap.add<OT>(app, nb, G, lv, lane);
+#pragma unroll
+        for (int t = 0; t < U; ++t) any |= cand[t] < cur[t];
+        if (!__any_sync(kFull, any)) continue;
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+          bool imp = false;
+          if (cand[t] < cur[t])
+            imp = cand[t] < atomicMin(g.values + static_cast<size_t>(nb[t]) * Qg + q, cand[t]);
+          const unsigned m = __ballot_sync(kFull, imp);
+          if (m == 0) continue;
+          uint32_t* fw = reinterpret_cast<uint32_t*>(lv.fnext + static_cast<size_t>(nb[t]) * W) + (q >> 5);
+          if (chunk) {
+            if (lane == 0) {
+              atomicOr(fw, m);
+              atomicOr(&un.word[q >> 5], m);
+            }
+          } else if (imp) {
+            atomicOr(fw, 1u << (q & 31));
+            atomicOr(&un.word[q >> 5], 1u << (q & 31));
+          }
+          improved += imp ? 1 : 0;
+          bool app = false;
+          if (lane == 0 && g.stamp[nb[t]] < lv.level + 1)
+            app = atomicMax(g.stamp + nb[t], lv.level + 1) < lv.level + 1;
+          ap.add<OT>(app, nb[t], G, lv, lane);
+        }
       }
     }
   }
 }
 
-// Dense SSSP vertices of a level, one warp per vertex (the tile kernel
-// queued them), so that this loop gets a register budget of its own.
-template <int W, typename OT, int WK, int U>
-__device__ __forceinline__ void sssp_dense_vertices(const GroupDev& g, const DevGraph& G,
-                                                    unsigned bid, unsigned nblk) {
-  const LevelCtl* ctl = g.ctl;
-  if (ctl->done || !ctl->sscatter) return;
-  const LevelView lv = level_view(g);
-  WarpAppender ap;
-  const unsigned long long n = ctl->dense_count;
-  const int lane = threadIdx.x & 31;
-  const unsigned long long gw = (static_cast<unsigned long long>(bid) * blockDim.x + threadIdx.x) >> 5;
-  const unsigned long long nwarps = (static_cast<unsigned long long>(nblk) * blockDim.x) >> 5;
-  uint64_t uni[W];
-#pragma unroll
-  for (int i = 0; i < W; ++i) uni[i] = 0;
-  unsigned long long improved = 0;
-  for (unsigned long long i = gw; i < n; i += nwarps) {
-    const int32_t u = g.dense_list[i];
-    const int64_t beg = row_at<OT>(G.row, u);
-    const int64_t end = row_at<OT>(G.row, static_cast<int64_t>(u) + 1);
-    uint64_t b[W];
-    load_mask<W>(lv.fcur + static_cast<size_t>(u) * W, b);
-#pragma unroll
-    for (int k = 0; k < W; ++k) b[k] &= ctl->ssel[k];
-    sssp_dense_edges<W, OT, WK, U>(g, G, lv, u, b, beg, end, lane, uni, improved, ap);
-  }
-  ap.flush<OT>(G, lv, lane);
-  flush_union<W>(uni, lv.nactive, lane);
-  warp_add(improved, &g.ctl->lc.improved, lane);
+// One flattened pair's improvement (cand < the value read): atomicMin, frontier
+// bit, union and stamp.  True when n must be appended.  Hub destinations
+// receive many improvements per level: a plain read of the frontier word and
+// of the stamp skips atomics that would change nothing (bits and stamps only
+// grow within a level).
+template <int W>
+__device__ __forceinline__ bool scatter_commit(const GroupDev& g, const LevelView& lv, int32_t n,
+                                               int q, uint32_t cand, SlotUnion<W>& un,
+                                               unsigned long long& improved) {
+  uint32_t* dst = g.values + static_cast<size_t>(n) * static_cast<size_t>(g.Qg) + q;
+  if (cand >= atomicMin(dst, cand)) return false;
+  const uint32_t bit = 1u << (q & 31);
+  uint32_t* fw = reinterpret_cast<uint32_t*>(lv.fnext + static_cast<size_t>(n) * W) + (q >> 5);
+  const bool seen = *fw & bit;
+  const bool listed = g.stamp[n] >= lv.level + 1;
+  if (!seen) atomicOr(fw, bit);
+  atomicOr(&un.word[q >> 5], bit);
+  ++improved;
+  return !listed && atomicMax(g.stamp + n, lv.level + 1) < lv.level + 1;
 }
 
-template <int W, typename OT, int WK, int U>
-__global__ void __launch_bounds__(kBlock, (U == 1 ? 4 : 3)) k_sssp_dense(GroupDev g, DevGraph G) {
-  sssp_dense_vertices<W, OT, WK, U>(g, G, blockIdx.x, gridDim.x);
-}
-
-// SSSP push over the frontier list: the (edge, active query) pairs of a tile
-// of 32 vertices are flattened and spread evenly over the warp's lanes, so a
-// vertex with k active queries and degree d costs k*d/32 warp steps.
 template <int W>
 struct SsspPushSmem {
   int64_t beg[kWarpsPerBlock][32];
-  long long inc[kWarpsPerBlock][32];
-  int32_t k[kWarpsPerBlock][32];
+  int32_t inc[kWarpsPerBlock][32];
   int32_t u[kWarpsPerBlock][32];
-  uint64_t b[kWarpsPerBlock][32][W];
+  uint8_t k[kWarpsPerBlock][32];
+  uint16_t q[kWarpsPerBlock][32][kListBits];
+  uint16_t slots[kWarpsPerBlock][64 * W];
+  SlotUnion<W> un;
 };
 
+// Frontiers of at most this many vertices have their listed vertices scattered
+// by the tile's own warp; larger ones queue them for sssp_list_vertices, which
+// spreads them over all warps.
+constexpr unsigned long long kInlineLists = 16384;
+
+// SSSP push over the frontier list, a warp per tile of 32 vertices.  Vertices
+// with few active bits: the tile's (edge, slot) pairs are flattened and spread
+// evenly over the lanes.  The others go by slot lists, here or queued.  sweep:
+// zero each vertex's mask once it is read (lists of the frontier must all be
+// scattered by the tiles themselves).
 template <int W, typename OT, int WK>
 __device__ __forceinline__ void sssp_push_tiles(const GroupDev& g, const DevGraph& G, unsigned bid,
-                                                unsigned nblk, SsspPushSmem<W>& sm) {
-  int64_t (&s_beg)[kWarpsPerBlock][32] = sm.beg;
-  long long (&s_inc)[kWarpsPerBlock][32] = sm.inc;
-  int32_t (&s_k)[kWarpsPerBlock][32] = sm.k;
-  int32_t (&s_u)[kWarpsPerBlock][32] = sm.u;
-  uint64_t (&s_b)[kWarpsPerBlock][32][W] = sm.b;
+                                                unsigned nblk, SsspPushSmem<W>& sm,
+                                                bool sweep = false) {
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || !ctl->sscatter) return;
   const LevelView lv = level_view(g);
   WarpAppender ap;
   const unsigned long long n = ctl->count[lv.par];
   const int64_t light = push_light_limit(g, G, n, ctl->edges[lv.par]);
-  uint64_t sel[W];
-#pragma unroll
-  for (int i = 0; i < W; ++i) sel[i] = ctl->ssel[i];
-  if (!mask_any<W>(sel)) return;
+  const bool here = n <= kInlineLists;
+  slot_union_clear<W>(sm.un);
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const unsigned long long gw = (static_cast<unsigned long long>(bid) * blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = (static_cast<unsigned long long>(nblk) * blockDim.x) >> 5;
-  uint64_t uni[W];
-#pragma unroll
-  for (int i = 0; i < W; ++i) uni[i] = 0;
+  const size_t Qg = static_cast<size_t>(g.Qg);
   unsigned long long improved = 0, spairs = 0, sactive = 0;
   for (unsigned long long tile = gw; tile * 32 < n; tile += nwarps) {
     const unsigned long long idx = tile * 32 + lane;
     const bool valid = idx < n;
-    int32_t u = valid ? lv.list[idx] : 0;
+    const int32_t u = valid ? lv.list[idx] : 0;
     int64_t beg = 0, end = 0;
-    uint64_t b[W];
     int k = 0;
+    {
+      uint64_t b[W];
 #pragma unroll
-    for (int i = 0; i < W; ++i) b[i] = 0;
-    if (valid) {
-      beg = row_at<OT>(G.row, u);
-      end = row_at<OT>(G.row, static_cast<int64_t>(u) + 1);
-      load_mask<W>(lv.fcur + static_cast<size_t>(u) * W, b);
+      for (int i = 0; i < W; ++i) b[i] = 0;
+      if (valid) {
+        beg = row_at<OT>(G.row, u);
+        end = row_at<OT>(G.row, static_cast<int64_t>(u) + 1);
+        load_mask<W>(lv.fcur + static_cast<size_t>(u) * W, b);
+      }
 #pragma unroll
       for (int i = 0; i < W; ++i) {
-        b[i] &= sel[i];
+        b[i] &= ctl->ssel[i];
         k += __popcll(b[i]);
+      }
+      if (k > 0 && k <= kListBits) {
+        int at = 0;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          while (b[i]) {
+            sm.q[wib][lane][at++] = static_cast<uint16_t>(64 * i + __ffsll(static_cast<long long>(b[i])) - 1);
+            b[i] &= b[i] - 1;
+          }
+        }
       }
     }
     const int64_t deg = end - beg;
     const bool work = valid && k > 0 && deg > 0 && deg <= light;
     spairs += work ? static_cast<unsigned long long>(k) * static_cast<unsigned long long>(deg) : 0ULL;
     sactive += static_cast<unsigned long long>(k);
-    // vertices with many active queries go to the dense kernel
-    {
-      const bool dq = work && k > kDenseBits;
-      const unsigned m = __ballot_sync(kFull, dq);
-      if (m) {
-        unsigned long long base = 0;
-        if (lane == __ffs(m) - 1)
-          base = atomicAdd(&g.ctl->dense_count, static_cast<unsigned long long>(__popc(m)));
-        base = __shfl_sync(kFull, base, __ffs(m) - 1);
-        if (dq) g.dense_list[base + __popc(m & ((1u << lane) - 1u))] = u;
-      }
+    unsigned lists = __ballot_sync(kFull, work && k > kListBits);
+    if (lists && !here) {
+      unsigned long long base = 0;
+      if (lane == 0)
+        base = atomicAdd(&g.ctl->dense_count, static_cast<unsigned long long>(__popc(lists)));
+      base = __shfl_sync(kFull, base, 0);
+      if ((lists >> lane) & 1u) g.dense_list[base + __popc(lists & ((1u << lane) - 1u))] = u;
+      lists = 0;
     }
-    // the rest: (edge, query) pairs flattened over the lanes
-    long long wk = (work && k <= kDenseBits) ? static_cast<long long>(k) * deg : 0;
-    long long inc = wk;
+    while (lists) {
+      const int src = __ffs(lists) - 1;
+      lists &= lists - 1;
+      const int32_t lu = __shfl_sync(kFull, u, src);
+      const int64_t lb = __shfl_sync(kFull, beg, src), le = __shfl_sync(kFull, end, src);
+      const uint32_t half = lane < 2 * W
+          ? reinterpret_cast<const uint32_t*>(lv.fcur + static_cast<size_t>(lu) * W)[lane] &
+                reinterpret_cast<const uint32_t*>(ctl->ssel)[lane]
+          : 0u;
+      const int lk = list_slots(half, lane, sm.slots[wib]);
+      scatter_list<W, OT, WK, 4>(g, G, lv, lu, sm.slots[wib], lk, lb, le, lane, sm.un, improved, ap);
+      __syncwarp();
+    }
+    if (sweep && valid) {  // no one reads the mask any more: clean for level + 1
+      uint64_t z[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) z[i] = 0;
+      store_mask<W>(const_cast<uint64_t*>(lv.fcur) + static_cast<size_t>(u) * W, z);
+    }
+    // the rest: (edge, slot) pairs flattened over the lanes
+    const int wk = (work && k <= kListBits) ? k * static_cast<int>(deg) : 0;
+    int inc = wk;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      long long t = __shfl_up_sync(kFull, inc, o);
+      const int t = __shfl_up_sync(kFull, inc, o);
       if (lane >= o) inc += t;
     }
-    const long long total = __shfl_sync(kFull, inc, 31);
+    const int total = __shfl_sync(kFull, inc, 31);
     if (total == 0) continue;
-    s_beg[wib][lane] = beg;
-    s_inc[wib][lane] = inc;
-    s_k[wib][lane] = k;
-    s_u[wib][lane] = u;
-#pragma unroll
-    for (int i = 0; i < W; ++i) s_b[wib][lane][i] = b[i];
+    sm.beg[wib][lane] = beg;
+    sm.inc[wib][lane] = inc;
+    sm.k[wib][lane] = static_cast<uint8_t>(k <= kListBits ? k : 0);
+    sm.u[wib][lane] = u;
     __syncwarp();
-    const size_t Qg = static_cast<size_t>(g.Qg);
-    for (long long b0 = 0; b0 < total; b0 += 32 * kPairSteps) {
+    for (int b0 = 0; b0 < total; b0 += 32 * kPairSteps) {
       int32_t nb[kPairSteps];
       int qq[kPairSteps];
       uint32_t cand[kPairSteps], cur[kPairSteps];
 #pragma unroll
       for (int t = 0; t < kPairSteps; ++t) {
-        const long long p = b0 + 32 * t + lane;
+        const int p = b0 + 32 * t + lane;
         nb[t] = 0;
         qq[t] = 0;
         cand[t] = 0xffffffffu;
         if (p < total) {
           int lo = 0, hi = 31;
           while (lo < hi) {
-            int mid = (lo + hi) >> 1;
-            if (s_inc[wib][mid] > p) hi = mid;
+            const int mid = (lo + hi) >> 1;
+            if (sm.inc[wib][mid] > p) hi = mid;
             else lo = mid + 1;
           }
-          const long long start = lo ? s_inc[wib][lo - 1] : 0;
-          const int local = static_cast<int>(p - start);  // < kDenseBits * heavy_degree
-          const int ko = s_k[wib][lo];
+          const int local = p - (lo ? sm.inc[wib][lo - 1] : 0);
+          const int ko = sm.k[wib][lo];
           const int eoff = local / ko;
-          const int j = local - eoff * ko;
-          qq[t] = jth_set_bit<W>(s_b[wib][lo], j);
-          const int64_t e = s_beg[wib][lo] + eoff;
+          qq[t] = sm.q[wib][lo][local - eoff * ko];
+          const int64_t e = sm.beg[wib][lo] + eoff;
           nb[t] = G.col[e];
-          cand[t] = relax<WK>(g.values[static_cast<size_t>(s_u[wib][lo]) * Qg + qq[t]], G.w, e);
+          cand[t] = relax<WK>(g.values[static_cast<size_t>(sm.u[wib][lo]) * Qg + qq[t]], G.w, e);
         }
       }
 #pragma unroll
@@ -1518,14 +1499,15 @@ __device__ __forceinline__ void sssp_push_tiles(const GroupDev& g, const DevGrap
         cur[t] = cand[t] != 0xffffffffu ? g.values[static_cast<size_t>(nb[t]) * Qg + qq[t]] : 0u;
 #pragma unroll
       for (int t = 0; t < kPairSteps; ++t) {
-        const bool app = cand[t] < cur[t] && sssp_commit<W>(g, lv, nb[t], qq[t], cand[t], uni, improved);
+        const bool app = cand[t] < cur[t] &&
+                         scatter_commit<W>(g, lv, nb[t], qq[t], cand[t], sm.un, improved);
         ap.add<OT>(app, nb[t], G, lv, lane);
       }
     }
     __syncwarp();
   }
   ap.flush<OT>(G, lv, lane);
-  flush_union<W>(uni, lv.nactive, lane);
+  slot_union_flush<W>(sm.un, lv.nactive);
   warp_add(improved, &g.ctl->lc.improved, lane);
   warp_add(spairs, &g.ctl->lc.sssp_pairs, lane);
   warp_add(sactive, &g.ctl->lc.sssp_active, lane);
@@ -1537,24 +1519,71 @@ __global__ void __launch_bounds__(kBlock) k_sssp_push(GroupDev g, DevGraph G) {
   sssp_push_tiles<W, OT, WK>(g, G, blockIdx.x, gridDim.x, sm);
 }
 
-// SSSP push for heavy frontier vertices: per chunk of kHeavyChunk edges the
-// CTA lists the active query ids once and walks (edge, query) pairs.
+template <int W>
+struct SsspListSmem {
+  uint16_t slots[kWarpsPerBlock][64 * W];
+  SlotUnion<W> un;
+};
+
+// The queued vertices of a level (more than kListBits active bits), one warp
+// per vertex; U edges per step.  Before, such vertices held 2W row chunks in
+// registers and walked all of them per edge whether active or not: on a grid
+// with 1024 slots and some 27 active bits per vertex, 34 ms of a 209 ms batch.
+template <int W, typename OT, int WK, int U>
+__device__ __forceinline__ void sssp_list_vertices(const GroupDev& g, const DevGraph& G,
+                                                   unsigned bid, unsigned nblk,
+                                                   SsspListSmem<W>& sm) {
+  const LevelCtl* ctl = g.ctl;
+  if (ctl->done || !ctl->sscatter) return;
+  const unsigned long long n = ctl->dense_count;
+  if (n == 0) return;
+  const LevelView lv = level_view(g);
+  WarpAppender ap;
+  slot_union_clear<W>(sm.un);
+  const int lane = threadIdx.x & 31;
+  const int wib = threadIdx.x >> 5;
+  const unsigned long long gw = (static_cast<unsigned long long>(bid) * blockDim.x + threadIdx.x) >> 5;
+  const unsigned long long nwarps = (static_cast<unsigned long long>(nblk) * blockDim.x) >> 5;
+  const uint32_t sel = lane < 2 * W ? reinterpret_cast<const uint32_t*>(ctl->ssel)[lane] : 0u;
+  unsigned long long improved = 0;
+  for (unsigned long long i = gw; i < n; i += nwarps) {
+    const int32_t u = g.dense_list[i];
+    const int64_t beg = row_at<OT>(G.row, u);
+    const int64_t end = row_at<OT>(G.row, static_cast<int64_t>(u) + 1);
+    const uint32_t half = lane < 2 * W
+        ? reinterpret_cast<const uint32_t*>(lv.fcur + static_cast<size_t>(u) * W)[lane] & sel
+        : 0u;
+    const int k = list_slots(half, lane, sm.slots[wib]);
+    scatter_list<W, OT, WK, U>(g, G, lv, u, sm.slots[wib], k, beg, end, lane, sm.un, improved, ap);
+    __syncwarp();
+  }
+  ap.flush<OT>(G, lv, lane);
+  slot_union_flush<W>(sm.un, lv.nactive);
+  warp_add(improved, &g.ctl->lc.improved, lane);
+}
+
+template <int W, typename OT, int WK, int U>
+__global__ void __launch_bounds__(kBlock, 4) k_sssp_list(GroupDev g, DevGraph G) {
+  __shared__ SsspListSmem<W> sm;
+  sssp_list_vertices<W, OT, WK, U>(g, G, blockIdx.x, gridDim.x, sm);
+}
+
 template <int W>
 struct SsspHeavySmem {
   int32_t h;
   int32_t k;
-  int16_t q[kMaxW * 64];
-  int32_t wpre[W + 1];
+  uint16_t q[64 * W];
+  SlotUnion<W> un;
 };
 
+// SSSP push for the queued heavy frontier vertices: per chunk of kHeavyChunk
+// edges the CTA lists the active slots once; with more than kListBits of them
+// each warp scatters a slice of the edges by the list, else the CTA walks the
+// (edge, slot) pairs.
 template <int W, typename OT, int WK>
 __device__ __forceinline__ void sssp_push_chunks(const GroupDev& g, const DevGraph& G,
                                                  unsigned bid, unsigned nblk,
                                                  SsspHeavySmem<W>& sm) {
-  int32_t& s_h = sm.h;
-  int32_t& s_k = sm.k;
-  int16_t (&s_q)[kMaxW * 64] = sm.q;
-  int32_t (&s_wpre)[W + 1] = sm.wpre;
   const LevelCtl* ctl = g.ctl;
   if (ctl->done || !ctl->sscatter) return;
   const unsigned long long hq = ctl->hq_packed;
@@ -1564,82 +1593,60 @@ __device__ __forceinline__ void sssp_push_chunks(const GroupDev& g, const DevGra
   if (nq == 0) return;
   const LevelView lv = level_view(g);
   WarpAppender ap;
+  slot_union_clear<W>(sm.un);
   const int lane = threadIdx.x & 31;
-  uint64_t uni[W];
-#pragma unroll
-  for (int i = 0; i < W; ++i) uni[i] = 0;
+  const int wib = threadIdx.x >> 5;
+  const size_t Qg = static_cast<size_t>(g.Qg);
   unsigned long long improved = 0;
   for (int64_t c = bid; c < nchunks; c += nblk) {
-    if (threadIdx.x == 0) s_h = heavy_queue_slot(g, nq, c);
+    if (threadIdx.x == 0) sm.h = heavy_queue_slot(g, nq, c);
     __syncthreads();
-    const int h = s_h;
+    const int h = sm.h;
     const int32_t u = g.hq_vertex[h];
-    uint64_t b[W];
-    load_mask<W>(lv.fcur + static_cast<size_t>(u) * W, b);
-#pragma unroll
-    for (int i = 0; i < W; ++i) b[i] &= ctl->ssel[i];
-    if (threadIdx.x == 0) {
-      int acc = 0;
-      for (int i = 0; i < W; ++i) {
-        s_wpre[i] = acc;
-        acc += __popcll(b[i]);
-      }
-      s_wpre[W] = acc;
-      s_k = acc;
+    if (wib == 0) {
+      const uint32_t half = lane < 2 * W
+          ? reinterpret_cast<const uint32_t*>(lv.fcur + static_cast<size_t>(u) * W)[lane] &
+                reinterpret_cast<const uint32_t*>(ctl->ssel)[lane]
+          : 0u;
+      const int k = list_slots(half, lane, sm.q);
+      if (lane == 0) sm.k = k;
     }
     __syncthreads();
-    const int k = s_k;
+    const int k = sm.k;
     if (k == 0) {
       __syncthreads();
       continue;
     }
-    if (k > kDenseBits) {
-      // each warp takes a contiguous slice of the chunk's edges
-      const int64_t beg = row_at<OT>(G.row, u);
-      const int64_t end = row_at<OT>(G.row, static_cast<int64_t>(u) + 1);
-      const int64_t cb = beg + (c - g.hq_start[h]) * kHeavyChunk;
-      const int64_t ce = min(end, cb + kHeavyChunk);
-      if (threadIdx.x == 0) {
-        atomicAdd(&g.ctl->lc.sssp_pairs, static_cast<unsigned long long>(ce - cb) * k);
-        if (c == g.hq_start[h]) atomicAdd(&g.ctl->lc.sssp_active, static_cast<unsigned long long>(k));
-      }
-      const int nw = blockDim.x >> 5;
-      const int64_t seg = (ce - cb + nw - 1) / nw;
-      const int64_t wb = cb + (threadIdx.x >> 5) * seg;
-      const int64_t we = min(ce, wb + seg);
-      sssp_dense_edges<W, OT, WK, 1>(g, G, lv, u, b, wb, we, lane, uni, improved, ap);
-      __syncthreads();
-      continue;
-    }
-    for (int t = threadIdx.x; t < W * 64; t += blockDim.x) {
-      const int i = t >> 6, bit = t & 63;
-      if ((b[i] >> bit) & 1ULL)
-        s_q[s_wpre[i] + __popcll(b[i] & ((1ULL << bit) - 1ULL))] = static_cast<int16_t>(t);
-    }
-    __syncthreads();
     const int64_t beg = row_at<OT>(G.row, u);
     const int64_t end = row_at<OT>(G.row, static_cast<int64_t>(u) + 1);
     const int64_t cb = beg + (c - g.hq_start[h]) * kHeavyChunk;
     const int64_t ce = min(end, cb + kHeavyChunk);
-    const long long pairs = static_cast<long long>(ce - cb) * k;
     if (threadIdx.x == 0) {
-      atomicAdd(&g.ctl->lc.sssp_pairs, static_cast<unsigned long long>(pairs));
+      atomicAdd(&g.ctl->lc.sssp_pairs, static_cast<unsigned long long>(ce - cb) * k);
       if (c == g.hq_start[h]) atomicAdd(&g.ctl->lc.sssp_active, static_cast<unsigned long long>(k));
     }
-    const size_t Qg = static_cast<size_t>(g.Qg);
-    for (long long p0 = threadIdx.x & ~31; p0 < pairs; p0 += kPairSteps * blockDim.x) {
+    if (k > kListBits) {
+      const int64_t seg = (ce - cb + kWarpsPerBlock - 1) / kWarpsPerBlock;
+      const int64_t wb = min(ce, cb + wib * seg);
+      const int64_t we = min(ce, wb + seg);
+      scatter_list<W, OT, WK, 4>(g, G, lv, u, sm.q, k, wb, we, lane, sm.un, improved, ap);
+      __syncthreads();
+      continue;
+    }
+    const int pairs = static_cast<int>(ce - cb) * k;
+    for (int p0 = threadIdx.x & ~31; p0 < pairs; p0 += kPairSteps * blockDim.x) {
       int32_t nb[kPairSteps];
       int qq[kPairSteps];
       uint32_t cand[kPairSteps], cur[kPairSteps];
 #pragma unroll
       for (int t = 0; t < kPairSteps; ++t) {
-        const long long p = p0 + t * blockDim.x + lane;
+        const int p = p0 + t * static_cast<int>(blockDim.x) + lane;
         nb[t] = 0;
         qq[t] = 0;
         cand[t] = 0xffffffffu;
         if (p < pairs) {
-          const int eoff = static_cast<int>(p) / k;  // pairs <= kHeavyChunk * kDenseBits
-          qq[t] = s_q[static_cast<int>(p) - eoff * k];
+          const int eoff = p / k;
+          qq[t] = sm.q[p - eoff * k];
           const int64_t e = cb + eoff;
           nb[t] = G.col[e];
           cand[t] = relax<WK>(g.values[static_cast<size_t>(u) * Qg + qq[t]], G.w, e);
@@ -1650,14 +1657,15 @@ __device__ __forceinline__ void sssp_push_chunks(const GroupDev& g, const DevGra
         cur[t] = cand[t] != 0xffffffffu ? g.values[static_cast<size_t>(nb[t]) * Qg + qq[t]] : 0u;
 #pragma unroll
       for (int t = 0; t < kPairSteps; ++t) {
-        const bool app = cand[t] < cur[t] && sssp_commit<W>(g, lv, nb[t], qq[t], cand[t], uni, improved);
+        const bool app = cand[t] < cur[t] &&
+                         scatter_commit<W>(g, lv, nb[t], qq[t], cand[t], sm.un, improved);
         ap.add<OT>(app, nb[t], G, lv, lane);
       }
     }
     __syncthreads();
   }
   ap.flush<OT>(G, lv, lane);
-  flush_union<W>(uni, lv.nactive, lane);
+  slot_union_flush<W>(sm.un, lv.nactive);
   warp_add(improved, &g.ctl->lc.improved, lane);
 }
 
@@ -3111,7 +3119,7 @@ __device__ __forceinline__ void level_end(const GroupDev& g, int lane) {
     ctl->edges[par] = 0;
   }
   __syncwarp();
-  compute_expand<W>(ctl, g.slots, g.Qg, l + 1, lane);
+  if (ctl->khop) compute_expand<W>(ctl, g.slots, g.Qg, l + 1, lane);
   const int32_t dir = decide_dir(ctl, nextc, nexte, any_bits<W>(ctl->bfs_bits));
   split_sssp_slots<W>(ctl, decide_sdir<W>(ctl, nextc, nexte), lane);
   if (lane != 0) return;
@@ -3308,6 +3316,7 @@ union TraverseSmem {
   HeavySlotSmem slot;
   PullHeavySmem<kBfs ? W : 1> pull_heavy;
   SsspPushSmem<kSssp ? W : 1> sssp_push;
+  SsspListSmem<kSssp ? W : 1> sssp_list;
   SsspHeavySmem<kSssp ? W : 1> sssp_heavy;
   GatherHeavySmem<kSssp ? W : 1> gather_heavy;
   GatherRowSmem gather_light;
@@ -3322,31 +3331,40 @@ union TraverseSmem {
 // their launches are the level's whole time.
 template <int W, typename OT, int DEPTH, int WK, bool kBfs, bool kSssp>
 __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev g, DevGraph G,
-                                                                      int levels) {
+                                                                      int levels, bool heavy) {
   __shared__ TraverseSmem<W, kBfs, kSssp> sm;
   const unsigned bid = blockIdx.x, nblk = gridDim.x;
   LevelCtl* ctl = g.ctl;
   GridBarrier bar(ctl, nblk);
+  bool swept = false;  // the previous level zeroed its own frontier's masks
   for (int l = 0; l < levels; ++l) {
     if (ctl->done) return;
     const bool bfs_pull = kBfs && ctl->dir == kDirPull;
     const bool gather = kSssp && ctl->sdir == kDirPull;
     const bool scatter = kSssp && ctl->sscatter != 0;
+    const bool queue = heavy && ((kBfs && !bfs_pull) || scatter);
+    const bool queued_lists = scatter && ctl->count[ctl->level & 1] > kInlineLists;
     bool summary = gather;
     if constexpr (kBfs) summary |= bfs_pull_uses_summary(g, ctl, level_view(g), G.V);
-    // what the level's phases read or add to: a pull over whole masks alone
+    // what the level's phases read or add to; a pull over whole masks alone
     // rewrites every next mask and needs nothing prepared
-    if (!bfs_pull || summary || scatter) {
-      clear_next<W>(g, G.E, bid, nblk);
+    const bool clear = ctl->dir == kDirPush && !swept && ctl->prev_count > 0;
+    if (clear || summary || queue) {
+      if (clear) clear_next<W>(g, G.E, bid, nblk);
       if (summary) frontier_summary<W, OT>(g, G, bid, nblk);
       if constexpr (kSssp) gather_bounds<W, OT, WK>(g, G, bid, nblk);
-      if (g.hq_vertex != nullptr) heavy_queue_scan<OT>(g, G, bid, nblk);
+      if (queue) heavy_queue_scan<OT>(g, G, bid, nblk);
       if (!bar.wait()) return;
     }
+    // A scattering level whose vertices are all expanded by the tiles reads each
+    // mask once and can zero it there: the next level has nothing to clear, and
+    // a level of a road-like graph is one phase and one barrier.
+    const bool sweep = kBfs != kSssp && !heavy && !bfs_pull && !gather && !queued_lists;
+    swept = sweep;
     if constexpr (kBfs) {
       if (!bfs_pull) {
-        bfs_push_tiles<W, OT, DEPTH>(g, G, bid, nblk, sm.push);
-        if (g.hq_vertex != nullptr) {
+        bfs_push_tiles<W, OT, DEPTH>(g, G, bid, nblk, sm.push, sweep);
+        if (heavy) {
           __syncthreads();
           bfs_push_chunks<W, OT, DEPTH>(g, G, nblk - 1 - bid, nblk, sm.slot);
         }
@@ -3365,13 +3383,15 @@ __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev 
     }
     if constexpr (kSssp) {
       if (scatter) {
-        sssp_push_tiles<W, OT, WK>(g, G, bid, nblk, sm.sssp_push);
-        if (g.hq_vertex != nullptr) {
+        sssp_push_tiles<W, OT, WK>(g, G, bid, nblk, sm.sssp_push, sweep);
+        if (heavy) {
           __syncthreads();
           sssp_push_chunks<W, OT, WK>(g, G, nblk - 1 - bid, nblk, sm.sssp_heavy);
         }
-        if (!bar.wait()) return;  // the list of dense vertices is complete
-        sssp_dense_vertices<W, OT, WK, 1>(g, G, bid, nblk);
+        if (queued_lists) {
+          if (!bar.wait()) return;  // the queue is complete
+          sssp_list_vertices<W, OT, WK, 4>(g, G, bid, nblk, sm.sssp_list);
+        }
         // a gather stores whole vectors of a row
         if (gather && !bar.wait()) return;
       }

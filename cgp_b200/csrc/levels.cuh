@@ -75,9 +75,9 @@ int enqueue_level_t(const LevelLaunch& L, cudaStream_t s) {
     k_sssp_push<W, OT, WK><<<t, kBlock, 0, s>>>(L.g, L.G);
     if (kt) kt->mark(kClassSsspDense, s);
     if (L.dense_unroll == 2)
-      k_sssp_dense<W, OT, WK, 2><<<L.gr.dense2, kBlock, 0, s>>>(L.g, L.G);
+      k_sssp_list<W, OT, WK, 8><<<L.gr.dense2, kBlock, 0, s>>>(L.g, L.G);
     else
-      k_sssp_dense<W, OT, WK, 1><<<L.gr.dense, kBlock, 0, s>>>(L.g, L.G);
+      k_sssp_list<W, OT, WK, 4><<<L.gr.dense, kBlock, 0, s>>>(L.g, L.G);
     n += 2;
     if (L.heavy_push) {
       if (kt) kt->mark(kClassSsspHeavy, s);
@@ -147,8 +147,8 @@ Grids grids_t(int sms) {
     gather_heavy_vec2 = occupancy_grid(k_sssp_pull_heavy_vec<W, OT, WK, 2>, sms);
     gather = occupancy_grid(k_sssp_pull<W, OT, WK>, sms);
     gather_heavy = occupancy_grid(k_sssp_pull_heavy<W, OT, WK>, sms);
-    dense = occupancy_grid(k_sssp_dense<W, OT, WK, 1>, sms);
-    dense2 = occupancy_grid(k_sssp_dense<W, OT, WK, 2>, sms);
+    dense = occupancy_grid(k_sssp_list<W, OT, WK, 4>, sms);
+    dense2 = occupancy_grid(k_sssp_list<W, OT, WK, 8>, sms);
     int a = occupancy_grid(k_bfs_push<W, OT, DEPTH>, sms);
     int b = occupancy_grid(k_bfs_pull<W, OT, DEPTH>, sms);
     int c = occupancy_grid(k_sssp_push<W, OT, WK>, sms);

@@ -90,6 +90,7 @@ __global__ void k_admit(GroupDev g, DevGraph G, const AdmitReq* reqs, int n) {
         atomic_or64(&ctl->ssel[w], bit);
         atomicAnd(reinterpret_cast<unsigned long long*>(&ctl->bfs_bits[w]), ~bit);
       }
+      if (r.kind == 3) ctl->khop = 1;
       if (r.kind == 3 && r.k <= 0)
         atomicAnd(reinterpret_cast<unsigned long long*>(&ctl->expand[w]), ~bit);
       else

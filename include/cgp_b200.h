@@ -105,7 +105,7 @@ typedef struct {
   int32_t max_queries;        /* run_options::max_queries; 0 = unlimited         */
   int32_t discard_results;    /* run_options::discard_results                    */
   int32_t profile_kernels;    /* time kernel classes with CUDA events (slower; no graphs) */
-  int32_t dense_unroll;       /* edges per step of the dense SSSP kernel: 1 or 2; 0 = 1 */
+  int32_t dense_unroll;       /* edges per step of the SSSP list kernel: 1: 4, 2: 8; 0 = 1 */
   double sssp_pull_edge_ratio; /* SSSP levels gather (pull) when frontier edges >= ratio * E;
                                   <= 0: always scatter (push)                              */
   int32_t light_chunks;       /* SSSP gathers take light vertices in CTA chunks (wider groups
