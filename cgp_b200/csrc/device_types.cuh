@@ -110,6 +110,7 @@ struct LevelCtl {
   unsigned long long prev_pull_edges; // in-edges the previous BFS pull level read
   int32_t prev_dir;                 // BFS direction of the previous level
   int32_t bfs_chunked;              // the BFS pull may run in CTA chunks (chunk table built)
+  int32_t has_bfs;                  // the group has BFS or k-hop slots
   int32_t khop;                     // the group has held k-hop slots: expand is recomputed
   int32_t bnd_avail;                // bounds arrays exist and the gather kernels read them
   int32_t bnd_on;                   // this gather level screens row chunks by bounds
@@ -156,6 +157,7 @@ struct DevGraph {
   const int32_t* plight;             // light vertices of the pull CSR (chunked gathers)
   const int32_t* plight_chunk_start; // [n_plight_chunks + 1]
   const int64_t* plight_beg;         // first pull-CSR in-edge of plight[i]
+  int32_t n_plight;                  // entries of plight
   int32_t n_plight_chunks;
   const int32_t* gitem_start;        // [n_gitems + 1] row gather items: runs of plight entries
   const int32_t* gitem_pre;          // in-edges of plight[i]'s item up to and including it
@@ -167,7 +169,8 @@ struct DevGraph {
   int32_t n_sheavy;
   int64_t sheavy_chunks;
   int32_t hub;                       // a vertex of largest in-degree (reference row of the bounds)
-  int32_t n_pmid;                    // plight[0 .. n_pmid) have in-degree > 32 (BFS pull mid kernel)
+  int32_t n_pmid;                    // plight[0 .. n_pmid) have in-degree > mid_degree
+  int32_t mid_degree;                // (BFS pull: a warp per vertex above it, a lane below)
 };
 
 struct GroupDev {

@@ -182,8 +182,10 @@ DevGraph GraphImpl::dev_graph(int64_t h, bool light_items) {
   d.plight = hp.plight.vertices.as<int32_t>();
   d.plight_chunk_start = hp.plight.chunk_start.as<int32_t>();
   d.plight_beg = hp.plight.beg.as<int64_t>();
+  d.n_plight = hp.plight.n;
   d.n_plight_chunks = hp.plight.chunks;
   d.n_pmid = hp.plight.n_mid;
+  d.mid_degree = hp.plight.mid_degree;
   d.gitem_start = hp.plight.item_start.as<int32_t>();
   d.gitem_pre = hp.plight.item_pre.as<int32_t>();
   d.n_gitems = hp.plight.items;
@@ -251,7 +253,8 @@ void build_heavy(const std::vector<int64_t>& row, int64_t V, int64_t h, HeavyTab
      "upload heavy chunks");
 }
 
-void build_light_chunks(const std::vector<int64_t>& row, int64_t V, int64_t h, LightChunks& t) {
+void build_light_chunks(const std::vector<int64_t>& row, int64_t V, int64_t h, int sms,
+                        LightChunks& t) {
   // light vertices by in-degree, largest first (ties by id): CTAs take chunks
   // roughly in this order, so within a gather level the better-connected
   // vertices settle first and the rest read their lowered distances
@@ -285,18 +288,39 @@ void build_light_chunks(const std::vector<int64_t>& row, int64_t V, int64_t h, L
   if (cur_v > 0) cs.push_back(static_cast<int32_t>(vs.size()));
   t.n = static_cast<int32_t>(vs.size());
   t.chunks = static_cast<int32_t>(cs.size()) - 1;
-  t.n_mid = 0;
-  while (t.n_mid < t.n && row[vs[t.n_mid] + 1] - row[vs[t.n_mid]] > 32) ++t.n_mid;
+  // BFS pull: a warp per vertex above mid_degree in-edges, a lane below.  Where
+  // the warps of the GPU hold every vertex of more than 8 at once, those get
+  // one each: a lane walks 32 in-edges in 8 dependent steps, a warp in one.
+  const int64_t warps = 24 * static_cast<int64_t>(sms);
+  auto above = [&](int64_t d) {
+    int32_t n = 0;
+    while (n < t.n && row[vs[n] + 1] - row[vs[n]] > d) ++n;
+    return n;
+  };
+  t.n_mid = above(8);
+  t.mid_degree = 8;
+  if (t.n_mid > 2 * warps) {
+    t.n_mid = above(32);
+    t.mid_degree = 32;
+  }
   // per entry: its first in-edge; and the row gather's items with their
   // in-edge prefixes, so that an item's header is three independent loads
   std::vector<int64_t> beg(vs.size());
   std::vector<int32_t> pre(vs.size()), is;
   int32_t run = 0, acc = 0;
+  // two items for each warp of the GPU at least: a 96 x 97 grid in items of 32
+  // vertices is 290 warps' serial work
+  int64_t edges = 0;
+  for (const int32_t v : vs) edges += std::min<int64_t>(row[v + 1] - row[v], dev::kGatherHeavy);
+  const int32_t most_v = static_cast<int32_t>(
+      std::min<int64_t>(32, std::max<int64_t>(1, static_cast<int64_t>(vs.size()) / (2 * warps))));
+  const int64_t most_e =
+      std::min<int64_t>(dev::kGatherHeavy, std::max<int64_t>(32, edges / (2 * warps)));
   for (size_t i = 0; i < vs.size(); ++i) {
     beg[i] = row[vs[i]];
     const int64_t d = row[vs[i] + 1] - row[vs[i]];
     if (d > dev::kGatherHeavy) continue;
-    if (is.empty() || run == 32 || acc + d > dev::kGatherHeavy) {
+    if (is.empty() || run == most_v || acc + d > most_e) {
       is.push_back(static_cast<int32_t>(i));
       run = 0;
       acc = 0;
@@ -340,7 +364,7 @@ const HeavyPair& GraphImpl::heavy_for(int64_t h) {
     build_heavy(hc.trow.empty() ? hc.row : hc.trow, V, h, hp->pheavy);
     build_heavy(hc.trow.empty() ? hc.row : hc.trow, V, std::min<int64_t>(h, dev::kGatherHeavy),
                 hp->gheavy);
-    build_light_chunks(hc.trow.empty() ? hc.row : hc.trow, V, h, hp->plight);
+    build_light_chunks(hc.trow.empty() ? hc.row : hc.trow, V, h, num_sms, hp->plight);
   }
   return *heavy_cache.emplace(h, std::move(hp)).first->second;
 }
@@ -615,6 +639,7 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
   c.chunk_dir = sssp_chunk_dir(spec, o) ? 1 : 0;
   c.bfs_chunked = (spec.has_bfs && (o.bfs_pull_form == 1 || o.bfs_pull_form == 2) &&
                    hp.plight.chunks > 0) ? o.bfs_pull_form : 0;
+  c.has_bfs = spec.has_bfs ? 1 : 0;
   c.bnd_avail = spec.bounds ? 1 : 0;
   c.prev_dir = kDirPush;
   c.sssp_pull_edge_threshold = static_cast<unsigned long long>(
@@ -682,7 +707,7 @@ bool fused_loop(const GroupSpec& spec, const cgp_options& o, const Dispatch& d,
   // serving groups on streams of their own: launched levels of different
   // groups overlap on the device, cooperative launches take all of it in turn
   if (spec.serving && (o.serve_groups > 1 || o.serve_admission == 2)) return false;
-  if (d.traverse(spec.has_bfs, spec.has_sssp).per_sm < 1) return false;
+  if (d.traverse(spec.has_sssp).per_sm < 1) return false;
   if (spec.has_sssp && (L.dense_unroll == 2 || (L.spull && !(L.gvec && L.lchunks)))) return false;
   return true;
 }
@@ -695,10 +720,10 @@ constexpr int kFusedLevels = 256;
 // Enqueues up to `levels` levels as one cooperative launch.
 int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelLaunch& L,
                   cudaStream_t s, int levels) {
-  const TraverseKernel k = d.traverse(spec.has_bfs, spec.has_sssp);
+  const TraverseKernel k = d.traverse(spec.has_sssp);
   const int most = k.per_sm * g->num_sms;
   const int blocks = static_cast<int>(std::max<int64_t>(
-      1, std::min<int64_t>(most, (g->E + g->V) / 512)));
+      1, std::min<int64_t>(most, (g->E + g->V) / 256)));
   bool heavy = L.heavy_push;
   void* args[] = {&L.g, &L.G, &levels, &heavy};
   ck(cudaLaunchCooperativeKernel(k.fn, dim3(blocks), dim3(kBlock), args, 0, s), "fused level loop");

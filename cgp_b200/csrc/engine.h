@@ -72,7 +72,8 @@ struct LightChunks {
   int32_t n = 0;
   int32_t chunks = 0;
   int32_t items = 0;
-  int32_t n_mid = 0;   // the first n_mid have in-degree > 32
+  int32_t mid_degree = 32;
+  int32_t n_mid = 0;   // the first n_mid have in-degree > mid_degree
 };
 
 struct HeavyPair {

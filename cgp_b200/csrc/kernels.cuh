@@ -16,6 +16,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include <cuda_runtime.h>
 
@@ -210,11 +211,26 @@ __device__ __forceinline__ LevelView level_view(const GroupDev& g) {
 // nothing to do.  (The heavy queue holds every vertex of out-degree > 32.)
 constexpr unsigned long long kSmallFrontier = 4096;
 
+// ... and at most this many out-edges stay with a tile on any level: a frontier
+// of 86K vertices is one tile per warp, and a list of 2,000 edges among them was
+// the level's whole time (R-MAT 20, 256 slots, 7.4M pairs: 1.6 ms).
+constexpr int64_t kTileDegree = 256;
+
 __device__ __forceinline__ int64_t push_light_limit(const GroupDev& g, const DevGraph& G,
                                                     unsigned long long count,
                                                     unsigned long long edges) {
   const bool spread = count <= kSmallFrontier || edges > 64ULL * count;
-  return (g.hq_vertex != nullptr && spread && G.heavy_degree > 32) ? 32 : G.heavy_degree;
+  if (g.hq_vertex == nullptr || G.heavy_degree <= 32) return G.heavy_degree;
+  return spread ? 32 : min(G.heavy_degree, kTileDegree);
+}
+
+// Frontier vertices per tile: 32, or fewer (a power of two) while that leaves
+// warps without a tile.  The lanes share a tile's edges either way, so a small
+// frontier is spread over more warps, each with a shorter chain of steps.
+__device__ __forceinline__ int tile_width(unsigned long long n, unsigned long long nwarps) {
+  int w = 1;
+  while (w < 32 && static_cast<unsigned long long>(w) * nwarps < n) w <<= 1;
+  return w;
 }
 
 // ------------------------------------------------------- depth recording
@@ -386,9 +402,10 @@ __device__ __forceinline__ void bfs_push_tiles(const GroupDev& g, const DevGraph
   for (int i = 0; i < W; ++i) uni[i] = 0;
   unsigned long long pairs = 0;
 
-  for (unsigned long long tile = gw; tile * 32 < n; tile += nw) {
-    const unsigned long long idx = tile * 32 + lane;
-    const bool valid = idx < n;
+  const int tw = tile_width(n, nw);
+  for (unsigned long long tile = gw; tile * tw < n; tile += nw) {
+    const unsigned long long idx = tile * tw + lane;
+    const bool valid = lane < tw && idx < n;
     int32_t u = valid ? lv.list[idx] : 0;
     int64_t beg = 0, end = 0;
     uint64_t f[W];
@@ -492,7 +509,7 @@ template <typename OT>
 __device__ __forceinline__ void heavy_queue_scan(const GroupDev& g, const DevGraph& G,
                                                  unsigned bid, unsigned nblk) {
   LevelCtl* ctl = g.ctl;
-  if (ctl->done || (ctl->dir != kDirPush && !ctl->sscatter)) return;
+  if (ctl->done || ((ctl->dir != kDirPush || !ctl->has_bfs) && !ctl->sscatter)) return;
   const LevelView lv = level_view(g);
   const unsigned long long n = ctl->count[lv.par];
   const int64_t light = push_light_limit(g, G, n, ctl->edges[lv.par]);
@@ -717,19 +734,26 @@ __device__ __forceinline__ void bfs_pull_tiles(const GroupDev& g, const DevGraph
       for (int i = 0; i < W; ++i) need[i] = ~vis[i] & act[i];
     }
     const int64_t deg = end - beg;
-    // heavy lists are the heavy kernels'; lists of 33 .. heavy_degree in-edges
-    // are k_bfs_pull_mid's when the light table lists them
-    const bool heavy = deg > G.heavy_degree || (G.n_pmid > 0 && deg > 32);
+    // heavy lists are the heavy kernels'; lists of mid_degree + 1 .. heavy_degree
+    // in-edges are k_bfs_pull_mid's when the light table lists them
+    const bool heavy = deg > G.heavy_degree || (G.n_pmid > 0 && deg > G.mid_degree);
     const bool work = valid && !heavy && deg > 0 && mask_any<W>(need);
     pverts += work ? 1 : 0;
     if (work && deg <= 32) {
       const uint32_t nch = chunk_bits<W>(need);
       // four in-edges per step: their column and mask loads are independent
       // and stay in flight together; early exit is checked once per step
+      // (and the next step's columns are loaded a step ahead)
+      int32_t un[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) un[j] = (beg + j < end) ? G.pcol[beg + j] : -1;
       for (int64_t e = beg; e < end; e += 4) {
         int32_t us[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) us[j] = (e + j < end) ? G.pcol[e + j] : -1;
+        for (int j = 0; j < 4; ++j) {
+          us[j] = un[j];
+          un[j] = (e + 4 + j < end) ? G.pcol[e + 4 + j] : -1;
+        }
         if (use_sum) {
 #pragma unroll
           for (int j = 0; j < 4; ++j)
@@ -957,7 +981,7 @@ __global__ void __launch_bounds__(kBlock) k_bfs_pull_chunked(GroupDev g, DevGrap
   warp_add(pedges, &g.ctl->lc.pull_edges, lane);
 }
 
-// Pull level, vertices with 33 .. heavy_degree in-edges (the first n_pmid
+// Pull level, vertices with mid_degree + 1 .. heavy_degree in-edges (the first n_pmid
 // entries of the pull CSR's light table, largest first): a warp per vertex,
 // 64 in-edges per step (two column -> mask loads in flight per lane, then a
 // warp OR-reduce and the early-exit test), one commit per vertex.  In the
@@ -1003,10 +1027,15 @@ __device__ __forceinline__ void bfs_pull_mid(const GroupDev& g, const DevGraph& 
       const int64_t beg = row_at<OT>(G.prow, v);
       const int64_t end = row_at<OT>(G.prow, static_cast<int64_t>(v) + 1);
       const uint32_t nch = chunk_bits<W>(need);
+      // the next step's columns are in flight while this one's masks load
+      int32_t n0 = -1, n1 = -1;
+      if (beg + lane < end) n0 = G.pcol[beg + lane];
+      if (beg + 32 + lane < end) n1 = G.pcol[beg + 32 + lane];
       for (int64_t e0 = beg; e0 < end; e0 += 64) {
-        int32_t u0 = -1, u1 = -1;
-        if (e0 + lane < end) u0 = G.pcol[e0 + lane];
-        if (e0 + 32 + lane < end) u1 = G.pcol[e0 + 32 + lane];
+        int32_t u0 = n0, u1 = n1;
+        n0 = n1 = -1;
+        if (e0 + 64 + lane < end) n0 = G.pcol[e0 + 64 + lane];
+        if (e0 + 96 + lane < end) n1 = G.pcol[e0 + 96 + lane];
         pedges += (u0 >= 0 ? 1 : 0) + (u1 >= 0 ? 1 : 0);
         if (use_sum) {
           if (u0 >= 0 && !(summary_chunks(g.fsum, lv.level, u0) & nch)) u0 = -1;
@@ -1390,9 +1419,10 @@ __device__ __forceinline__ void sssp_push_tiles(const GroupDev& g, const DevGrap
   const unsigned long long nwarps = (static_cast<unsigned long long>(nblk) * blockDim.x) >> 5;
   const size_t Qg = static_cast<size_t>(g.Qg);
   unsigned long long improved = 0, spairs = 0, sactive = 0;
-  for (unsigned long long tile = gw; tile * 32 < n; tile += nwarps) {
-    const unsigned long long idx = tile * 32 + lane;
-    const bool valid = idx < n;
+  const int tw = tile_width(n, nwarps);
+  for (unsigned long long tile = gw; tile * tw < n; tile += nwarps) {
+    const unsigned long long idx = tile * tw + lane;
+    const bool valid = lane < tw && idx < n;
     const int32_t u = valid ? lv.list[idx] : 0;
     int64_t beg = 0, end = 0;
     int k = 0;
@@ -1690,13 +1720,12 @@ __global__ void __launch_bounds__(kBlock) k_sssp_push_heavy(GroupDev g, DevGraph
 // Several in-edges are in flight per warp (GatherSteps) to cover latency.
 
 // Relaxation of a stored value `du` over an edge with raw weight bits.  The
-// unreached markers (0xffffffff; +inf for f32) never improve anything.
+// unreached markers (0xffffffff; +inf for f32, whose sums stay +inf or become a
+// NaN, larger than every value as a uint32) never improve anything.
 template <int WK>
 __device__ __forceinline__ uint32_t gather_relax(uint32_t du, uint32_t wbits) {
   if constexpr (WK == kWeightF32) {
-    return du >= 0x7f800000u
-               ? 0xffffffffu
-               : __float_as_uint(__fadd_rn(__uint_as_float(du), __uint_as_float(wbits)));
+    return __float_as_uint(__fadd_rn(__uint_as_float(du), __uint_as_float(wbits)));
   } else {
     const uint32_t wt = (WK == kWeightU32) ? wbits : 1u;
     return min(du, ~wt) + wt;  // saturates at 0xffffffff
@@ -1939,6 +1968,26 @@ __device__ __forceinline__ void load_vec_cg(const uint32_t* p, uint32_t* x) {
   }
 }
 
+// load_vec_cg under a predicate; x keeps its values where on is 0.  (As an if
+// the compiler branches around each load, and the rows of a step are no longer
+// in flight together: R-MAT 20 gather levels 0.73 -> 1.1 ms.)
+template <int E>
+__device__ __forceinline__ void load_vec_cg_if(uint32_t on, const uint32_t* p, uint32_t* x) {
+  if constexpr (E == 4) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %4, 0;\n\t"
+        "@q ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%5];\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3])
+        : "r"(on), "l"(p));
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t"
+        "@q ld.global.cg.v2.u32 {%0, %1}, [%3];\n\t}"
+        : "+r"(x[0]), "+r"(x[1])
+        : "r"(on), "l"(p));
+  }
+}
+
 template <int E>
 __device__ __forceinline__ void load_vec(const uint32_t* p, uint32_t* x) {
   if constexpr (E == 4) {
@@ -1956,19 +2005,75 @@ __device__ __forceinline__ void store_vec(uint32_t* p, const uint32_t* x) {
   else *reinterpret_cast<uint2*>(p) = make_uint2(x[0], x[1]);
 }
 
-// best[j] = min(best[j], relax(du[j], w)) for the lane's slots.
-template <int WK, int N>
-__device__ __forceinline__ void relax_min_row(uint32_t (&best)[N], const uint32_t* du,
-                                              uint32_t wbits) {
+// Weight of a row chunk that was not read: relaxing with it changes nothing,
+// whatever the registers hold.
+template <int WK>
+__device__ __forceinline__ uint32_t dead_weight() {
+  return WK == kWeightF32 ? 0x7f800000u : 0xffffffffu;
+}
+
+// best[j] = min(best[j], du[j] + w) for the E slots of one part; w is a raw
+// weight (1 on unweighted graphs) or dead_weight().
+template <int WK, int E>
+__device__ __forceinline__ void relax_part(uint32_t* best, const uint32_t* du, uint32_t w) {
   if constexpr (WK == kWeightF32) {
 #pragma unroll
-    for (int j = 0; j < N; ++j) best[j] = min(best[j], gather_relax<WK>(du[j], wbits));
+    for (int k = 0; k < E; ++k)
+      best[k] = min(best[k], __float_as_uint(__fadd_rn(__uint_as_float(du[k]), __uint_as_float(w))));
   } else {
-    const uint32_t wt = (WK == kWeightU32) ? wbits : 1u;
-    const uint32_t lim = ~wt;
+    const uint32_t lim = ~w;
 #pragma unroll
-    for (int j = 0; j < N; ++j) best[j] = min(best[j], min(du[j], lim) + wt);
+    for (int k = 0; k < E; ++k) best[k] = min(best[k], min(du[k], lim) + w);
   }
+}
+
+// Reads rows stage[i .. i + S) of a staging list of n (all of them when kWhole)
+// into cur, for the lane's slots.  pbit[r] is the row chunk of the lane's part
+// r, 0 when the lane has no gathering slot there.  Without kChunks every chunk
+// is read.  Parts that are not read keep what the registers held.  (The
+// entries are read again when they are relaxed: held across the loads they
+// cost 4 registers a row, and the row gather spilled.)
+template <int W, bool kChunks, bool kWhole, int S>
+__device__ __forceinline__ void load_rows(const uint32_t* lanebase, unsigned Qg, const int4* stage,
+                                          int i, int n,
+                                          const uint32_t (&pbit)[GatherVec<W>::kParts],
+                                          uint32_t (&cur)[S][GatherVec<W>::kSlots]) {
+  using GV = GatherVec<W>;
+  constexpr int E = GV::kElem;
+#pragma unroll
+  for (int t = 0; t < S; ++t) {
+    if (!kWhole && i + t >= n) break;  // uniform
+    const uint32_t u = static_cast<uint32_t>(stage[i + t].x);
+    const uint32_t cm = kChunks ? static_cast<uint32_t>(stage[i + t].w) : 0xffffffffu;
+    const uint32_t* row = lanebase + static_cast<uint64_t>(u) * Qg;
+#pragma unroll
+    for (int r = 0; r < GV::kParts; ++r)
+      load_vec_cg_if<E>(cm & pbit[r], row + 32 * E * r, &cur[t][r * E]);
+  }
+}
+
+// Relaxes one loaded row (weight w, row chunks cm).
+template <int W, int WK, bool kChunks>
+__device__ __forceinline__ void relax_row(uint32_t (&best)[GatherVec<W>::kSlots],
+                                          const uint32_t (&cur)[GatherVec<W>::kSlots], uint32_t w,
+                                          uint32_t cm,
+                                          const uint32_t (&pbit)[GatherVec<W>::kParts]) {
+  using GV = GatherVec<W>;
+  if (WK == kWeightNone) w = 1u;
+#pragma unroll
+  for (int r = 0; r < GV::kParts; ++r)
+    relax_part<WK, GV::kElem>(&best[r * GV::kElem], &cur[r * GV::kElem],
+                              !kChunks || (cm & pbit[r]) ? w : dead_weight<WK>());
+}
+
+// The lane's row chunks, part by part (see load_rows).
+template <int W>
+__device__ __forceinline__ void part_chunks(uint32_t pmask, int lane,
+                                            uint32_t (&pbit)[GatherVec<W>::kParts]) {
+  using GV = GatherVec<W>;
+#pragma unroll
+  for (int r = 0; r < GV::kParts; ++r)
+    pbit[r] = (pmask >> r) & 1u ? 1u << (((32 * r + lane) * GV::kElem) >> 5) : 0u;
 }
 
 // Lane masks for the vectorised gather: bit r of *parts: the lane's vector of
@@ -2092,14 +2197,6 @@ __global__ void __launch_bounds__(kBlock) k_frontier_summary(GroupDev g, DevGrap
   frontier_summary<W, OT>(g, G, blockIdx.x, gridDim.x);
 }
 
-// Whether the lane reads part r of a source row whose 32-slot chunk bits are
-// `cm`.
-template <int W>
-__device__ __forceinline__ bool chunk_live(uint32_t cm, int r, int lane) {
-  constexpr int E = GatherVec<W>::kElem;
-  return (cm >> (((32 * r + lane) * E) >> 5)) & 1u;
-}
-
 // ------------------------------------------------- bounds on row chunks
 // An in-edge (u, v) of weight w can lower v's slot q only if d[u][q] + w <
 // d[v][q].  With any reference value b[q] per slot, subtracted on both sides,
@@ -2116,38 +2213,39 @@ __device__ __forceinline__ bool chunk_live(uint32_t cm, int r, int lane) {
 // during a level, so a skipped chunk never hides an improvement: a vertex
 // lowered during the level is in the next frontier.
 //
-// uint32 distances: int32 offsets within +-2^30 (kBoundNone: no frontier
-// slot, or no upper bound); f32: the offsets as floats (+inf for both).
+// uint32 distances: int32 offsets within +-2^30, larger values clamped the safe
+// way (kBoundNone: no frontier slot, or no upper bound); f32: the offsets as
+// floats (+inf for both).
 constexpr uint32_t kBoundNone = 0x7fffffffu;
 constexpr uint32_t kBoundNoneF32 = 0x7f800000u;
+constexpr uint32_t kBoundMax = (1u << 30) - 1u;
 
 template <int WK>
 __device__ __forceinline__ uint32_t bound_none() {
   return WK == kWeightF32 ? kBoundNoneF32 : kBoundNone;
 }
 
+// Reference value of a slot: the hub's distance, 0 where there is none.
+template <int WK>
+__device__ __forceinline__ uint32_t bound_ref(uint32_t d) {
+  if constexpr (WK == kWeightF32) return d >= 0x7f800000u ? 0u : d;
+  else return d > kBoundMax ? 0u : d;
+}
+
 template <int WK>
 __device__ __forceinline__ uint32_t bound_low(uint32_t d, uint32_t b) {
-  if constexpr (WK == kWeightF32) {
+  if constexpr (WK == kWeightF32)
     return __float_as_uint(__fsub_rd(__uint_as_float(d), __uint_as_float(b)));
-  } else {
-    const long long x = static_cast<long long>(d) - static_cast<long long>(b);
-    return x < -(1LL << 30) ? 0x80000000u
-                            : static_cast<uint32_t>(static_cast<int32_t>(min(x, (1LL << 30) - 1)));
-  }
+  else
+    return min(d, kBoundMax) - b;
 }
 
 template <int WK>
 __device__ __forceinline__ uint32_t bound_high(uint32_t d, uint32_t b) {
-  if constexpr (WK == kWeightF32) {
-    return d >= 0x7f800000u ? kBoundNoneF32
-                            : __float_as_uint(__fsub_ru(__uint_as_float(d), __uint_as_float(b)));
-  } else {
-    const long long x = static_cast<long long>(d) - static_cast<long long>(b);
-    return d == 0xffffffffu || x >= (1LL << 30)
-               ? kBoundNone
-               : static_cast<uint32_t>(static_cast<int32_t>(max(x, -(1LL << 30))));
-  }
+  if constexpr (WK == kWeightF32)
+    return __float_as_uint(__fsub_ru(__uint_as_float(d), __uint_as_float(b)));  // inf stays inf
+  else
+    return d > kBoundMax ? kBoundNone : d - b;
 }
 
 template <int WK>
@@ -2174,7 +2272,7 @@ __device__ __forceinline__ bool bound_improves(uint32_t lo, uint32_t hi, uint32_
     return __fadd_rd(__uint_as_float(lo), __uint_as_float(wbits)) < __uint_as_float(hi);
   } else {
     // no sum of a clamped bound and a clamped weight reaches kBoundNone
-    const int32_t w = static_cast<int32_t>(min(WK == kWeightU32 ? wbits : 1u, (1u << 30) - 1u));
+    const int32_t w = static_cast<int32_t>(min(WK == kWeightU32 ? wbits : 1u, kBoundMax));
     return lo != kBoundNone && static_cast<int32_t>(lo) + w < static_cast<int32_t>(hi);
   }
 }
@@ -2198,11 +2296,12 @@ __device__ __forceinline__ uint32_t bound_chunks(const uint32_t* lo, const uint3
   return cm;
 }
 
-// Writes both bounds of every vertex at the start of a gather level that uses
-// them (a warp per vertex and slice of WS words: one pass over the values) and
-// counts the live chunks, as the frontier summary does on other levels.  R-MAT
-// 20, 256 slots: about 0.15 ms against 3.4 ms for a level that reads every
-// source row.
+// Writes both bounds of every vertex with in-edges at the start of a gather
+// level that uses them (a warp per vertex and slice of WS words: one pass over
+// their values) and counts the live chunks, as the frontier summary does on
+// other levels.  A vertex without in-edges has nothing lowered and is in no
+// frontier after the first: its bounds are never written and whatever they
+// hold skips or reads rows that change nothing.
 template <int W, typename OT, int WK>
 __device__ __forceinline__ void gather_bounds(const GroupDev& g, const DevGraph& G, unsigned bid,
                                               unsigned nblk) {
@@ -2213,11 +2312,15 @@ __device__ __forceinline__ void gather_bounds(const GroupDev& g, const DevGraph&
   constexpr int E = GV::kElem;
   constexpr int P = GV::kParts;
   constexpr int L = GV::kLanesPerHalf;
+  constexpr uint32_t kNone = WK == kWeightF32 ? kBoundNoneF32 : kBoundNone;
+  constexpr uint32_t kLeast = WK == kWeightF32 ? 0xff800000u : 0x80000000u;
   const LevelView lv = level_view(g);
   const int lane = threadIdx.x & 31;
   const size_t Qg = static_cast<size_t>(g.Qg);
-  const long long gw = (static_cast<long long>(bid) * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = (static_cast<long long>(nblk) * blockDim.x) >> 5;
+  const int n_light = G.n_plight;
+  const int n = n_light + G.n_pheavy;
+  const int gw = static_cast<int>((static_cast<long long>(bid) * blockDim.x + threadIdx.x) >> 5);
+  const int nwarps = static_cast<int>((static_cast<long long>(nblk) * blockDim.x) >> 5);
   unsigned long long live = 0;
   for (int sl = 0; sl < W / WS; ++sl) {
     const int s0 = sl * 64 * WS;
@@ -2236,25 +2339,28 @@ __device__ __forceinline__ void gather_bounds(const GroupDev& g, const DevGraph&
         for (int k = 0; k < E; ++k) ref[r * E + k] = 0u;
       }
 #pragma unroll
-      for (int k = 0; k < E; ++k)  // a slot that has not reached the hub: no offset
-        if (ref[r * E + k] >= (WK == kWeightF32 ? 0x7f800000u : 0xffffffffu)) ref[r * E + k] = 0u;
+      for (int k = 0; k < E; ++k) ref[r * E + k] = bound_ref<WK>(ref[r * E + k]);
     }
-    // two vertices per step, every load of both in flight at once (a row that
-    // turns out to be neither source nor destination is read all the same)
+    // two vertices per step, every load of both in flight at once; the next
+    // step's vertex ids are loaded a step ahead
     constexpr int U = 2;
-    for (long long v0 = gw * U; v0 < G.V; v0 += nwarps * U) {
+    auto vertex = [&](int i) { return i < n_light ? G.plight[i] : G.pheavy[i - n_light]; };
+    int32_t nv[U];
+#pragma unroll
+    for (int t = 0; t < U; ++t) nv[t] = gw + t * nwarps < n ? vertex(gw + t * nwarps) : 0;
+    for (int i0 = gw; i0 < n; i0 += nwarps * U) {
+      int32_t v[U];
       uint32_t d[U][GV::kSlots];
       uint32_t fr[U][P];  // the lane's frontier bits
 #pragma unroll
       for (int t = 0; t < U; ++t) {
-        const size_t v = static_cast<size_t>(v0 + t < G.V ? v0 + t : v0);
+        v[t] = nv[t];
 #pragma unroll
         for (int r = 0; r < P; ++r) {
           const int q = s0 + (32 * r + lane) * E;
-          fr[t][r] = static_cast<uint32_t>(lv.fcur[v * W + (q >> 6)] >> (q & 63)) &
-                     (smask >> (r * E)) & ((1u << E) - 1u);
+          fr[t][r] = static_cast<uint32_t>(lv.fcur[static_cast<size_t>(v[t]) * W + (q >> 6)] >> (q & 63));
           if ((pmask >> r) & 1u) {
-            load_vec<E>(g.values + v * Qg + q, &d[t][r * E]);
+            load_vec<E>(g.values + static_cast<size_t>(v[t]) * Qg + q, &d[t][r * E]);
           } else {
 #pragma unroll
             for (int k = 0; k < E; ++k) d[t][r * E + k] = 0u;
@@ -2263,18 +2369,24 @@ __device__ __forceinline__ void gather_bounds(const GroupDev& g, const DevGraph&
       }
 #pragma unroll
       for (int t = 0; t < U; ++t) {
-        const long long v = v0 + t;
-        if (v >= G.V) break;  // uniform
+        const int i = i0 + (U + t) * nwarps;
+        if (i < n) nv[t] = vertex(i);
+      }
+#pragma unroll
+      for (int t = 0; t < U; ++t) {
+        if (i0 + t * nwarps >= n) break;  // uniform
         uint32_t chunks = 0;
 #pragma unroll
         for (int r = 0; r < P; ++r) {
-          uint32_t lo = bound_none<WK>();
-          uint32_t hi = WK == kWeightF32 ? 0xff800000u : 0x80000000u;
+          const uint32_t fs = fr[t][r] & (smask >> (r * E));
+          uint32_t lo = kNone, hi = kLeast;
 #pragma unroll
           for (int k = 0; k < E; ++k) {
             const uint32_t x = d[t][r * E + k], b = ref[r * E + k];
-            if ((fr[t][r] >> k) & 1u) lo = bound_min<WK>(lo, bound_low<WK>(x, b));
-            if ((smask >> (r * E + k)) & 1u) hi = bound_max<WK>(hi, bound_high<WK>(x, b));
+            const uint32_t xl = (fs >> k) & 1u ? bound_low<WK>(x, b) : kNone;
+            const uint32_t xh = (smask >> (r * E + k)) & 1u ? bound_high<WK>(x, b) : kLeast;
+            lo = bound_min<WK>(lo, xl);
+            hi = bound_max<WK>(hi, xh);
           }
 #pragma unroll
           for (int o = L / 2; o > 0; o >>= 1) {
@@ -2283,13 +2395,13 @@ __device__ __forceinline__ void gather_bounds(const GroupDev& g, const DevGraph&
           }
           if (lane % L == 0) {
             const size_t at =
-                static_cast<size_t>(v) * (2 * W) + sl * 2 * WS + (32 / L) * r + lane / L;
+                static_cast<size_t>(v[t]) * (2 * W) + sl * 2 * WS + (32 / L) * r + lane / L;
             g.blo[at] = lo;
             g.bhi[at] = hi;
-            chunks += lo != bound_none<WK>() ? 1u : 0u;
+            chunks += lo != kNone ? 1u : 0u;
           }
         }
-        if (chunks) live += chunks * degree_of<OT>(G.row, static_cast<int32_t>(v));
+        if (chunks) live += chunks * degree_of<OT>(G.row, v[t]);
       }
     }
   }
@@ -2314,10 +2426,11 @@ __device__ __forceinline__ void gather_edges_vec(const GroupDev& g, const DevGra
                                                  uint32_t gch, const uint32_t* hi = nullptr) {
   using GV = GatherVec<W>;
   constexpr int E = GV::kElem;
-  constexpr int P = GV::kParts;
   constexpr int S = GV::kSteps;
   const size_t Qg = static_cast<size_t>(g.Qg);
   const uint32_t* lanebase = g.values + lane * E;
+  uint32_t pbit[GV::kParts];
+  part_chunks<W>(pmask, lane, pbit);
   for (int64_t e0 = eb; e0 < ee; e0 += 32) {
     const int64_t e = e0 + lane;
     int k = 0;
@@ -2358,53 +2471,28 @@ __device__ __forceinline__ void gather_edges_vec(const GroupDev& g, const DevGra
     const unsigned lm = __ballot_sync(kFull, k > 0);
     if (k > 0)
       stage[__popc(lm & ((1u << lane) - 1u))] =
-          make_int4(u, static_cast<int>(wb), 0, kChunks ? static_cast<int>(cm) : -1);
+          make_int4(u, static_cast<int>(wb), 0, static_cast<int>(cm));
     __syncwarp();
     const int n = __popc(lm);
     int i = 0;
+    uint32_t cur[S][GV::kSlots] = {};
+    auto relax = [&](int t) {
+      const int4 ed = stage[i + t];
+      relax_row<W, WK, kChunks>(best, cur[t], static_cast<uint32_t>(ed.y),
+                                static_cast<uint32_t>(ed.w), pbit);
+    };
     for (; i + S <= n; i += S) {
-      int4 ed[S];
+      load_rows<W, kChunks, true, S>(lanebase, static_cast<unsigned>(Qg), stage, i, n, pbit, cur);
 #pragma unroll
-      for (int t = 0; t < S; ++t) ed[t] = stage[i + t];
-      uint32_t cur[S][GV::kSlots];
-#pragma unroll
-      for (int t = 0; t < S; ++t) {
-        const uint32_t* row = lanebase + static_cast<size_t>(ed[t].x) * Qg;
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-          if (((pmask >> r) & 1u) && (!kChunks || chunk_live<W>(static_cast<uint32_t>(ed[t].w), r, lane))) {
-            load_vec_cg<E>(row + 32 * E * r, &cur[t][r * E]);
-          } else {
-#pragma unroll
-            for (int q = 0; q < E; ++q) cur[t][r * E + q] = 0xffffffffu;
-          }
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < S; ++t) relax_min_row<WK>(best, cur[t], static_cast<uint32_t>(ed[t].y));
+      for (int t = 0; t < S; ++t) relax(t);
     }
-    if (i < n) {
-      // the remaining 1..S-1 edges in one step (uniform predicates), so that
-      // a short list costs one round trip instead of one per edge
-      int4 ed[S];
-#pragma unroll
-      for (int t = 0; t < S; ++t) ed[t] = stage[i + t < n ? i + t : i];
-      uint32_t cur[S][GV::kSlots];
+    if (i < n) {  // the remaining 1 .. S-1 rows in one step
+      load_rows<W, kChunks, false, S>(lanebase, static_cast<unsigned>(Qg), stage, i, n, pbit, cur);
 #pragma unroll
       for (int t = 0; t < S; ++t) {
-        const uint32_t* row = lanebase + static_cast<size_t>(ed[t].x) * Qg;
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-          if (i + t < n && ((pmask >> r) & 1u) && (!kChunks || chunk_live<W>(static_cast<uint32_t>(ed[t].w), r, lane))) {
-            load_vec_cg<E>(row + 32 * E * r, &cur[t][r * E]);
-          } else {
-#pragma unroll
-            for (int q = 0; q < E; ++q) cur[t][r * E + q] = 0xffffffffu;
-          }
-        }
+        if (i + t >= n) break;
+        relax(t);
       }
-#pragma unroll
-      for (int t = 0; t < S; ++t) relax_min_row<WK>(best, cur[t], static_cast<uint32_t>(ed[t].y));
     }
     __syncwarp();
   }
@@ -2591,6 +2679,7 @@ constexpr int kRowStage = 64;  // 32 in-edges and as many own rows
 struct GatherRowSmem {
   int4 stage[kWarpsPerBlock][kRowStage];
   alignas(16) uint32_t hi[kWarpsPerBlock][32][8];
+  alignas(16) uint32_t own[kWarpsPerBlock][256];  // the row of the vertex in work as it was
 };
 
 template <int W, typename OT, int WK, int WF>
@@ -2611,22 +2700,23 @@ __device__ __forceinline__ void sssp_pull_light_rows(const GroupDev& g, const De
   const unsigned below = (1u << lane) - 1u;
   int4* stage = sm.stage[wib];
   uint32_t(*s_hi)[8] = sm.hi[wib];
+  uint32_t* own = sm.own[wib] + lane * E;
   const bool bounds = ctl->bnd_on != 0;
   const bool screened = gather_screen_qs<WF>(g, ctl, lv, G.E) < 0;
   // only this kernel adds bits to its vertices' next masks: plain stores
   const bool plain = !ctl->sscatter && !any_bits<WF>(ctl->bfs_bits);
-  const size_t Qg = static_cast<size_t>(g.Qg);
-  const long long n_items = G.n_gitems;
-  const long long total_items = n_items * (WF / W);
-  const long long gw = (static_cast<long long>(bid) * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = (static_cast<long long>(nblk) * blockDim.x) >> 5;
+  const unsigned Qg = static_cast<unsigned>(g.Qg);
+  const int n_items = G.n_gitems;
+  const int total_items = n_items * (WF / W);
+  const int gw = static_cast<int>((bid * blockDim.x + threadIdx.x) >> 5);
+  const int nwarps = static_cast<int>((nblk * blockDim.x) >> 5);
 
   int sl = -1;             // current slice
   uint32_t pmask = 0, smask = 0, gch = 0;
+  uint32_t pbit[P];
   int qs = 0;              // gathering slots of the slice
   uint32_t uacc = 0;       // union of the slice's improved bits
-  unsigned long long improved = 0, pairs = 0;
-  unsigned scanned = 0, verts = 0;
+  unsigned improved = 0, scanned = 0, verts = 0, pairs = 0;  // of this lane
   int32_t pend_v = 0;      // lane i: i-th vertex waiting to be appended
   int pend_n = 0;          // uniform
 
@@ -2649,27 +2739,28 @@ __device__ __forceinline__ void sssp_pull_light_rows(const GroupDev& g, const De
 
   // header of the next item: lane k holds its k-th vertex
   int32_t hv = 0, hpre = 0;
-  int64_t hbeg = 0;
+  OT hbeg = 0;
   int hnv = 0;
-  auto load_header = [&](long long it) {
-    const long long i = WF > W ? it % n_items : it;
+  auto load_header = [&](int it) {
+    const int i = WF > W ? it % n_items : it;
     const int cs = G.gitem_start[i];
     hnv = G.gitem_start[i + 1] - cs;
     if (lane < hnv) {
       hv = G.plight[cs + lane];
-      hbeg = G.plight_beg[cs + lane];
+      hbeg = static_cast<OT>(G.plight_beg[cs + lane]);
       hpre = G.gitem_pre[cs + lane];
     }
   };
   if (gw < total_items) load_header(gw);
-  for (long long it = gw; it < total_items; it += nwarps) {
-    const int nsl = WF > W ? static_cast<int>(it / n_items) : 0;
+  for (int it = gw; it < total_items; it += nwarps) {
+    const int nsl = WF > W ? it / n_items : 0;
     if (nsl != sl) {
       if (sl >= 0) flush_union_bits();
       sl = nsl;
       const uint64_t* sb = ctl->gsel + sl * W;
       gather_vec_masks<W>(sb, g.Qg - sl * 64 * W, lane, &pmask, &smask);
       gch = gather_chunks<W>(sb);
+      part_chunks<W>(pmask, lane, pbit);
       qs = 0;
 #pragma unroll
       for (int i = 0; i < W; ++i) qs += __popcll(sb[i]);
@@ -2679,7 +2770,7 @@ __device__ __forceinline__ void sssp_pull_light_rows(const GroupDev& g, const De
     const int total = __shfl_sync(kFull, hpre, nv - 1);
     int start = __shfl_up_sync(kFull, hpre, 1);
     if (lane == 0) start = 0;
-    const int64_t base = hbeg - start;  // in-edge f of the item: base + f
+    const OT base = hbeg - start;  // in-edge f of the item: base + f
     if (lane >= nv) start = 0x7fffffff;
     if (it + nwarps < total_items) load_header(it + nwarps);
     if (gch == 0) continue;  // no gathering slot in this slice
@@ -2702,22 +2793,23 @@ __device__ __forceinline__ void sssp_pull_light_rows(const GroupDev& g, const De
       for (int f = lane; f < total; f += 32) ++scanned;
     }
     const uint32_t* lanebase = g.values + sl * 64 * W + lane * E;
-    uint32_t best[GV::kSlots], own[GV::kSlots];
+    uint32_t best[GV::kSlots];
     int cur_k = -1;     // vertex in work (uniform)
     int32_t cur_v = 0;
     auto commit = [&]() {
       uint32_t imp = 0;
 #pragma unroll
       for (int r = 0; r < P; ++r) {
-        uint32_t b = 0;
+        uint32_t b = 0, o[E];
+        load_vec<E>(&own[32 * E * r], o);
 #pragma unroll
         for (int q = 0; q < E; ++q) {
           const int j = r * E + q;
-          const bool up = ((smask >> j) & 1u) && best[j] < own[j];
-          best[j] = up ? best[j] : own[j];
+          const bool up = ((smask >> j) & 1u) && best[j] < o[q];
+          best[j] = up ? best[j] : o[q];
           b |= static_cast<uint32_t>(up) << q;
         }
-        if (b) store_vec<E>(const_cast<uint32_t*>(lanebase) + static_cast<size_t>(cur_v) * Qg + 32 * E * r, &best[r * E]);
+        if (b) store_vec<E>(const_cast<uint32_t*>(lanebase) + static_cast<uint64_t>(static_cast<uint32_t>(cur_v)) * Qg + 32 * E * r, &best[r * E]);
         imp |= b << (r * E);
       }
       if (!__any_sync(kFull, imp != 0)) return;
@@ -2734,13 +2826,49 @@ __device__ __forceinline__ void sssp_pull_light_rows(const GroupDev& g, const De
       if (++pend_n == 32) flush_pending();
     };
 
+    // the staged rows: an own row commits the vertex before it and starts its
+    // vertex, the others are relaxed into it
+    auto walk = [&](auto chunks, int n) {
+      constexpr bool kChunks = decltype(chunks)::value;
+      uint32_t cur[S][GV::kSlots] = {};
+      int i = 0;
+      auto take = [&](int t) {
+        const int4 ed = stage[i + t];
+        if (ed.z < 0) {  // uniform
+          if (cur_k >= 0) commit();
+          cur_k = ~ed.z;
+          cur_v = ed.x;
+#pragma unroll
+          for (int j = 0; j < GV::kSlots; ++j) best[j] = cur[t][j];
+#pragma unroll
+          for (int r = 0; r < P; ++r) store_vec<E>(&own[32 * E * r], &best[r * E]);
+        } else {
+          relax_row<W, WK, kChunks>(best, cur[t], static_cast<uint32_t>(ed.y),
+                                    static_cast<uint32_t>(ed.w), pbit);
+        }
+      };
+      for (; i + S <= n; i += S) {
+        load_rows<W, kChunks, true, S>(lanebase, Qg, stage, i, n, pbit, cur);
+#pragma unroll
+        for (int t = 0; t < S; ++t) take(t);
+      }
+      if (i < n) {
+        load_rows<W, kChunks, false, S>(lanebase, Qg, stage, i, n, pbit, cur);
+#pragma unroll
+        for (int t = 0; t < S; ++t) {
+          if (i + t >= n) break;  // uniform
+          take(t);
+        }
+      }
+    };
+
     // in-edges f0 .. f0 + 31, lane by lane (the next batch is loaded ahead)
     int nk = 0;
     int32_t nu = 0;
     uint32_t nw = 0;
     auto load_batch = [&](int f0) {
       nk = chunk_edge_owner(start, f0, lane);
-      const int64_t e = __shfl_sync(kFull, base, nk) + f0 + lane;
+      const OT e = __shfl_sync(kFull, base, nk) + f0 + lane;
       if (f0 + lane < total) {
         nu = G.pcol[e];
         nw = weight_bits<WK>(G.pw, e);
@@ -2771,8 +2899,8 @@ __device__ __forceinline__ void sssp_pull_light_rows(const GroupDev& g, const De
       const bool live = cm != 0;
       const unsigned lm = __ballot_sync(kFull, live);
       if (lm == 0) continue;
-      pairs += (bounds || screened) ? static_cast<unsigned long long>(__popc(cm)) << 5
-                                    : (live ? static_cast<unsigned long long>(qs) : 0ULL);
+      pairs += (bounds || screened) ? static_cast<unsigned>(__popc(cm)) << 5
+                                    : (live ? static_cast<unsigned>(qs) : 0u);
       // the vertex's own row goes before its first live in-edge
       const unsigned lb = lm & below;
       const int kp = __shfl_sync(kFull, k, lb ? 31 - __clz(lb) : lane);
@@ -2784,38 +2912,8 @@ __device__ __forceinline__ void sssp_pull_light_rows(const GroupDev& g, const De
       if (first) stage[pos - 1] = make_int4(vk, 0, ~k, static_cast<int>(gch));
       __syncwarp();
       const int n = __popc(lm) + __popc(fm);
-      for (int i = 0; i < n; i += S) {
-        int4 ed[S];
-        uint32_t cur[S][GV::kSlots];
-#pragma unroll
-        for (int t = 0; t < S; ++t) {
-          ed[t] = stage[i + t < n ? i + t : i];
-          const uint32_t* row = lanebase + static_cast<size_t>(ed[t].x) * Qg;
-#pragma unroll
-          for (int r = 0; r < P; ++r) {
-            if (i + t < n && ((pmask >> r) & 1u) &&
-                chunk_live<W>(static_cast<uint32_t>(ed[t].w), r, lane)) {
-              load_vec_cg<E>(row + 32 * E * r, &cur[t][r * E]);
-            } else {
-#pragma unroll
-              for (int q = 0; q < E; ++q) cur[t][r * E + q] = 0xffffffffu;
-            }
-          }
-        }
-#pragma unroll
-        for (int t = 0; t < S; ++t) {
-          if (i + t >= n) break;  // uniform
-          if (ed[t].z < 0) {      // uniform: a new vertex starts
-            if (cur_k >= 0) commit();
-            cur_k = ~ed[t].z;
-            cur_v = ed[t].x;
-#pragma unroll
-            for (int j = 0; j < GV::kSlots; ++j) own[j] = best[j] = cur[t][j];
-          } else {
-            relax_min_row<WK>(best, cur[t], static_cast<uint32_t>(ed[t].y));
-          }
-        }
-      }
+      if (bounds || screened) walk(std::true_type{}, n);
+      else walk(std::false_type{}, n);
       __syncwarp();
     }
     if (cur_k >= 0) commit();
@@ -2937,7 +3035,7 @@ __device__ __forceinline__ void sssp_pull_heavy_chunks(const GroupDev& g, const 
 }
 
 template <int W, typename OT, int WK, int kMode>
-__global__ void __launch_bounds__(kBlock) k_sssp_pull_heavy_vec(GroupDev g, DevGraph G) {
+__global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_sssp_pull_heavy_vec(GroupDev g, DevGraph G) {
   __shared__ GatherHeavySmem<W> sm;
   sssp_pull_heavy_chunks<W, OT, WK, kMode>(g, G, blockIdx.x, gridDim.x, sm);
 }
@@ -3310,11 +3408,11 @@ struct GridBarrier {
   }
 };
 
-template <int W, bool kBfs, bool kSssp>
+template <int W, bool kSssp>
 union TraverseSmem {
-  PushSmem<kBfs ? W : 1> push;
+  PushSmem<W> push;
   HeavySlotSmem slot;
-  PullHeavySmem<kBfs ? W : 1> pull_heavy;
+  PullHeavySmem<W> pull_heavy;
   SsspPushSmem<kSssp ? W : 1> sssp_push;
   SsspListSmem<kSssp ? W : 1> sssp_list;
   SsspHeavySmem<kSssp ? W : 1> sssp_heavy;
@@ -3329,23 +3427,24 @@ union TraverseSmem {
 // A launched level is 10 to 16 dependent kernels, most of which find nothing
 // to do; with small graphs and in the first and last levels of deep ones
 // their launches are the level's whole time.
-template <int W, typename OT, int DEPTH, int WK, bool kBfs, bool kSssp>
+template <int W, typename OT, int DEPTH, int WK, bool kSssp>
 __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev g, DevGraph G,
                                                                       int levels, bool heavy) {
-  __shared__ TraverseSmem<W, kBfs, kSssp> sm;
+  __shared__ TraverseSmem<W, kSssp> sm;
   const unsigned bid = blockIdx.x, nblk = gridDim.x;
   LevelCtl* ctl = g.ctl;
   GridBarrier bar(ctl, nblk);
   bool swept = false;  // the previous level zeroed its own frontier's masks
   for (int l = 0; l < levels; ++l) {
     if (ctl->done) return;
-    const bool bfs_pull = kBfs && ctl->dir == kDirPull;
+    const bool bfs = !kSssp || ctl->has_bfs != 0;
+    const bool bfs_pull = bfs && ctl->dir == kDirPull;
     const bool gather = kSssp && ctl->sdir == kDirPull;
     const bool scatter = kSssp && ctl->sscatter != 0;
-    const bool queue = heavy && ((kBfs && !bfs_pull) || scatter);
+    const bool queue = heavy && ((bfs && !bfs_pull) || scatter);
     const bool queued_lists = scatter && ctl->count[ctl->level & 1] > kInlineLists;
     bool summary = gather;
-    if constexpr (kBfs) summary |= bfs_pull_uses_summary(g, ctl, level_view(g), G.V);
+    if (bfs) summary |= bfs_pull_uses_summary(g, ctl, level_view(g), G.V);
     // what the level's phases read or add to; a pull over whole masks alone
     // rewrites every next mask and needs nothing prepared
     const bool clear = ctl->dir == kDirPush && !swept && ctl->prev_count > 0;
@@ -3359,9 +3458,9 @@ __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev 
     // A scattering level whose vertices are all expanded by the tiles reads each
     // mask once and can zero it there: the next level has nothing to clear, and
     // a level of a road-like graph is one phase and one barrier.
-    const bool sweep = kBfs != kSssp && !heavy && !bfs_pull && !gather && !queued_lists;
+    const bool sweep = !(bfs && kSssp) && !heavy && !bfs_pull && !gather && !queued_lists;
     swept = sweep;
-    if constexpr (kBfs) {
+    if (bfs) {
       if (!bfs_pull) {
         bfs_push_tiles<W, OT, DEPTH>(g, G, bid, nblk, sm.push, sweep);
         if (heavy) {

@@ -178,9 +178,9 @@ void seed_t(const GroupDev& g, const DevGraph& G, cudaStream_t s) {
   k_seed<W, OT><<<1, kBlock, 0, s>>>(g, G);
 }
 
-template <int W, typename OT, int DEPTH, int WK, bool kBfs, bool kSssp>
+template <int W, typename OT, int DEPTH, int WK, bool kSssp>
 TraverseKernel traverse_kernel() {
-  auto* fn = k_traverse<W, OT, DEPTH, WK, kBfs, kSssp>;
+  auto* fn = k_traverse<W, OT, DEPTH, WK, kSssp>;
   static const int per_sm = [&] {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kBlock, 0) != cudaSuccess) {
@@ -193,15 +193,14 @@ TraverseKernel traverse_kernel() {
 }
 
 template <int W, typename OT, int DEPTH, int WK>
-TraverseKernel traverse_t(bool has_bfs, bool has_sssp) {
+TraverseKernel traverse_t(bool has_sssp) {
   // wider groups: a level's work outweighs its launches (see fused_loop)
   if constexpr (W > 4) return {nullptr, 0};
-  else if (!has_sssp) return traverse_kernel<W, OT, DEPTH, kWeightNone, true, false>();
+  else if (!has_sssp) return traverse_kernel<W, OT, DEPTH, kWeightNone, false>();
   else if constexpr (DEPTH == kDepthPlanes) {
     return {nullptr, 0};  // planes hold BFS depths only
   } else {
-    return has_bfs ? traverse_kernel<W, OT, DEPTH, WK, true, true>()
-                   : traverse_kernel<W, OT, DEPTH, WK, false, true>();
+    return traverse_kernel<W, OT, DEPTH, WK, true>();
   }
 }
 

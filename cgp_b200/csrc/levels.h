@@ -52,13 +52,13 @@ using GridsFn = Grids (*)(int);
 using SeedFn = void (*)(const GroupDev&, const DevGraph&, cudaStream_t);
 
 
-// The fused level loop for a group's kinds, and how many of its blocks an SM
+// The fused level loop (of BFS groups or of groups with SSSP slots), and how many of its blocks an SM
 // holds (0: not available).
 struct TraverseKernel {
   const void* fn;
   int per_sm;
 };
-using TraverseFn = TraverseKernel (*)(bool has_bfs, bool has_sssp);
+using TraverseFn = TraverseKernel (*)(bool has_sssp);
 
 struct Dispatch {
   EnqueueFn enqueue;

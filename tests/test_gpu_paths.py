@@ -1,0 +1,176 @@
+"""The forms a traversal may take, at the sizes where they change: the fused
+and the launched level loop, row gather items and heavy in-lists, row chunks
+skipped by bounds, slot lists and flattened pairs of a scatter, padded rows,
+depth planes added on the way, union-find sampling, and results copied out
+through pinned slots.  Everything is compared with the CPU oracle for
+equality (distances are the same sums in the same order: exact)."""
+import numpy as np
+import pytest
+
+import cgp_b200 as cgp
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _path(n):
+    v = np.arange(n - 1)
+    return cgp.csr_from_edges(n, v, v + 1)
+
+
+def _stars(degrees, extra=40):
+    """Hubs of exactly the given degrees: shared leaves, and a path through the hubs."""
+    leaves = max(degrees) + extra
+    src, dst = [], []
+    for h, d in enumerate(degrees):
+        n = d - (h > 0) - (h + 1 < len(degrees))
+        src += [h] * n
+        dst += list(range(len(degrees), len(degrees) + n))
+    src += list(range(len(degrees) - 1))
+    dst += list(range(1, len(degrees)))
+    return cgp.csr_from_edges(len(degrees) + leaves, src, dst)
+
+
+def _run(graph, kind, src, loop="auto", **kw):
+    o = cgp.RunOptions(level_loop=loop, **kw)
+    return cgp.run(kind, graph, src, options=o, layout="query").values
+
+
+@pytest.mark.parametrize("loop", ["auto", "chunks"])
+@pytest.mark.parametrize("n,q", [(1, 1), (2, 3), (33, 31), (300, 64), (700, 20)])
+def test_path_graphs_in_both_loops(n, q, loop):
+    """Depths past 15 and 255 add depth planes; 700 vertices take more levels
+    than one launch of the fused loop; two vertices and one take none."""
+    g = _path(n).with_weights("u32", 1, 9, seed=5) if n > 1 else cgp.csr_from_edges(1, [], [])
+    graph = cgp.CsrGraph(g)
+    src = np.arange(q) % n
+    np.testing.assert_array_equal(_run(graph, "bfs", src, loop), oracle.batch("bfs", g, src)[0])
+    if n > 1:
+        np.testing.assert_array_equal(_run(graph, "sssp", src, loop).view(np.uint32),
+                                      oracle.batch("sssp", g, src)[0])
+
+
+@pytest.mark.parametrize("loop", ["auto", "chunks"])
+@pytest.mark.parametrize("kinds", [("bfs",), ("sssp",), ("bfs", "sssp", "khop")])
+def test_grid_levels_swept_or_cleared(kinds, loop):
+    """Road-like graph: the fused loop zeroes masks as it reads them and clears
+    nothing between levels; mixed groups clear as before."""
+    g = cgp.gen_grid(37, 41, 0.1, 0.002, seed=3).with_weights("f32", 1.0, 100.0, seed=4)
+    graph = cgp.CsrGraph(g)
+    src = g.pick_sources(45, seed=6)
+    descs = [cgp.QueryDescriptor(int(s), kinds[i % len(kinds)], 3 + i % 9) for i, s in enumerate(src)]
+    r = cgp.run_batch(graph, descs, cgp.RunOptions(level_loop=loop), layout="query").values
+    for i, d in enumerate(descs):
+        if d.kind == "sssp":
+            np.testing.assert_array_equal(r[i].view(np.float32), oracle.sssp(g, d.source))
+        else:
+            want = oracle.bfs(g, d.source, d.k if d.kind == "khop" else -1)
+            np.testing.assert_array_equal(r[i].view(np.int32), want)
+
+
+@pytest.mark.parametrize("mode", ["pull", "hybrid", "push"])
+@pytest.mark.parametrize("q", [1, 2, 6, 63, 129, 257, 500])
+def test_in_degrees_around_the_gather_and_tile_limits(q, mode):
+    """In-degrees 1, 32, 33, 255 .. 257 and 2047 .. 2049 beside items of one to
+    32 vertices; slot counts that pad to the next multiple of 4."""
+    g = _stars([1, 31, 32, 33, 255, 256, 257, 2047, 2048, 2049]).with_weights("u32", 1, 50, seed=8)
+    graph = cgp.CsrGraph(g)
+    src = g.pick_sources(q, seed=9)
+    got = _run(graph, "sssp", src, traversal_mode=mode, sssp_pull_edge_ratio=0.05,
+               sssp_pull_pair_ratio=0.01)
+    np.testing.assert_array_equal(got.view(np.uint32), oracle.batch("sssp", g, src)[0])
+
+
+@pytest.mark.parametrize("q", [32, 64, 100, 256, 320])
+@pytest.mark.parametrize("weights", ["unit", "small", "zero", "huge", "lognormal", "f32zero"])
+def test_bounds_skip_no_improvement(weights, q):
+    """Every gather level after the first may skip row chunks by bounds.  Two
+    components (the hub is unreachable for some slots), weights whose sums pass
+    2^30 and saturate, zero weights, and float weights over a wide range."""
+    a = cgp.gen_rmat(10, 8, seed=11)
+    s = np.repeat(np.arange(a.num_vertices), a.degrees())
+    off = a.num_vertices
+    g = cgp.csr_from_edges(off + 60, np.r_[s, off + np.arange(59)],
+                           np.r_[a.col_indices, off + 1 + np.arange(59)])
+    if weights == "small":
+        g = g.with_weights("u32", 1, 64, seed=12)
+    elif weights == "zero":
+        g = g.with_weights("u32", 0, 2, seed=12)
+    elif weights == "huge":
+        g = g.with_weights("u32", 1 << 28, 3000000000, seed=12)
+    elif weights == "lognormal":
+        g = g.with_weights("f32", 0.0, 2.0, seed=12, lognormal=True)
+    elif weights == "f32zero":
+        g = g.with_weights("f32", 0.0, 1e-3, seed=12)
+    graph = cgp.CsrGraph(g)
+    src = np.r_[g.pick_sources(q - 3, seed=13), off, off + 30, off + 59]
+    ref = oracle.batch("sssp", g, src)[0] if weights != "unit" else None
+    for mode in ("pull", "hybrid"):
+        for loop in ("auto", "chunks"):
+            got = _run(graph, "sssp", src, loop, traversal_mode=mode)
+            if ref is None:  # unit weights: hop counts
+                hops = oracle.batch("bfs", g, src)[0].view(np.uint32)
+                want = np.where(hops == 0x7fffffff, np.uint32(0xffffffff), hops)
+            else:
+                want = ref
+            np.testing.assert_array_equal(got.view(want.dtype), want)
+
+
+@pytest.mark.parametrize("k", [1, 6, 7, 31, 32, 33, 64, 65, 200, 1024])
+def test_scatter_of_k_slots_at_one_vertex(k):
+    """k queries from one source: every vertex carries k active slots, below
+    and above the list limit, in whole and partial runs of 32; lists of 40, 257
+    and 2100 edges go to tiles and to the heavy queue."""
+    g = _stars([3, 40, 257, 2100]).with_weights("u32", 1, 30, seed=15)
+    graph = cgp.CsrGraph(g)
+    src = np.full(k, g.num_vertices - 45)
+    got = _run(graph, "sssp", src, traversal_mode="push", mask_words=16 if k > 512 else 0)
+    want = oracle.sssp(g, int(src[0]))
+    np.testing.assert_array_equal(got.view(np.uint32), np.tile(want, (k, 1)))
+
+
+@pytest.mark.parametrize("frontier", [3000, 40000])
+def test_scatter_lists_queued_and_in_place(frontier):
+    """The second level holds `frontier` vertices of 70 active slots each: small
+    frontiers scatter their lists in the tile, larger ones queue them."""
+    n = frontier
+    src = np.zeros(n, np.int64)
+    ring = np.arange(n)
+    g = cgp.csr_from_edges(n + 1, np.r_[src, 1 + ring], np.r_[1 + ring, 1 + (ring + 1) % n])
+    g = g.with_weights("u32", 1, 40, seed=17)
+    graph = cgp.CsrGraph(g)
+    want = oracle.sssp(g, 0)
+    got = _run(graph, "sssp", np.zeros(70, np.int64), traversal_mode="push")
+    np.testing.assert_array_equal(got.view(np.uint32), np.tile(want, (70, 1)))
+
+
+@pytest.mark.parametrize("make", [
+    lambda: cgp.csr_from_edges(1, [], []),
+    lambda: _path(1000),
+    lambda: cgp.gen_grid(150, 130, 0.45, 0.0, seed=21),     # many components
+    lambda: cgp.gen_rmat(12, 8, seed=22),
+    lambda: cgp.csr_from_edges(4000, np.arange(0, 4000, 2), np.arange(1, 4000, 2)),  # pairs
+    lambda: cgp.csr_from_edges(3000, np.arange(2999), np.arange(1, 3000)[::-1], symmetrize=False),
+    lambda: cgp.csr_from_edges(5000, np.arange(1, 5000), np.zeros(4999), symmetrize=False),
+])
+def test_wcc_sampling(make):
+    g = make()
+    got = cgp.run("wcc", cgp.CsrGraph(g), [0]).values[:, 0].view(np.uint32)
+    np.testing.assert_array_equal(got, oracle.wcc_components(g))
+
+
+@pytest.mark.parametrize("n,q", [(100, 1), (131072, 1), (131073, 4), (65536, 37)])
+@pytest.mark.parametrize("layout", ["vertex", "query"])
+def test_results_into_pageable_and_pinned_memory(n, q, layout):
+    """Result sizes below, at and beyond the copy slots and their count."""
+    import torch
+    g = _path(n) if n < 1000 else cgp.csr_from_edges(n, np.zeros(n - 1), np.arange(1, n))
+    graph = cgp.CsrGraph(g, symmetric=True)
+    src = (np.arange(q) * 7) % n
+    descs = [cgp.QueryDescriptor(int(s), "bfs") for s in src]
+    want = oracle.batch("bfs", g, src)[0]
+    want = want if layout == "query" else want.T
+    np.testing.assert_array_equal(cgp.run_batch(graph, descs, layout=layout).values, want)
+    pinned = torch.empty(want.shape, dtype=torch.int32, pin_memory=True)
+    cgp.run_batch(graph, descs, layout=layout, out=pinned)
+    np.testing.assert_array_equal(pinned.numpy(), want)
