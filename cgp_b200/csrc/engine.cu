@@ -726,7 +726,12 @@ int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelL
       1, std::min<int64_t>(most, (g->E + g->V) / 256)));
   bool heavy = L.heavy_push;
   void* args[] = {&L.g, &L.G, &levels, &heavy};
-  ck(cudaLaunchCooperativeKernel(k.fn, dim3(blocks), dim3(kBlock), args, 0, s), "fused level loop");
+  const cudaError_t e = cudaLaunchCooperativeKernel(k.fn, dim3(blocks), dim3(kBlock), args, 0, s);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the GPU is reserved: launch the levels
+    cudaGetLastError();
+    return 0;
+  }
+  ck(e, "fused level loop");
   return 1;
 }
 
@@ -738,8 +743,11 @@ int enqueue_levels(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp
                    cudaStream_t s, int levels, KernelTimer* kt) {
   Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
   LevelLaunch L = level_launch(g, ws, spec, o, d);
-  if (kt == nullptr && levels > 0 && fused_loop(spec, o, d, L))
-    return enqueue_fused(g, spec, d, L, s, levels);
+  if (kt == nullptr && levels > 0 && fused_loop(spec, o, d, L)) {
+    const int n = enqueue_fused(g, spec, d, L, s, levels);
+    if (n > 0) return n;
+    levels = std::min(levels, 8);
+  }
   L.kt = kt;
   if (!o.use_cuda_graph || kt != nullptr) {
     int n = 0;
