@@ -17,7 +17,8 @@ constexpr int kMaxW = 16;
 constexpr int kMaxPlanes = 24;
 constexpr int kLightChunkVerts = 32;    // light vertices per chunked-gather CTA item
 constexpr int kLightChunkEdges = 2048;  // and their in-edges
-constexpr int kGatherHeavy = 256;       // in-edges one warp of the row gather takes at most
+constexpr int kGatherHeavy = 256;       // in-edges one warp of the row gather takes at most: 8 steps
+                                        // of 32; the 8 warps of a CTA share longer lists
 
 enum : int32_t { kDirPush = 0, kDirPull = 1 };
 enum : int32_t { kDepthNone = 0, kDepthDirect = 1, kDepthPlanes = 2 };

@@ -695,7 +695,11 @@ LevelLaunch level_launch(GraphImpl* g, Workspace* ws, const GroupSpec& spec, con
   return L;
 }
 
-// Edges x mask words up to which SSSP levels run fused.
+// Edges x mask words up to which SSSP levels run fused: below the line the
+// launches weigh more (mixed R-MAT 17, 48 slots, 3.7M: 1.33 ms fused against
+// 1.72 launched; directed 200K, 100 slots, 4.8M: 3.4 against 3.6), above it the
+// launched kernels' own register budgets do (R-MAT 20, 256 slots, 126M: 12.7
+// against 12.3; a 1024-slot grid, 36M: 253 against 209).
 constexpr int64_t kFusedWork = 1 << 24;
 
 // Whether the group's levels run as the fused loop: the automatic loop form,
@@ -1258,9 +1262,9 @@ cgp_status cgp_batch_run(cgp_graph* graph, const cgp_query* queries, int32_t nq,
     if (!wcc_idx.empty()) {
       if (kt) kt->mark(kClassWcc, s);
       ws->wcc.ensure(static_cast<size_t>(V + 1) * 4);
-      wcc_labels(g, ws->wcc.as<uint32_t>(), s);
+      launches += wcc_labels(g, ws->wcc.as<uint32_t>(), s);
       for (int i : wcc_idx) broadcast_labels(ws->wcc.as<uint32_t>(), V, om, i, s);
-      launches += 9 + (g->symmetric ? 0 : 1) + wcc_idx.size();
+      launches += wcc_idx.size();
       if (kt) kt->mark(-1, s);
     }
     // Traversal groups of up to 64*W queries, in submission order.  A batch

@@ -105,7 +105,7 @@ enum KernelClass {
   kClassInit,
   kClassOutput,
   kClassWcc,
-  kClassSsspDense,  // SSSP dense kernel (many active queries per vertex)
+  kClassSsspDense,  // SSSP list kernel (vertices with several active queries)
   kClassSsspHeavy,  // SSSP heavy-vertex chunks
   kClassSsspPull,   // SSSP gather levels (light and heavy vertices)
   kNumClasses
@@ -246,8 +246,8 @@ void group_write_output(GraphImpl* g, Workspace* ws, GroupSpec& spec,
 int choose_words(int n, int requested);
 int64_t group_state_bytes(const GraphImpl* g, int W, int Qg, int depth_mode);
 // WCC: minimum vertex id of each weak component into labels[0 .. V) (device,
-// V + 1 entries).
-void wcc_labels(GraphImpl* g, uint32_t* labels, cudaStream_t s);
+// V + 1 entries); returns the kernels launched.
+int wcc_labels(GraphImpl* g, uint32_t* labels, cudaStream_t s);
 // Writes labels[v] into global column `col` of the output mapping.
 void broadcast_labels(const uint32_t* labels, int64_t V, dev::OutMap om, int col,
                       cudaStream_t s);

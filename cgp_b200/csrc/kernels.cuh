@@ -1506,7 +1506,9 @@ struct SsspPushSmem {
 
 // Frontiers of at most this many vertices have their listed vertices scattered
 // by the tile's own warp; larger ones queue them for sssp_list_vertices, which
-// spreads them over all warps.
+// spreads them over all warps.  16,384 is what fills every warp's tile a few
+// vertices wide (tile_width): up to there a queue would only add a barrier or a
+// launch, beyond it one tile's lists are the level's tail.
 constexpr unsigned long long kInlineLists = 16384;
 
 // SSSP push over the frontier list, a warp per tile of 32 vertices.  Vertices

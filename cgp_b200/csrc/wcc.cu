@@ -14,6 +14,12 @@ namespace {
 
 using namespace dev;
 
+__global__ void k_uf_self(int32_t* parent, int64_t V) {
+  for (int64_t v = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < V;
+       v += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    parent[v] = static_cast<int32_t>(v);
+}
+
 // Every vertex starts below its first neighbour if that has the smaller id (a
 // forest: parents are smaller), else as its own root: the first link of each
 // vertex costs no atomic.
@@ -77,6 +83,43 @@ __device__ __forceinline__ void uf_union(int32_t* parent, int32_t a, int32_t b) 
     if (old == ra) return;
     ra = uf_find(parent, old);
     rb = uf_find(parent, rb);
+  }
+}
+
+// Every CSR entry u->v joins u and v.  On a symmetric CSR each undirected
+// edge is visited once (v < u).  Warp per tile of 32 vertices; vertices with
+// more than 32 entries are walked by the whole warp.
+template <typename OT>
+__global__ void __launch_bounds__(kBlock) k_uf_hook(const void* row, const int32_t* col,
+                                                    int32_t* parent, int64_t V, int symmetric) {
+  const int lane = threadIdx.x & 31;
+  const int64_t gw = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t tile = gw; tile * 32 < V; tile += nw) {
+    const int64_t u = tile * 32 + lane;
+    int64_t beg = 0, end = 0;
+    if (u < V) {
+      beg = row_at<OT>(row, u);
+      end = row_at<OT>(row, u + 1);
+    }
+    if (end - beg <= 32) {
+      for (int64_t e = beg; e < end; ++e) {
+        const int32_t v = col[e];
+        if (!symmetric || v < u) uf_union(parent, static_cast<int32_t>(u), v);
+      }
+    }
+    unsigned big = __ballot_sync(kFull, end - beg > 32);
+    while (big) {
+      const int src = __ffs(big) - 1;
+      big &= big - 1;
+      const int64_t bu = __shfl_sync(kFull, u, src);
+      const int64_t bb = __shfl_sync(kFull, beg, src);
+      const int64_t be = __shfl_sync(kFull, end, src);
+      for (int64_t e = bb + lane; e < be; e += 32) {
+        const int32_t v = col[e];
+        if (!symmetric || v < bu) uf_union(parent, static_cast<int32_t>(bu), v);
+      }
+    }
   }
 }
 
@@ -186,10 +229,22 @@ __global__ void k_broadcast(const uint32_t* labels, int64_t V, OutMap om, int co
 
 namespace {
 
+// Entries per vertex from which neighbours are sampled.  Below, two links per
+// vertex are a good part of all entries and the passes between them cost more
+// than they save: on 1100 x 1300 grids (3.6 entries) sampling took 264 to 304 us
+// for most and 536 and 1040 us for two of ten, all entries at once 356 to 424;
+// on R-MAT 18 (29 entries) 130 to 240 us against 890 to 2700.
+constexpr int64_t kSampleDegree = 8;
+
 template <typename OT>
-void link_all(GraphImpl* g, int32_t* parent, int32_t* most, int blocks, cudaStream_t s) {
+int link_all(GraphImpl* g, int32_t* parent, int32_t* most, int blocks, cudaStream_t s) {
   const int64_t V = g->V;
   const int32_t* col = g->col.as<int32_t>();
+  if (g->E < kSampleDegree * V) {
+    k_uf_self<<<blocks, kBlock, 0, s>>>(parent, V);
+    k_uf_hook<OT><<<blocks, kBlock, 0, s>>>(g->row.p, col, parent, V, g->symmetric ? 1 : 0);
+    return 2;
+  }
   k_uf_init<OT><<<blocks, kBlock, 0, s>>>(g->row.p, col, parent, V);
   k_uf_compress<<<blocks, kBlock, 0, s>>>(parent, V);
   k_uf_second<OT><<<blocks, kBlock, 0, s>>>(g->row.p, col, parent, V, 61);
@@ -198,8 +253,9 @@ void link_all(GraphImpl* g, int32_t* parent, int32_t* most, int blocks, cudaStre
   k_uf_compress<<<blocks, kBlock, 0, s>>>(parent, V);
   k_uf_sample<<<1, kSamples, 0, s>>>(parent, V, most);
   k_uf_rest<OT><<<blocks, kBlock, 0, s>>>(g->row.p, col, parent, V, most);
-  if (!g->symmetric)
-    k_uf_rest<OT><<<blocks, kBlock, 0, s>>>(g->trow.p, g->tcol.as<int32_t>(), parent, V, most);
+  if (g->symmetric) return 8;
+  k_uf_rest<OT><<<blocks, kBlock, 0, s>>>(g->trow.p, g->tcol.as<int32_t>(), parent, V, most);
+  return 9;
 }
 
 }  // namespace
@@ -207,17 +263,19 @@ void link_all(GraphImpl* g, int32_t* parent, int32_t* most, int blocks, cudaStre
 // Union-find with neighbour sampling (Sutton, Ben-Nun, Barak: Optimizing
 // parallel graph connectivity computation via subgraph sampling, 2018): two
 // links per vertex, then only the vertices outside the component most of them
-// have ended up in visit their lists.  Visiting every entry took 0.86 ms on
-// R-MAT 17, where the finds and links of 1.9M edges meet at a few roots.
-void wcc_labels(GraphImpl* g, uint32_t* labels, cudaStream_t s) {
+// have ended up in visit their lists; graphs of low degree link every entry.
+// Visiting every entry took 0.86 ms on R-MAT 17, where the finds and links of
+// 1.9M edges meet at a few roots; sampling takes 0.1.
+int wcc_labels(GraphImpl* g, uint32_t* labels, cudaStream_t s) {
   // parent array lives in `labels` itself (int32 view), the sampled root
   // behind it; the final pass rewrites every entry with its root.
   int32_t* parent = reinterpret_cast<int32_t*>(labels);
   const int blocks = g->num_sms * 8;
-  if (g->offset_bytes == 8) link_all<int64_t>(g, parent, parent + g->V, blocks, s);
-  else link_all<int32_t>(g, parent, parent + g->V, blocks, s);
+  const int n = g->offset_bytes == 8 ? link_all<int64_t>(g, parent, parent + g->V, blocks, s)
+                                     : link_all<int32_t>(g, parent, parent + g->V, blocks, s);
   k_uf_labels<<<blocks, kBlock, 0, s>>>(parent, g->V);
   ck(cudaGetLastError(), "wcc");
+  return n + 1;
 }
 
 void broadcast_labels(const uint32_t* labels, int64_t V, OutMap om, int col, cudaStream_t s) {

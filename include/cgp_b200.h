@@ -108,8 +108,9 @@ typedef struct {
   int32_t dense_unroll;       /* edges per step of the SSSP list kernel: 1: 4, 2: 8; 0 = 1 */
   double sssp_pull_edge_ratio; /* SSSP levels gather (pull) when frontier edges >= ratio * E;
                                   <= 0: always scatter (push)                              */
-  int32_t light_chunks;       /* SSSP gathers take light vertices in CTA chunks (wider groups
-                                 in 256-slot slices): 0 = on, -1 = one warp per vertex     */
+  int32_t light_chunks;       /* SSSP gathers take light vertices by items of up to 32 per warp
+                                 (wider groups in 256-slot slices): 0 = on, -1 = one warp
+                                 per vertex                                              */
   int32_t level_loop;         /* CGP_LOOP_*: how a traversal to convergence is driven     */
   int32_t sssp_chunk_direction; /* SSSP gather/scatter decided per 32-slot chunk from the
                                    chunk's own frontier (1), or for the whole group (-1);
@@ -131,18 +132,20 @@ typedef struct {
                                   the next frontier's mean out-degree) to reach ratio x E x
                                   the group's SSSP 32-slot chunks to gather: a scatter costs
                                   per pair, a gather per (in-edge, chunk); default 0.5;
-                                  <= 0: edges alone decide                               */
+                                  <= 0: edges alone decide.  Ratio x E once bounds let
+                                  a gather skip most row chunks                          */
   void* stream;               /* cudaStream_t; NULL = the library's own stream   */
 } cgp_options;
 
-/* level_loop values.  CHUNKS: CUDA graphs of levels_per_sync levels, the host
+/* level_loop values.  AUTO: BFS groups of up to 256 slots, and groups with SSSP
+ * slots up to 2^24 (edge, mask word) pairs, run up to 256 levels per cooperative
+ * launch (levels_per_sync, when given, instead of 256); others as CHUNKS.  CHUNKS: CUDA graphs of levels_per_sync levels, the host
  * reads the control block once per chunk (one chunk in flight).  DEVICE: one
  * CUDA graph whose WHILE conditional node runs a level per iteration until
  * the device-side done flag is set: the host waits once per traversal (it
  * replaces the reference's per-level host synchronisation,
- * frontier_engine.hxx:3044-3071).  AUTO is CHUNKS: kernels inside a graph
- * with conditional nodes are invisible to kernel profilers, so the device
- * loop is asked for explicitly. */
+ * frontier_engine.hxx:3044-3071); kernels inside a graph with conditional nodes
+ * are invisible to kernel profilers, so it is asked for explicitly. */
 #define CGP_LOOP_AUTO 0
 #define CGP_LOOP_CHUNKS 1
 #define CGP_LOOP_DEVICE 2

@@ -174,3 +174,55 @@ def test_results_into_pageable_and_pinned_memory(n, q, layout):
     pinned = torch.empty(want.shape, dtype=torch.int32, pin_memory=True)
     cgp.run_batch(graph, descs, layout=layout, out=pinned)
     np.testing.assert_array_equal(pinned.numpy(), want)
+
+
+@pytest.mark.parametrize("q", [1, 65, 129, 257, 513, 1024])
+@pytest.mark.parametrize("depth", ["planes", "direct"])
+def test_pull_masks_shared_by_lanes(q, depth):
+    """Masks of 1 to 16 words: one lane each, or 16 bytes per lane; light, mid
+    and heavy in-lists; queries of two components, k-hop bounds among them."""
+    a = cgp.gen_rmat(11, 12, seed=31)
+    s = np.repeat(np.arange(a.num_vertices), a.degrees())
+    off = a.num_vertices
+    g = cgp.csr_from_edges(off + 50, np.r_[s, off + np.arange(49)],
+                           np.r_[a.col_indices, off + 1 + np.arange(49)])
+    graph = cgp.CsrGraph(g)
+    src = np.r_[g.pick_sources(q, seed=32), off][1:]
+    descs = [cgp.QueryDescriptor(int(v), "khop" if i % 5 == 4 else "bfs", 1 + i % 4)
+             for i, v in enumerate(src)]
+    for mode in ("pull", "hybrid"):
+        for loop in ("auto", "chunks"):
+            o = cgp.RunOptions(traversal_mode=mode, level_loop=loop, depth_mode=depth,
+                               heavy_degree=200)
+            r = cgp.run_batch(graph, descs, o, layout="query").values.view(np.int32)
+            for i in {0, q // 2, q - 1, 4 % q, min(q - 1, 64)}:
+                d = descs[i]
+                np.testing.assert_array_equal(
+                    r[i], oracle.bfs(g, d.source, d.k if d.kind == "khop" else -1))
+
+
+@pytest.mark.parametrize("offsets64", [False, True])
+@pytest.mark.parametrize("weights", ["none", "u32", "f32"])
+@pytest.mark.parametrize("q", [5, 70, 200])
+def test_directed_gathers_over_the_transpose(q, weights, offsets64):
+    """Vertices without in-edges, in-lists from 1 to 700, asymmetric weights."""
+    r = np.random.default_rng(41)
+    n, m = 900, 14000
+    dst = (n * r.random(m) ** 3).astype(np.int64) + 20
+    g = cgp.csr_from_edges(n + 20, r.integers(0, n + 20, m), np.minimum(dst, n + 19),
+                           symmetrize=False)
+    if weights == "u32":
+        g.weights = r.integers(0, 40, g.num_edges).astype(np.uint32)
+    elif weights == "f32":
+        g.weights = r.random(g.num_edges).astype(np.float32) * 10
+    graph = cgp.CsrGraph(g, offsets64=offsets64)
+    src = r.integers(0, n + 20, q)
+    if weights == "none":
+        hops = oracle.batch("bfs", g, src)[0].view(np.uint32)
+        want = np.where(hops == 0x7fffffff, np.uint32(0xffffffff), hops)
+    else:
+        want = oracle.batch("sssp", g, src)[0]
+    for mode in ("pull", "hybrid"):
+        for loop in ("auto", "chunks"):
+            got = _run(graph, "sssp", src, loop, traversal_mode=mode)
+            np.testing.assert_array_equal(got.view(want.dtype), want)
