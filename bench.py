@@ -59,13 +59,7 @@ BFS_INF = 2**31 - 1
 # + dram__bytes_write.sum summed over the level's kernels), with where and when
 # they were measured.  Reported beside the run's own numbers; never computed
 # from files at run time.
-NCU_TRAFFIC = {
-    ("c2", "sssp_gather"): {
-        "bytes_per_level": 5.812e10,
-        "source": "profiles/dram_traffic_sssp_gather_rmat22.md (one-pass ncu metrics, full size)",
-        "captured": "2026-12-03",
-    },
-}
+NCU_TRAFFIC = {}  # none for the present gather kernels
 
 
 WORKLOADS = {
@@ -355,8 +349,8 @@ def level_bytes(p, kind, V, W, ob=4, qs=0):
 CLASS_KERNELS = {
     "bfs_push": "k_bfs_push, k_bfs_push_heavy",
     "bfs_pull": "k_bfs_pull, k_bfs_pull_heavy(_commit)",
-    "sssp_scatter": "k_sssp_push, k_sssp_dense, k_sssp_push_heavy",
-    "sssp_gather": "k_sssp_pull_chunked, k_sssp_pull_heavy_vec",
+    "sssp_scatter": "k_sssp_push, k_sssp_list, k_sssp_push_heavy",
+    "sssp_gather": "k_sssp_pull_rows, k_sssp_pull_heavy_vec",
 }
 
 
