@@ -59,7 +59,13 @@ BFS_INF = 2**31 - 1
 # + dram__bytes_write.sum summed over the level's kernels), with where and when
 # they were measured.  Reported beside the run's own numbers; never computed
 # from files at run time.
-NCU_TRAFFIC = {}  # none for the present gather kernels
+NCU_TRAFFIC = {
+    ("c2", "sssp_gather"): {
+        "bytes_per_level": 2.93e10,
+        "source": "profiles/dram_traffic_sssp_gather_rmat22.md (ncu, full size, mean of 4 levels)",
+        "captured": "2026-12-05",
+    },
+}
 
 
 WORKLOADS = {
