@@ -3632,6 +3632,12 @@ __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev 
         if (G.n_sheavy > 0) {
           sssp_pull_heavy_chunks<W, OT, WK, (W <= 4 ? 3 : 0)>(g, G, bid, nblk, sm.gather_heavy);
           if (!bar.wait()) return;
+        } else if (bfs && !bfs_pull && !scatter) {
+          // the light gather stores whole vectors of a row: depths a push of this
+          // level writes into the same vectors must be in place before their row
+          // is read (after a scatter, a pull or a heavy gather they are; the heavy
+          // gather itself only lowers its own words)
+          if (!bar.wait()) return;
         }
         sssp_pull_light_rows<(W < 4 ? W : 4), OT, WK, W>(g, G, bid, nblk, sm.gather_light);
       }

@@ -68,6 +68,26 @@ def test_grid_levels_swept_or_cleared(kinds, loop):
             np.testing.assert_array_equal(r[i].view(np.int32), want)
 
 
+@pytest.mark.parametrize("loop", ["auto", "chunks"])
+@pytest.mark.parametrize("q,words", [(45, 0), (90, 0), (126, 4)])
+def test_bfs_push_beside_an_sssp_gather(q, words, loop):
+    """BFS pushes while SSSP gathers, in one group whose kinds alternate by slot
+    (so they share the row vectors the gather writes back), on a grid: no
+    in-list is long enough for the heavy gather to come between the two."""
+    for seed in range(4):
+        g = cgp.gen_grid(61 + seed, 67, 0.1, 0.002, seed=seed).with_weights("f32", 1.0, 100.0, seed=4)
+        graph = cgp.CsrGraph(g)
+        src = g.pick_sources(q, seed=60 + seed)
+        descs = [cgp.QueryDescriptor(int(s), "sssp" if i % 2 else "bfs") for i, s in enumerate(src)]
+        o = cgp.RunOptions(level_loop=loop, mask_words=words, sssp_pull_edge_ratio=0.01,
+                           sssp_pull_pair_ratio=0.0, pull_edge_ratio=2.0, pull_frontier_ratio=2.0)
+        r = cgp.run_batch(graph, descs, o, layout="query")
+        assert r.pull_levels == 0 and r.counters["sssp_pull_edges"] > 0
+        np.testing.assert_array_equal(r.values[::2].view(np.int32), oracle.batch("bfs", g, src[::2])[0])
+        np.testing.assert_array_equal(r.values[1::2].view(np.uint32),
+                                      oracle.batch("sssp", g, src[1::2])[0].view(np.uint32))
+
+
 @pytest.mark.parametrize("mode", ["pull", "hybrid", "push"])
 @pytest.mark.parametrize("q", [1, 2, 6, 63, 129, 257, 500])
 def test_in_degrees_around_the_gather_and_tile_limits(q, mode):
