@@ -54,7 +54,7 @@ cgp_status cgp_enactor_create(cgp_graph* graph, const cgp_query* queries, int32_
     e->ws = std::make_unique<Workspace>(g->device);
     e->stream = e->opts.stream ? static_cast<cudaStream_t>(e->opts.stream) : e->ws->stream;
     e->spec = make_group(queries, nq, choose_words(nq, e->opts.mask_words), e->opts.depth_mode);
-    if (e->spec.has_sssp) pad_rows(e->spec);
+    pad_rows(g, e->ws.get(), e->spec, e->opts, false);
     for (int i = 0; i < nq; ++i)
       if (queries[i].kind == CGP_KIND_WCC) e->wcc_slots.push_back(i);
     *out = e;

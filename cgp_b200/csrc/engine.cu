@@ -451,11 +451,6 @@ GroupSpec make_group(const cgp_query* q, int n, int W, int depth_mode) {
   return g;
 }
 
-void pad_rows(GroupSpec& g) {
-  g.Qg = (g.n + 3) & ~3;
-  g.slots.resize(g.Qg, dev::SlotDev{-1, -1, 0, 0});
-}
-
 static constexpr int kInitialPlanes = 8;  // depth planes allocated at first
 static constexpr int kStartPlanes = 4;    // ... and zeroed: depths up to 15
 
@@ -529,14 +524,37 @@ bool sssp_chunk_dir(const GroupSpec& spec, const cgp_options& o) {
   return o.sssp_chunk_direction > 0 || (o.sssp_chunk_direction == 0 && spec.serving);
 }
 
-// Rows the vectorised gather can read: whole kElem-slot vectors, aligned.
+// Slots per vector load of the gather kernels (GatherVec::kElem).
+int row_vector(int W) { return W == 1 ? 2 : 4; }
+
+// Rows the vectorised gather can read: whole vectors, aligned.
 bool vector_rows(const GroupSpec& spec, const uint32_t* values) {
-  const int elem = spec.W == 1 ? 2 : 4;
+  const int elem = row_vector(spec.W);
   return values != nullptr && spec.Qg % elem == 0 &&
          reinterpret_cast<uintptr_t>(values) % (4 * elem) == 0;
 }
 
 }  // namespace
+
+bool pad_rows(const GraphImpl* g, const Workspace* ws, GroupSpec& spec, const cgp_options& o,
+              bool external) {
+  const int elem = row_vector(spec.W);
+  if (!spec.has_sssp || spec.n % elem == 0 || !sssp_gather_on(g, o)) return false;
+  const int padded = (spec.n + elem - 1) / elem * elem;
+  const size_t need = static_cast<size_t>(g->V) * padded * 4;
+  if (ws->values.bytes < need) {
+    size_t free_b = 0, total_b = 0;
+    ck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+    // all that group_prepare may still allocate: the group's state, and up to 32
+    // bytes per vertex of lists and summaries
+    const size_t state = static_cast<size_t>(group_state_bytes(g, spec.W, padded, spec.depth_mode)) +
+                         static_cast<size_t>(g->V) * 32;
+    if (external ? need > free_b / 4 : state > free_b) return false;
+  }
+  spec.Qg = padded;
+  spec.slots.resize(padded, dev::SlotDev{-1, -1, 0, 0});
+  return true;
+}
 
 void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options& o,
                    cudaStream_t s) {
@@ -1315,22 +1333,7 @@ cgp_status cgp_batch_run(cgp_graph* graph, const cgp_query* queries, int32_t nq,
       // used directly as the working value matrix (no copy at the end).
       bool in_place = out_on_device && !qmajor && single && wcc_idx.empty() &&
                       spec.depth_mode != kDepthPlanes;
-      // SSSP rows of a slot count that is no multiple of 4 are padded to one in
-      // a matrix of the engine's own: the gather then reads 16-byte vectors
-      // (499 slots on Chung-Lu, 300K vertices: see GroupSpec::Qg).  An output
-      // that could be used in place is left for that only where the matrix is
-      // small beside the free memory.
-      if (spec.has_sssp && n % 4 != 0 && sssp_gather_on(g, o)) {
-        const size_t need = static_cast<size_t>(V) * ((n + 3) & ~3) * 4;
-        if (in_place && ws->values.bytes < need) {
-          size_t free_b = 0, total_b = 0;
-          ck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-          if (need <= free_b / 4) in_place = false;
-        } else {
-          in_place = false;
-        }
-        if (!in_place) pad_rows(spec);
-      }
+      if (pad_rows(g, ws.get(), spec, o, in_place)) in_place = false;
       if (in_place) spec.external_values = dout;
       if (kt) kt->mark(kClassInit, s);
       group_prepare(g, ws.get(), spec, o, s);

@@ -200,7 +200,7 @@ struct GraphImpl {
 struct GroupSpec {
   int W = 1;
   int n = 0;   // queries (slots 0 .. n-1)
-  int Qg = 0;  // slots per value row: n, or n rounded up to 4 (pad_rows)
+  int Qg = 0;  // slots per value row: n, or n rounded up to whole vectors (pad_rows)
   std::vector<dev::SlotDev> slots;
   int depth_mode = dev::kDepthDirect;
   bool has_bfs = false;
@@ -228,9 +228,17 @@ struct GroupRun {
 
 // Engine entry points (engine.cu).
 GroupSpec make_group(const cgp_query* q, int n, int W, int depth_mode);
-// Rounds the value rows up to a multiple of 4 slots; the added slots belong to
-// no query (kind and source -1: never seeded, never written out).
-void pad_rows(GroupSpec& g);
+// Rounds an SSSP group's value rows up to whole vectors of the gather kernels, so
+// that its gathers read 8 (one mask word) or 16 bytes per load instead of 4 (499
+// slots on Chung-Lu, 300K vertices: the batch 34.7 -> 11.7 ms with the rest of the
+// vector path).  The added slots belong to no query (kind and source -1: never
+// seeded, never written out).  False, and rows as they are, where nothing is to be
+// added, where the group never gathers, or where the padded matrix has no room:
+// it must leave the memory that the unpadded group needs as well, and, where the
+// values could live in the caller's buffer (`external`), take at most a quarter
+// of the free memory.
+bool pad_rows(const GraphImpl* g, const Workspace* ws, GroupSpec& spec, const cgp_options& o,
+              bool external);
 void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options& o,
                    cudaStream_t s);
 // Runs levels until convergence (done != 0) or, with max_levels > 0, that

@@ -246,3 +246,27 @@ def test_directed_gathers_over_the_transpose(q, weights, offsets64):
         for loop in ("auto", "chunks"):
             got = _run(graph, "sssp", src, loop, traversal_mode=mode)
             np.testing.assert_array_equal(got.view(want.dtype), want)
+
+
+def test_rows_stay_unpadded_without_room():
+    """9 SSSP slots over 16M vertices in memory that holds their 576 MB value
+    matrix but not one of 10 or 12 slots per row beside the rest of the group."""
+    import torch
+    n = 1 << 24
+    g = cgp.csr_from_edges(n, np.zeros(n - 1), np.arange(1, n))
+    graph = cgp.CsrGraph(g, symmetric=True)
+    src = [0, 1, 5, n - 1, 77, 4096, n // 2, 3, 2]
+    descs = [cgp.QueryDescriptor(s, "sssp") for s in src]
+    out = torch.empty((len(src), n), dtype=torch.int32, device="cuda")
+    cgp.run_batch(graph, descs[:4], layout="query", out=out)  # the 4-slot group's memory stays
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (416 << 20), dtype=torch.uint8, device="cuda")
+    cgp.run_batch(graph, descs, layout="query", out=out)
+    del fill
+    torch.cuda.empty_cache()
+    want = torch.full((n,), 2, dtype=torch.int32, device="cuda")
+    want[0] = 1
+    for i, s in enumerate(src):
+        w = want.clone() if s else torch.ones_like(want)
+        w[s] = 0
+        assert torch.equal(out[i], w)
