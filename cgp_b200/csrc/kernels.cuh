@@ -810,6 +810,7 @@ __device__ __forceinline__ void bfs_pull_tiles(const GroupDev& g, const DevGraph
     const bool open = (want_lanes & group) != 0;  // some lane of the vertex
     const bool work = valid && !heavy && deg > 0 && open;
     pverts += work && sub == 0 ? 1 : 0;
+    int walked = 0;  // in-edges this lane's words needed
     if (work && wants && deg <= 32) {
       const uint32_t nch = chunk_bits<WL>(need) << (2 * w0);
       // four in-edges per step: their column and mask loads are independent
@@ -830,7 +831,7 @@ __device__ __forceinline__ void bfs_pull_tiles(const GroupDev& g, const DevGraph
           for (int j = 0; j < 4; ++j)
             if (us[j] >= 0 && !(summary_chunks(g.fsum, lv.level, us[j]) & nch)) us[j] = -1;
         }
-        if (sub == 0) pedges += static_cast<unsigned long long>(end - e < 4 ? end - e : 4);
+        walked += end - e < 4 ? static_cast<int>(end - e) : 4;
         bool full = true;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -845,6 +846,10 @@ __device__ __forceinline__ void bfs_pull_tiles(const GroupDev& g, const DevGraph
         if (full) break;
       }
     }
+    // a vertex's in-edges count once: as far as the lane that needed most went
+#pragma unroll
+    for (int o = LP / 2; o > 0; o >>= 1) walked = max(walked, __shfl_xor_sync(kFull, walked, o));
+    if (sub == 0) pedges += static_cast<unsigned long long>(walked);
     // longer lists, where no kernel of their own takes them: the warp per
     // vertex, kGroups in-edges per step
     unsigned big = __ballot_sync(kFull, work && deg > 32 && sub == 0);

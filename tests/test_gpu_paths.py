@@ -270,3 +270,22 @@ def test_rows_stay_unpadded_without_room():
         w = want.clone() if s else torch.ones_like(want)
         w[s] = 0
         assert torch.equal(out[i], w)
+
+
+@pytest.mark.parametrize("loop", ["auto", "chunks"])
+@pytest.mark.parametrize("words", [2, 4, 8, 16])
+def test_pull_edges_counted_for_any_words(words, loop):
+    """One BFS in the last slot of a wide group whose other slots have stopped
+    (0-hop): the pull reads, and counts, the in-edges the query alone would."""
+    for g in (cgp.gen_grid(40, 50, 0.1, 0.01, seed=5), cgp.gen_rmat(11, 8, seed=6)):
+        graph = cgp.CsrGraph(g)
+        s = int(g.pick_sources(1, seed=7)[0])
+        o = dict(traversal_mode="pull", level_loop=loop, depth_mode="direct")
+        alone = cgp.run_batch(graph, [cgp.QueryDescriptor(s, "bfs")], cgp.RunOptions(**o))
+        descs = [cgp.QueryDescriptor(i % g.num_vertices, "khop", 0) for i in range(64 * words - 1)]
+        r = cgp.run_batch(graph, descs + [cgp.QueryDescriptor(s, "bfs")],
+                          cgp.RunOptions(mask_words=words, **o))
+        np.testing.assert_array_equal(r.values[:, -1].view(np.int32), oracle.bfs(g, s, -1))
+        assert r.mask_words == words
+        for k in ("pull_vertices", "pull_edges", "new_pairs"):
+            assert r.counters[k] == alone.counters[k], k
