@@ -104,6 +104,7 @@ SIGNATURES = {
     "cgp_set_device": (c_int32, [c_int32]),
     "cgp_last_kernel_profile": (c_int32, [POINTER(CgpKernelProfile)]),
     "cgp_debug_fail_allocations": (c_int32, [c_int64]),
+    "cgp_debug_grid_launches": (c_int32, [c_int32]),
     "cgp_graph_create": (c_int32, [c_void_p, c_int32, c_void_p, c_void_p, c_int32, c_int64,
                                    c_int64, c_int32, POINTER(c_void_p)]),
     "cgp_graph_destroy": (c_int32, [c_void_p]),

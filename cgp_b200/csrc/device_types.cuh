@@ -32,6 +32,12 @@ enum : uint32_t {
   kStatusBarrier = 8u,          // a grid barrier gave up waiting (the traversal is incomplete)
 };
 
+// How the fused level loop's grid barrier waits: for this many blocks, this long.
+struct GridWait {
+  uint32_t blocks;
+  uint64_t limit_ns;
+};
+
 struct LevelProfile {
   int32_t level;
   int32_t dir;

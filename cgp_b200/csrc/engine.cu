@@ -27,6 +27,7 @@ namespace {
 // Fault-injection hook for tests: >= 0 counts down the device allocations
 // still allowed before one fails as if the device were out of memory; -1 off.
 std::atomic<int64_t> g_fail_alloc_countdown{-1};
+std::atomic<int32_t> g_grid_failure{CGP_GRID_OK};
 
 bool injected_alloc_failure() {
   int64_t c = g_fail_alloc_countdown.load();
@@ -739,7 +740,10 @@ bool fused_loop(const GroupSpec& spec, const cgp_options& o, const Dispatch& d,
 // weights) keeps coming back to the host.
 constexpr int kFusedLevels = 256;
 
-// Enqueues up to `levels` levels as one cooperative launch.
+// A grid barrier's wait, on a device that runs every block of the launch.
+constexpr uint64_t kBarrierLimitNs = 20ULL * 1000 * 1000 * 1000;
+
+// Enqueues up to `levels` levels as one cooperative launch; 0 when it does not fit.
 int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelLaunch& L,
                   cudaStream_t s, int levels) {
   const TraverseKernel k = d.traverse(spec.has_sssp);
@@ -747,7 +751,11 @@ int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelL
   const int blocks = static_cast<int>(std::max<int64_t>(
       1, std::min<int64_t>(most, (g->E + g->V) / 256)));
   bool heavy = L.heavy_push;
-  void* args[] = {&L.g, &L.G, &levels, &heavy};
+  GridWait wait{static_cast<uint32_t>(blocks), kBarrierLimitNs};
+  const int32_t injected = g_grid_failure.load();
+  if (injected == CGP_GRID_DOES_NOT_FIT) return 0;
+  if (injected == CGP_GRID_BLOCK_MISSING) wait = {wait.blocks + 1, 50 * 1000 * 1000};
+  void* args[] = {&L.g, &L.G, &levels, &heavy, &wait};
   const cudaError_t e = cudaLaunchCooperativeKernel(k.fn, dim3(blocks), dim3(kBlock), args, 0, s);
   if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the GPU is reserved: launch the levels
     cudaGetLastError();
@@ -758,11 +766,13 @@ int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelL
 }
 
 // Enqueues `levels` levels as one launch of the fused loop, as a replayed
-// CUDA graph or as plain launches; levels < 0: the whole traversal as one
-// device-looped graph (a WHILE conditional node around one level, the
-// condition set by the level's last kernel from the done flag).
+// CUDA graph or as plain launches, and returns the kernels launched; levels < 0:
+// the whole traversal as one device-looped graph (a WHILE conditional node
+// around one level, the condition set by the level's last kernel from the done
+// flag).  A fused launch that does not fit becomes at most 8 launched levels:
+// `levels` is then what was enqueued.
 int enqueue_levels(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp_options& o,
-                   cudaStream_t s, int levels, KernelTimer* kt) {
+                   cudaStream_t s, int& levels, KernelTimer* kt) {
   Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
   LevelLaunch L = level_launch(g, ws, spec, o, d);
   if (kt == nullptr && levels > 0 && fused_loop(spec, o, d, L)) {
@@ -859,7 +869,8 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
   const bool device_loop = kt == nullptr && max_levels <= 0 && o.use_cuda_graph &&
                            o.level_loop == CGP_LOOP_DEVICE;
   if (device_loop) {
-    const int per_level = enqueue_levels(g, ws, spec, o, s, -1, nullptr);
+    int whole = -1;
+    const int per_level = enqueue_levels(g, ws, spec, o, s, whole, nullptr);
     ck(cudaStreamSynchronize(s), "device level loop");
     ck(cudaMemcpy(&snap[0], ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost), "read ctl");
     last = 0;
@@ -1210,6 +1221,14 @@ cgp_status cgp_last_profiles(cgp_level_profile* out, int32_t cap, int32_t* count
 
 cgp_status cgp_debug_fail_allocations(int64_t after) {
   g_fail_alloc_countdown.store(after < 0 ? -1 : after);
+  return CGP_OK;
+}
+
+cgp_status cgp_debug_grid_launches(int32_t failure) {
+  clear_error();
+  if (failure < CGP_GRID_OK || failure > CGP_GRID_BLOCK_MISSING)
+    return set_error(CGP_ERR_INVALID_ARG, "unknown grid launch failure");
+  g_grid_failure.store(failure);
   return CGP_OK;
 }
 

@@ -3463,10 +3463,9 @@ __global__ void k_level_end_loop(GroupDev g, cudaGraphConditionalHandle loop, in
 // Barrier over all blocks of a cooperative launch.  The last block to arrive
 // runs `last(lane)` with its first warp before it lets the others go, so the
 // end of a level costs no barrier of its own.  A wait gives up after
-// kBarrierLimitNs (the other blocks are co-resident, so this means the device
-// is not running them), raises kStatusBarrier and tells every block to leave:
-// wait() then returns false in all of them.
-constexpr unsigned long long kBarrierLimitNs = 20ULL * 1000 * 1000 * 1000;
+// `limit_ns` (the other blocks are co-resident, so this means the device is not
+// running them), raises kStatusBarrier and tells every block to leave: wait()
+// then returns false in all of them.
 
 __device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
   unsigned v;
@@ -3486,13 +3485,14 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 struct GridBarrier {
   LevelCtl* ctl;
-  unsigned nblk;
+  unsigned nblk;   // arrivals that complete a barrier
   unsigned epoch;  // barriers passed
+  unsigned long long limit_ns;
 
   // Every block reads the epoch before it first arrives, so none can miss a
   // release of this launch.
-  __device__ __forceinline__ GridBarrier(LevelCtl* c, unsigned n)
-      : ctl(c), nblk(n), epoch(load_acquire(&c->bar_release)) {}
+  __device__ __forceinline__ GridBarrier(LevelCtl* c, const GridWait& w)
+      : ctl(c), nblk(w.blocks), epoch(load_acquire(&c->bar_release)), limit_ns(w.limit_ns) {}
 
   template <typename F>
   __device__ __forceinline__ bool wait(F&& last) {
@@ -3525,7 +3525,7 @@ struct GridBarrier {
           }
           const unsigned long long t = global_ns();
           if (t0 == 0) t0 = t;
-          if (t - t0 > kBarrierLimitNs) {
+          if (t - t0 > limit_ns) {
             atomicOr(&ctl->status, kStatusBarrier);
             __threadfence();
             store_release(&ctl->bar_abort, 1u);
@@ -3567,11 +3567,12 @@ union TraverseSmem {
 // their launches are the level's whole time.
 template <int W, typename OT, int DEPTH, int WK, bool kSssp>
 __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev g, DevGraph G,
-                                                                      int levels, bool heavy) {
+                                                                      int levels, bool heavy,
+                                                                      GridWait wait) {
   __shared__ TraverseSmem<W, kSssp> sm;
   const unsigned bid = blockIdx.x, nblk = gridDim.x;
   LevelCtl* ctl = g.ctl;
-  GridBarrier bar(ctl, nblk);
+  GridBarrier bar(ctl, wait);
   bool swept = false;  // the previous level zeroed its own frontier's masks
   for (int l = 0; l < levels; ++l) {
     if (ctl->done) return;

@@ -279,6 +279,16 @@ cgp_status cgp_autotune(cgp_graph* g, const cgp_query* sample, int32_t n,
  * leaves the graph and its cached state usable. */
 cgp_status cgp_debug_fail_allocations(int64_t after);
 
+/* Fault-injection hook for tests: until it is called with CGP_GRID_OK, every
+ * fused level loop (CGP_LOOP_AUTO) is launched as if the GPU could not hold its
+ * blocks at once (the levels are launched one by one instead), or with a grid
+ * barrier that waits for one block more than there are, for 50 ms (the call
+ * returns CGP_ERR_DEVICE and leaves the graph usable). */
+#define CGP_GRID_OK 0
+#define CGP_GRID_DOES_NOT_FIT 1
+#define CGP_GRID_BLOCK_MISSING 2
+cgp_status cgp_debug_grid_launches(int32_t failure);
+
 /* Per-level profiles of the last cgp_batch_run on this thread (group 0). */
 cgp_status cgp_last_profiles(cgp_level_profile* out, int32_t cap, int32_t* count);
 cgp_status cgp_last_kernel_profile(cgp_kernel_profile* out);

@@ -113,3 +113,41 @@ def test_server_budget_below_one_slot_is_rejected():
         t = s.submit(d, out)
         assert s.wait(t, 60000).state == "done"
     np.testing.assert_array_equal(out, oracle.bfs(g, d.source))
+
+
+@pytest.fixture
+def grid_launches():
+    yield lambda how: N.check(N.lib().cgp_debug_grid_launches(how))
+    N.lib().cgp_debug_grid_launches(0)
+
+
+def _fused_batches():
+    """A grid (more levels than one launch of the fused loop or one fallback
+    chunk holds) with BFS alone, SSSP alone and both."""
+    g = cgp.gen_grid(9, 400, 0.02, 0.0, seed=411).with_weights("u32", 1, 32, seed=412)
+    src, both = _bfs_sssp(g, 24, seed=413)
+    want = _expect(g, src, 24)
+    return cgp.CsrGraph(g), [(both[:12], want[:12]), (both[12:], want[12:]), (both, want)]
+
+
+def test_fused_loop_that_does_not_fit_launches_its_levels(grid_launches):
+    graph, batches = _fused_batches()
+    for descs, want in batches:
+        fused = cgp.run_batch(graph, descs, layout="query")
+        grid_launches(1)
+        r = cgp.run_batch(graph, descs, layout="query")
+        grid_launches(0)
+        np.testing.assert_array_equal(fused.values.view(np.uint32), want)
+        np.testing.assert_array_equal(r.values.view(np.uint32), want)
+        assert r.kernel_launches > 4 * r.iterations > fused.kernel_launches
+
+
+def test_grid_barrier_gives_up_and_the_graph_stays_usable(grid_launches):
+    graph, batches = _fused_batches()
+    for descs, want in batches:
+        grid_launches(2)
+        with pytest.raises(cgp.CgpError, match="grid barrier timed out"):
+            cgp.run_batch(graph, descs, layout="query")
+        grid_launches(0)
+        r = cgp.run_batch(graph, descs, layout="query")
+        np.testing.assert_array_equal(r.values.view(np.uint32), want)
