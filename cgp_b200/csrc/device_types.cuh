@@ -150,11 +150,9 @@ struct DevGraph {
   int64_t V;
   int64_t E;
   const int32_t* heavy;             // vertices with out-degree > heavy_degree
-  const int64_t* heavy_chunk_start; // [n_heavy + 1] prefix of chunk counts
   int32_t n_heavy;
   int64_t heavy_chunks;
   const int32_t* pheavy;            // same for the pull CSR
-  const int64_t* pheavy_chunk_start;
   const int32_t* pheavy_ch;         // per 2048-edge chunk: table index of its vertex
   const int64_t* pheavy_cb;         // per chunk: first in-edge
   const int64_t* pheavy_ce;         // per chunk: one past its last in-edge

@@ -170,11 +170,9 @@ DevGraph GraphImpl::dev_graph(int64_t h, bool light_items) {
   d.V = V;
   d.E = E;
   d.heavy = hp.heavy.vertices.as<int32_t>();
-  d.heavy_chunk_start = hp.heavy.chunk_start.as<int64_t>();
   d.n_heavy = hp.heavy.n;
   d.heavy_chunks = hp.heavy.chunks;
   d.pheavy = hp.pheavy.vertices.as<int32_t>();
-  d.pheavy_chunk_start = hp.pheavy.chunk_start.as<int64_t>();
   d.pheavy_ch = hp.pheavy.chunk_h.as<int32_t>();
   d.pheavy_cb = hp.pheavy.chunk_beg.as<int64_t>();
   d.pheavy_ce = hp.pheavy.chunk_end.as<int64_t>();
@@ -236,7 +234,6 @@ void build_heavy(const std::vector<int64_t>& row, int64_t V, int64_t h, HeavyTab
     }
   }
   t.vertices.ensure(std::max<size_t>(vs.size(), 1) * sizeof(int32_t));
-  t.chunk_start.ensure(cs.size() * sizeof(int64_t));
   t.chunk_h.ensure(std::max<size_t>(ch.size(), 1) * sizeof(int32_t));
   t.chunk_beg.ensure(std::max<size_t>(cb.size(), 1) * sizeof(int64_t));
   t.chunk_end.ensure(std::max<size_t>(ce.size(), 1) * sizeof(int64_t));
@@ -250,8 +247,6 @@ void build_heavy(const std::vector<int64_t>& row, int64_t V, int64_t h, HeavyTab
     ck(cudaMemcpy(t.chunk_end.p, ce.data(), ce.size() * sizeof(int64_t), cudaMemcpyHostToDevice),
        "upload heavy chunk ends");
   }
-  ck(cudaMemcpy(t.chunk_start.p, cs.data(), cs.size() * sizeof(int64_t), cudaMemcpyHostToDevice),
-     "upload heavy chunks");
 }
 
 void build_light_chunks(const std::vector<int64_t>& row, int64_t V, int64_t h, int sms,

@@ -689,22 +689,10 @@ __device__ __forceinline__ void pull_commit(const GroupDev& g, int64_t V, const 
 // ORs the lanes' parts over the lanes with the same words (sub = lane %
 // kLanes): every lane gets its words' union.  All lanes call.
 template <int W>
-__device__ __forceinline__ void part_or_reduce(uint64_t (&m)[PullLanes<W>::kWords], int sub) {
+__device__ __forceinline__ void part_or_reduce(uint64_t (&m)[PullLanes<W>::kWords]) {
   using PL = PullLanes<W>;
-  if constexpr (PL::kLanes <= 2) {
-    // redux.sync: two per word and sub
-#pragma unroll
-    for (int i = 0; i < PL::kWords; ++i) {
-      uint64_t r = 0;
-#pragma unroll
-      for (int k = 0; k < PL::kLanes; ++k) {
-        const uint64_t x = PL::kLanes == 1 || sub == k ? m[i] : 0ULL;
-        const unsigned lo = __reduce_or_sync(kFull, static_cast<unsigned>(x));
-        const unsigned hi = __reduce_or_sync(kFull, static_cast<unsigned>(x >> 32));
-        if (PL::kLanes == 1 || sub == k) r = (static_cast<uint64_t>(hi) << 32) | lo;
-      }
-      m[i] = r;
-    }
+  if constexpr (PL::kLanes == 1) {
+    warp_or_reduce<W>(m);
   } else {
 #pragma unroll
     for (int o = 16; o >= PL::kLanes; o >>= 1) {
@@ -719,7 +707,7 @@ template <int W>
 __device__ __forceinline__ void flush_union_parts(uint64_t (&uni)[PullLanes<W>::kWords],
                                                   uint64_t* dst, int lane) {
   using PL = PullLanes<W>;
-  part_or_reduce<W>(uni, lane % PL::kLanes);
+  part_or_reduce<W>(uni);
   if (lane < PL::kLanes) {
 #pragma unroll
     for (int i = 0; i < PL::kWords; ++i)
@@ -877,7 +865,7 @@ __device__ __forceinline__ void bfs_pull_tiles(const GroupDev& g, const DevGraph
             for (int i = 0; i < WL; ++i) a[i] |= fu[i] & bn[i];
           }
         }
-        part_or_reduce<W>(a, sub);
+        part_or_reduce<W>(a);
         bool full = true;
 #pragma unroll
         for (int i = 0; i < WL; ++i) full &= a[i] == bn[i];
@@ -1146,7 +1134,7 @@ __device__ __forceinline__ void bfs_pull_mid(const GroupDev& g, const DevGraph& 
             for (int k = 0; k < WL; ++k) a[k] |= f[j][k] & need[k];
           }
         }
-        part_or_reduce<W>(a, sub);
+        part_or_reduce<W>(a);
         bool full = true;
 #pragma unroll
         for (int k = 0; k < WL; ++k) full &= a[k] == need[k];
@@ -1253,7 +1241,7 @@ __device__ __forceinline__ void bfs_pull_chunks(const GroupDev& g, const DevGrap
 #pragma unroll
       for (int i = 0; i < WL; ++i) a[i] |= (f[0][i] | f[1][i]) & mine[i];
     }
-    part_or_reduce<W>(a, sub);
+    part_or_reduce<W>(a);
     if (lane < LP) {
 #pragma unroll
       for (int i = 0; i < WL; ++i) s_red[wib][w0 + i] = a[i];
@@ -3014,15 +3002,8 @@ __device__ __forceinline__ void sssp_pull_light_rows(const GroupDev& g, const De
           cm = bound_chunks<W, WK>(g.blo + static_cast<size_t>(u) * (2 * WF) + hoff, s_hi[k], wb) & gch;
         else if (!screened)
           cm = gch;
-        else if (g.fsum != nullptr)
+        else
           cm = (summary_chunks(g.fsum, lv.level, u) >> hoff) & gch;
-        else {
-          uint64_t m[W];
-          load_mask<W>(lv.fcur + static_cast<size_t>(u) * WF + sl * W, m);
-#pragma unroll
-          for (int i = 0; i < W; ++i) m[i] &= ctl->gsel[sl * W + i];
-          cm = chunk_bits<W>(m);
-        }
       }
       if (f0 + 32 < total) load_batch(f0 + 32);
       const bool live = cm != 0;
@@ -3566,9 +3547,9 @@ union TraverseSmem {
 // to do; with small graphs and in the first and last levels of deep ones
 // their launches are the level's whole time.
 template <int W, typename OT, int DEPTH, int WK, bool kSssp>
-__global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev g, DevGraph G,
-                                                                      int levels, bool heavy,
-                                                                      GridWait wait) {
+__global__ void __launch_bounds__(kBlock, 3) k_traverse(GroupDev g, DevGraph G,
+                                                        int levels, bool heavy, GridWait wait) {
+  static_assert(W <= 4, "wider groups are launched level by level");
   __shared__ TraverseSmem<W, kSssp> sm;
   const unsigned bid = blockIdx.x, nblk = gridDim.x;
   LevelCtl* ctl = g.ctl;
@@ -3636,7 +3617,7 @@ __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev 
       if (gather) {
         // heavy vertices first: the light ones read their lowered distances
         if (G.n_sheavy > 0) {
-          sssp_pull_heavy_chunks<W, OT, WK, (W <= 4 ? 3 : 0)>(g, G, bid, nblk, sm.gather_heavy);
+          sssp_pull_heavy_chunks<W, OT, WK, 3>(g, G, bid, nblk, sm.gather_heavy);
           if (!bar.wait()) return;
         } else if (bfs && !bfs_pull && !scatter) {
           // the light gather stores whole vectors of a row: depths a push of this
@@ -3645,7 +3626,7 @@ __global__ void __launch_bounds__(kBlock, (W <= 4 ? 3 : 2)) k_traverse(GroupDev 
           // gather itself only lowers its own words)
           if (!bar.wait()) return;
         }
-        sssp_pull_light_rows<(W < 4 ? W : 4), OT, WK, W>(g, G, bid, nblk, sm.gather_light);
+        sssp_pull_light_rows<W, OT, WK, W>(g, G, bid, nblk, sm.gather_light);
       }
       if (ctl->chunk_dir) {
         if (!bar.wait()) return;
