@@ -289,3 +289,54 @@ def test_pull_edges_counted_for_any_words(words, loop):
         assert r.mask_words == words
         for k in ("pull_vertices", "pull_edges", "new_pairs"):
             assert r.counters[k] == alone.counters[k], k
+
+
+def _islands(sizes, degree, seed):
+    """Random components of the given sizes, about `degree` entries per vertex."""
+    r = np.random.default_rng(seed)
+    src, dst, at = [], [], 0
+    for n in sizes:
+        src.append(at + np.tile(np.arange(n), degree))
+        dst.append(at + r.integers(0, n, n * degree))
+        at += n
+    return at, np.concatenate(src), np.concatenate(dst)
+
+
+def _two_dense_with_hubs(n):
+    """Two components, each a ring of 9 neighbours a side and a hub: one of them
+    is outside whatever root is sampled, with a list of n entries."""
+    r = np.arange(n)
+    src = np.concatenate([np.full(n, n)] + [r] * 9)
+    dst = np.concatenate([r] + [(r + j) % n for j in range(1, 10)])
+    return cgp.csr_from_edges(2 * n + 2, np.r_[src, n + 1 + src], np.r_[dst, n + 1 + dst])
+
+
+def _directed_with_sinks(n, sinks):
+    """A dense directed component and vertices that only its out-entries lead to
+    (high ids, so that they are nobody's first or second neighbour)."""
+    r = np.random.default_rng(61)
+    src = np.r_[np.tile(np.arange(n), 14), r.integers(0, n, sinks)]
+    dst = np.r_[r.integers(0, n, 14 * n), n + np.arange(sinks)]
+    return cgp.csr_from_edges(n + sinks, src, dst, symmetrize=False)
+
+
+@pytest.mark.parametrize("offsets64", [False, True])
+@pytest.mark.parametrize("make,launches", [
+    (lambda: cgp.csr_from_edges(*_islands([900, 40, 1000, 3, 950, 1], 9, 62)), 10),
+    (lambda: cgp.csr_from_edges(*_islands([33] * 200, 12, 63)), 10),
+    (lambda: _two_dense_with_hubs(700), 10),
+    (lambda: cgp.csr_from_edges(*_islands([2000, 1999, 30], 12, 64), symmetrize=False), 11),
+    (lambda: _directed_with_sinks(1500, 400), 11),
+    (lambda: cgp.csr_from_edges(*_islands([500, 20], 3, 65)), 4),
+])
+def test_wcc_by_sampling_and_by_every_entry(make, launches, offsets64):
+    """From 8 entries per vertex on the neighbours are sampled (8 kernels, 9 with
+    the transpose of a directed graph, then labels and a column), below every
+    entry is linked."""
+    g = make()
+    graph = cgp.CsrGraph(g, offsets64=offsets64)
+    assert (g.num_edges >= 8 * g.num_vertices) == (launches > 4)
+    for _ in range(3):
+        r = cgp.run("wcc", graph, [0])
+        assert r.kernel_launches == launches
+        np.testing.assert_array_equal(r.values[:, 0].view(np.uint32), oracle.wcc_components(g))
