@@ -123,7 +123,9 @@ typedef struct {
   int32_t serve_admission;    /* serving loop: 0 = any free slot, preferring the chunk of the
                                  latest admissions; 1 = whole 32-slot cohorts: requests enter
                                  only chunks whose slots are all free; 2 = group cohorts:
-                                 requests enter only an empty group, all pending at once     */
+                                 requests enter only an empty group, all pending at once;
+                                 with several groups, none of them empty, the rest of a burst
+                                 (0.5 ms between admissions, 5 ms in all) joins its cohort   */
   int32_t serve_groups;       /* serving loop: traversal groups the slots are split into, each
                                  with its own masks and stream, their levels overlapping on
                                  the device (1..8); 0 = 1                                    */

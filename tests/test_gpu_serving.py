@@ -220,3 +220,28 @@ def test_retire_mixes_device_host_and_discarded_outputs(rmat, policy):
             continue
         got = o.cpu().numpy().view(np.uint32) if hasattr(o, "cpu") else o
         np.testing.assert_array_equal(got, _expected(g, d))
+
+
+def test_group_cohorts_take_a_single_request_at_once():
+    """A request that finds an idle group is admitted in the next pass, also
+    while another group runs a cohort."""
+    g = cgp.gen_grid(256, 256, 0.05, 0.0, seed=71).with_weights("u32", 1, 16, seed=72)
+    graph = cgp.CsrGraph(g)
+    a, b = (cgp.QueryDescriptor(int(s), "sssp") for s in g.pick_sources(2, seed=73))
+    outs = [np.zeros(g.num_vertices, np.uint32) for _ in range(2)]
+    opts = cgp.RunOptions(serve_admission="group", serve_groups=2, levels_per_sync=1)
+    waits = []
+    with cgp.Server(graph, slots=64, options=opts) as s:
+        for _ in range(15):
+            first = s.submit(a, outs[0])
+            while s.poll(first).state == "queued":
+                time.sleep(0.0002)
+            time.sleep(0.002)
+            second = s.submit(b, outs[1])
+            s.drain(timeout_ms=60000)
+            i = s.poll(second)
+            assert i.admit_ms < s.poll(first).finish_ms
+            waits.append(i.admit_ms - i.submit_ms)
+    for d, o in zip((a, b), outs):
+        np.testing.assert_array_equal(o, _expected(g, d))
+    assert np.median(waits) < 0.3, waits  # a level takes 0.1 ms
