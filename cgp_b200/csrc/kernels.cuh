@@ -2615,6 +2615,101 @@ __device__ __forceinline__ void gather_edges_vec(const GroupDev& g, const DevGra
   }
 }
 
+// The same for the warp-per-vertex kernel below, whose register budget (4 blocks
+// of 64 registers per SM at W = 4) holds neither a batch loaded ahead nor the
+// predicated row loads: loads under branches, 0xffffffff where nothing is read.
+// 120 and 200 slots on R-MAT 20, all lists by warps: 39 and 76 ms against 97 and 119
+// with gather_edges_vec.
+template <int W, int WK>
+__device__ __forceinline__ void gather_vertex_edges(const GroupDev& g, const DevGraph& G,
+                                                    const LevelView& lv, uint32_t pmask,
+                                                    int64_t eb, int64_t ee, int lane, int4* stage,
+                                                    uint32_t (&best)[GatherVec<W>::kSlots],
+                                                    unsigned long long& pairs, unsigned& scanned,
+                                                    int screen_qs, uint32_t gch) {
+  using GV = GatherVec<W>;
+  constexpr int E = GV::kElem;
+  constexpr int S = GV::kSteps;
+  const size_t Qg = static_cast<size_t>(g.Qg);
+  const uint32_t* lanebase = g.values + lane * E;
+  for (int64_t e0 = eb; e0 < ee; e0 += 32) {
+    const int64_t e = e0 + lane;
+    int k = 0;
+    int32_t u = 0;
+    uint32_t wb = 0;
+    uint32_t cm = 0xffffffffu;  // 32-slot chunks of the source row to read
+    if (e < ee) {
+      u = G.pcol[e];
+      wb = weight_bits<WK>(G.pw, e);
+      if (screen_qs < 0) {
+        cm = summary_chunks(g.fsum, lv.level, u) & gch;
+        k = __popc(cm) << 5;
+      } else {
+        k = screen_qs;
+      }
+      ++scanned;
+    }
+    pairs += static_cast<unsigned long long>(k);
+    const unsigned lm = __ballot_sync(kFull, k > 0);
+    if (k > 0)
+      stage[__popc(lm & ((1u << lane) - 1u))] =
+          make_int4(u, static_cast<int>(wb), 0, static_cast<int>(cm));
+    __syncwarp();
+    const int n = __popc(lm);
+    int i = 0;
+    for (; i + S <= n; i += S) {
+      int4 ed[S];
+#pragma unroll
+      for (int t = 0; t < S; ++t) ed[t] = stage[i + t];
+      uint32_t cur[S][GV::kSlots];
+#pragma unroll
+      for (int t = 0; t < S; ++t) {
+        const uint32_t* row = lanebase + static_cast<size_t>(ed[t].x) * Qg;
+#pragma unroll
+        for (int r = 0; r < GV::kParts; ++r) {
+          if (((pmask >> r) & 1u) && ((static_cast<uint32_t>(ed[t].w) >> (((32 * r + lane) * E) >> 5)) & 1u)) {
+            load_vec_cg<E>(row + 32 * E * r, &cur[t][r * E]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < E; ++q) cur[t][r * E + q] = 0xffffffffu;
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < S; ++t) {
+#pragma unroll
+        for (int j = 0; j < GV::kSlots; ++j)
+          best[j] = min(best[j], gather_relax<WK>(cur[t][j], static_cast<uint32_t>(ed[t].y)));
+      }
+    }
+    if (i < n) {
+      int4 ed[S];
+#pragma unroll
+      for (int t = 0; t < S; ++t) ed[t] = stage[i + t < n ? i + t : i];
+      uint32_t cur[S][GV::kSlots];
+#pragma unroll
+      for (int t = 0; t < S; ++t) {
+        const uint32_t* row = lanebase + static_cast<size_t>(ed[t].x) * Qg;
+#pragma unroll
+        for (int r = 0; r < GV::kParts; ++r) {
+          if (i + t < n && ((pmask >> r) & 1u) && ((static_cast<uint32_t>(ed[t].w) >> (((32 * r + lane) * E) >> 5)) & 1u)) {
+            load_vec_cg<E>(row + 32 * E * r, &cur[t][r * E]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < E; ++q) cur[t][r * E + q] = 0xffffffffu;
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < S; ++t) {
+#pragma unroll
+        for (int j = 0; j < GV::kSlots; ++j)
+          best[j] = min(best[j], gather_relax<WK>(cur[t][j], static_cast<uint32_t>(ed[t].y)));
+      }
+    }
+    __syncwarp();
+  }
+}
 
 // Gather level (vectorised), vertices of in-degree <= heavy_degree.
 template <int W, typename OT, int WK>
@@ -2628,7 +2723,6 @@ __global__ void __launch_bounds__(kBlock, (W == 4 ? 4 : (W <= 8 ? 3 : 2))) k_sss
   const LevelView lv = level_view(g);
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
-  const uint64_t* sb = ctl->gsel;
   uint32_t pmask, smask;
   gather_vec_masks<W>(ctl->gsel, g.Qg, lane, &pmask, &smask);
   const unsigned long long gw = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -2668,8 +2762,8 @@ __global__ void __launch_bounds__(kBlock, (W == 4 ? 4 : (W <= 8 ? 3 : 2))) k_sss
         for (int q = 0; q < E; ++q) best[r * E + q] = 0u;
       }
     }
-    gather_edges_vec<W, WK>(g, G, lv, sb, pmask, beg, end, lane, s_stage[wib], best, pairs,
-                            scanned, screen_qs, gch);
+    gather_vertex_edges<W, WK>(g, G, lv, pmask, beg, end, lane, s_stage[wib], best, pairs, scanned,
+                               screen_qs, gch);
     // commit (the warp owns v's row this level: the row read above is current)
     uint32_t imp = 0;
 #pragma unroll
