@@ -152,6 +152,7 @@ cgp_status cgp_enactor_enact(cgp_enactor* e, cgp_stats* stats) {
     ck(cudaEventRecord(t0, e->stream), "event");
     cgp_options o = e->opts;
     o.use_cuda_graph = 1;
+    const OnDevice running(e->g->device);
     GroupRun r;
     group_enact(e->g, e->ws.get(), e->spec, o, e->stream, &r, 0);
     ck(cudaEventRecord(t1, e->stream), "event");

@@ -22,6 +22,24 @@ namespace cgp {
 
 using namespace dev;
 
+// --------------------------------------------------- traversals per device
+OnDevice::Load OnDevice::loads_[OnDevice::kDevices];
+
+static int64_t steady_ns() {
+  return std::chrono::duration_cast<std::chrono::nanoseconds>(
+             std::chrono::steady_clock::now().time_since_epoch()).count();
+}
+
+OnDevice::OnDevice(int device) : load_(loads_[device % kDevices]) {
+  if (++load_.running > 1) load_.shared_until = steady_ns() + kSharedNs;
+}
+
+int OnDevice::callers(int device) {
+  const Load& l = loads_[device % kDevices];
+  const int n = l.running;
+  return n < 2 && steady_ns() < l.shared_until ? 2 : n;
+}
+
 // ------------------------------------------------------------- buffers
 namespace {
 // Fault-injection hook for tests: >= 0 counts down the device allocations
@@ -716,16 +734,42 @@ LevelLaunch level_launch(GraphImpl* g, Workspace* ws, const GroupSpec& spec, con
 // against 12.3; a 1024-slot grid, 36M: 253 against 209).
 constexpr int64_t kFusedWork = 1 << 24;
 
+// Blocks of a fused launch: one per 256 vertices and entries, as far as the GPU
+// holds them all at once.
+int fused_blocks(const GraphImpl* g, int most) {
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, (g->E + g->V) / 256)));
+}
+
 // Whether the group's levels run as the fused loop: the automatic loop form,
 // with the kernel variants the loop holds (the default ones).
-bool fused_loop(const GroupSpec& spec, const cgp_options& o, const Dispatch& d,
-                const LevelLaunch& L) {
+bool fused_loop(const GraphImpl* g, const GroupSpec& spec, const cgp_options& o,
+                const Dispatch& d, const LevelLaunch& L) {
   if (spec.W > 4 || (spec.has_sssp && L.G.E * spec.W > kFusedWork)) return false;
   if (o.level_loop != CGP_LOOP_AUTO || !o.use_cuda_graph || o.bfs_pull_form != 0) return false;
   // serving groups on streams of their own: launched levels of different
   // groups overlap on the device, cooperative launches take all of it in turn
   if (spec.serving && (o.serve_groups > 1 || o.serve_admission == 2)) return false;
-  if (d.traverse(spec.has_sssp).per_sm < 1) return false;
+  const int most = d.traverse(spec.has_sssp).per_sm * g->num_sms;
+  if (most < 1) return false;
+  const int64_t work = L.G.E * spec.W;
+  const bool short_lists = !L.heavy_push;  // no list above 32 edges: many levels as a rule
+  // Beside other traversals only tiny groups, and others as far as their launches
+  // do not queue up: cooperative launches that do not fit next to each other run in
+  // turn, each leaving the GPU idle at its barriers, where launched levels
+  // interleave.  Calls/s of 2, 4 and 8 callers, fused against launched: 256 BFS on
+  // R-MAT 20 557, 559, 563 against 586, 646, 656; mixed R-MAT 17 801, 836, 845
+  // against 830, 1051, 1117; 16 SSSP on a 96 x 97 grid (a third of the GPU's blocks)
+  // 997, 1024, 1014 against 650, 966, 1121; but one BFS on R-MAT 11 14152, 26189,
+  // 25108 against 6328, 10429, 8878, and on R-MAT 12 12305, 12096, 12202 against
+  // 6252, 10734, 11703: a traversal of a few levels on so small a graph is over
+  // before the next call's launch.  One BFS on R-MAT 12 beside the R-MAT 20 batch
+  // took 400 us (90%: 1590) when both were fused, 184 (359) by this rule.
+  const int callers = OnDevice::callers(g->device), blocks = fused_blocks(g, most);
+  if (callers > 1 && work > (spec.has_sssp ? 1 << 15 : 1 << 16)) {
+    if (2 * callers * blocks > 5 * most) return false;
+    const bool quick = !spec.has_sssp && !short_lists && work <= 1 << 18;
+    if (5 * blocks > 3 * most && !quick) return false;
+  }
   if (spec.has_sssp && (L.dense_unroll == 2 || (L.spull && !(L.gvec && L.lchunks)))) return false;
   return true;
 }
@@ -742,9 +786,7 @@ constexpr uint64_t kBarrierLimitNs = 20ULL * 1000 * 1000 * 1000;
 int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelLaunch& L,
                   cudaStream_t s, int levels) {
   const TraverseKernel k = d.traverse(spec.has_sssp);
-  const int most = k.per_sm * g->num_sms;
-  const int blocks = static_cast<int>(std::max<int64_t>(
-      1, std::min<int64_t>(most, (g->E + g->V) / 256)));
+  const int blocks = fused_blocks(g, k.per_sm * g->num_sms);
   bool heavy = L.heavy_push;
   GridWait wait{static_cast<uint32_t>(blocks), kBarrierLimitNs};
   const int32_t injected = g_grid_failure.load();
@@ -760,17 +802,17 @@ int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelL
   return 1;
 }
 
-// Enqueues `levels` levels as one launch of the fused loop, as a replayed
+// Enqueues `levels` levels as one launch of the fused loop (`fused`), as a replayed
 // CUDA graph or as plain launches, and returns the kernels launched; levels < 0:
 // the whole traversal as one device-looped graph (a WHILE conditional node
 // around one level, the condition set by the level's last kernel from the done
 // flag).  A fused launch that does not fit becomes at most 8 launched levels:
 // `levels` is then what was enqueued.
 int enqueue_levels(GraphImpl* g, Workspace* ws, const GroupSpec& spec, const cgp_options& o,
-                   cudaStream_t s, int& levels, KernelTimer* kt) {
+                   cudaStream_t s, int& levels, KernelTimer* kt, bool fused) {
   Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
   LevelLaunch L = level_launch(g, ws, spec, o, d);
-  if (kt == nullptr && levels > 0 && fused_loop(spec, o, d, L)) {
+  if (fused) {
     const int n = enqueue_fused(g, spec, d, L, s, levels);
     if (n > 0) return n;
     levels = std::min(levels, 8);
@@ -850,7 +892,7 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
   bool fused = false;
   if (kt == nullptr) {
     const Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
-    fused = fused_loop(spec, o, d, level_launch(g, ws, spec, o, d));
+    fused = fused_loop(g, spec, o, d, level_launch(g, ws, spec, o, d));
   }
   const int per_chunk = kt ? 1 : (o.levels_per_sync > 0 ? o.levels_per_sync
                                                         : (fused ? kFusedLevels : 8));
@@ -865,7 +907,7 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
                            o.level_loop == CGP_LOOP_DEVICE;
   if (device_loop) {
     int whole = -1;
-    const int per_level = enqueue_levels(g, ws, spec, o, s, whole, nullptr);
+    const int per_level = enqueue_levels(g, ws, spec, o, s, whole, nullptr, false);
     ck(cudaStreamSynchronize(s), "device level loop");
     ck(cudaMemcpy(&snap[0], ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost), "read ctl");
     last = 0;
@@ -886,7 +928,7 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
       return x;
     };
     const double before = kt ? level_sum(kt) : 0.0;
-    spec.launches += enqueue_levels(g, ws, spec, o, s, n, kt);
+    spec.launches += enqueue_levels(g, ws, spec, o, s, n, kt, fused);
     enqueued += n;
     ck(cudaMemcpyAsync(&snap[chunk & 1], ws->ctl.p, sizeof(LevelCtl), cudaMemcpyDeviceToHost, s),
        "read ctl");
@@ -971,7 +1013,9 @@ void group_enact(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options
 
 void group_enqueue_levels(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_options& o,
                           cudaStream_t s, int levels) {
-  spec.launches += enqueue_levels(g, ws, spec, o, s, levels, nullptr);
+  const Dispatch d = dispatch(spec.W, g->offset_bytes, spec.depth_mode, g->weight_kind);
+  const bool fused = fused_loop(g, spec, o, d, level_launch(g, ws, spec, o, d));
+  spec.launches += enqueue_levels(g, ws, spec, o, s, levels, nullptr, fused);
 }
 
 void group_write_output(GraphImpl* g, Workspace* ws, GroupSpec& spec, OutMap om,
@@ -1349,6 +1393,7 @@ cgp_status cgp_batch_run(cgp_graph* graph, const cgp_query* queries, int32_t nq,
                       spec.depth_mode != kDepthPlanes;
       if (pad_rows(g, ws.get(), spec, o, in_place)) in_place = false;
       if (in_place) spec.external_values = dout;
+      const OnDevice running(g->device);
       if (kt) kt->mark(kClassInit, s);
       group_prepare(g, ws.get(), spec, o, s);
       GroupRun r;

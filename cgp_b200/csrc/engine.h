@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <map>
 #include <memory>
@@ -31,6 +32,30 @@ struct ApiError {
 inline void ck(cudaError_t e, const char* where) {
   if (e != cudaSuccess) throw CudaError{e, where};
 }
+
+// A traversal that is on a device: its group is being started, its levels run or
+// its results are being written.
+class OnDevice {
+ public:
+  explicit OnDevice(int device);
+  ~OnDevice() { --load_.running; }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+  // Traversals on the device now, over every graph, thread and kind of call; at
+  // least 2 for a while after any two have run side by side, so that callers who
+  // share a device are seen between their calls too.
+  static int callers(int device);
+
+ private:
+  struct Load {
+    std::atomic<int> running{0};
+    std::atomic<int64_t> shared_until{0};  // steady clock, ns
+  };
+  static constexpr int kDevices = 64;
+  static constexpr int64_t kSharedNs = 100 * 1000 * 1000;
+  static Load loads_[kDevices];
+  Load& load_;
+};
 
 // One device allocation that only grows.
 struct DevBuf {

@@ -20,6 +20,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <deque>
+#include <optional>
 #include <thread>
 #include <unordered_map>
 
@@ -633,6 +634,7 @@ void cgp_server::loop() {
       // timing the groups' level chunks are enqueued on their own streams
       // first and waited for afterwards, so they overlap on the device
       bool any = false;
+      std::optional<OnDevice> running;
       for (ServeGroup& gr : groups) {
         gr.ran = false;
         int act;
@@ -646,6 +648,7 @@ void cgp_server::loop() {
         }
         gr.ran = true;
         any = true;
+        if (!running) running.emplace(g->device);
         if (kt) {
           GroupRun r;
           group_enact(g, gr.ws.get(), gr.spec, o, gr.stream, &r, per, kt.get());
@@ -659,6 +662,7 @@ void cgp_server::loop() {
       if (!any) continue;
       for (ServeGroup& gr : groups)
         if (gr.ran) ck(cudaStreamSynchronize(gr.stream), "levels");
+      running.reset();
       busy_ms += now_ms() - tb;
       for (ServeGroup& gr : groups) {
         if (!gr.ran) continue;

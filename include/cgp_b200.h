@@ -141,10 +141,11 @@ typedef struct {
 
 /* level_loop values.  AUTO: BFS groups of up to 256 slots, and groups with SSSP
  * slots up to 2^24 (edge, mask word) pairs, run up to 256 levels per cooperative
- * launch (levels_per_sync, when given, instead of 256); others as CHUNKS.  CHUNKS: CUDA graphs of levels_per_sync levels, the host
- * reads the control block once per chunk (one chunk in flight).  DEVICE: one
- * CUDA graph whose WHILE conditional node runs a level per iteration until
- * the device-side done flag is set: the host waits once per traversal (it
+ * launch (levels_per_sync, when given, instead of 256); others, and where several
+ * callers share the device, as CHUNKS.  CHUNKS: CUDA graphs of levels_per_sync
+ * levels, the host reads the control block once per chunk (one chunk in flight).
+ * DEVICE: one CUDA graph whose WHILE conditional node runs a level per iteration
+ * until the device-side done flag is set: the host waits once per traversal (it
  * replaces the reference's per-level host synchronisation,
  * frontier_engine.hxx:3044-3071); kernels inside a graph with conditional nodes
  * are invisible to kernel profilers, so it is asked for explicitly. */

@@ -291,6 +291,37 @@ def test_pull_edges_counted_for_any_words(words, loop):
             assert r.counters[k] == alone.counters[k], k
 
 
+@pytest.mark.parametrize("kind", ["bfs", "sssp"])
+def test_calls_beside_one_another_launch_their_levels(kind):
+    """A traversal that would take the whole GPU for its levels runs them one
+    launch each while others are on the device, and as one launch alone."""
+    import threading
+    import time
+    g = cgp.gen_rmat(15, 16, seed=51).with_weights("u32", 1, 64, seed=52)
+    graph = cgp.CsrGraph(g)
+    src = g.pick_sources(48, seed=53)
+    want = oracle.batch(kind, g, src)[0]
+    descs = [cgp.QueryDescriptor(int(s), kind) for s in src]
+    launched, exact = [0, 0, 0], [0, 0, 0]
+
+    def caller(i):
+        for _ in range(15):
+            r = cgp.run_batch(graph, descs, layout="query")
+            exact[i] += np.array_equal(r.values, want)
+            launched[i] += r.kernel_launches > 2 * r.iterations
+
+    threads = [threading.Thread(target=caller, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert exact == [15, 15, 15] and sum(launched) > 0
+    time.sleep(0.3)  # callers count as side by side for 0.1 s
+    alone = cgp.run_batch(graph, descs, layout="query")
+    assert alone.kernel_launches < alone.iterations + 3
+    np.testing.assert_array_equal(alone.values, want)
+
+
 def _islands(sizes, degree, seed):
     """Random components of the given sizes, about `degree` entries per vertex."""
     r = np.random.default_rng(seed)
