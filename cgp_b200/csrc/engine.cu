@@ -733,6 +733,8 @@ LevelLaunch level_launch(GraphImpl* g, Workspace* ws, const GroupSpec& spec, con
 // launched kernels' own register budgets do (R-MAT 20, 256 slots, 126M: 12.7
 // against 12.3; a 1024-slot grid, 36M: 253 against 209).
 constexpr int64_t kFusedWork = 1 << 24;
+// Edges x slots up to which groups that only scatter run fused (see fused_loop).
+constexpr int64_t kFusedScatter = 1 << 21;
 
 // Blocks of a fused launch: one per 256 vertices and entries, as far as the GPU
 // holds them all at once.
@@ -753,6 +755,11 @@ bool fused_loop(const GraphImpl* g, const GroupSpec& spec, const cgp_options& o,
   if (most < 1) return false;
   const int64_t work = L.G.E * spec.W;
   const bool short_lists = !L.heavy_push;  // no list above 32 edges: many levels as a rule
+  // Scatter levels want more warps per SM than the loop's register budget leaves:
+  // groups that only scatter run fused while launches weigh more.  Push mode, 64
+  // slots on 150K vertices of 10 out-edges: 5.2 ms fused, 4.1 launched; one slot
+  // 0.67 against 0.72.  (Gathering, 100 slots on 200K vertices: 3.2 against 3.4.)
+  if (spec.has_sssp && !L.spull && short_lists && L.G.E * spec.n > kFusedScatter) return false;
   // Beside other traversals only tiny groups, and others as far as their launches
   // do not queue up: cooperative launches that do not fit next to each other run in
   // turn, each leaving the GPU idle at its barriers, where launched levels

@@ -140,8 +140,9 @@ typedef struct {
 } cgp_options;
 
 /* level_loop values.  AUTO: BFS groups of up to 256 slots, and groups with SSSP
- * slots up to 2^24 (edge, mask word) pairs, run up to 256 levels per cooperative
- * launch (levels_per_sync, when given, instead of 256); others, and where several
+ * slots up to 2^24 (edge, mask word) pairs (2^21 (edge, slot) pairs where levels
+ * only scatter over short lists), run up to 256 levels per cooperative launch
+ * (levels_per_sync, when given, instead of 256); others, and where several
  * callers share the device, as CHUNKS.  CHUNKS: CUDA graphs of levels_per_sync
  * levels, the host reads the control block once per chunk (one chunk in flight).
  * DEVICE: one CUDA graph whose WHILE conditional node runs a level per iteration

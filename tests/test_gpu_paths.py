@@ -322,6 +322,22 @@ def test_calls_beside_one_another_launch_their_levels(kind):
     np.testing.assert_array_equal(alone.values, want)
 
 
+@pytest.mark.parametrize("q,fused", [(1, True), (3, True), (4, False), (64, False)])
+def test_scatter_only_groups_by_edges_and_slots(q, fused):
+    """Push mode over short lists: few (edge, slot) pairs in one launch, more
+    than 2^21 level by level."""
+    r = np.random.default_rng(71)
+    n = 60000
+    g = cgp.csr_from_edges(n, r.integers(0, n, 10 * n), r.integers(0, n, 10 * n), symmetrize=False)
+    g = g.with_weights("u32", 1, 64, seed=72)
+    assert 3 * g.num_edges <= 1 << 21 < 4 * g.num_edges and g.degrees().max() <= 32
+    src = r.integers(0, n, q)
+    got = cgp.run("sssp", cgp.CsrGraph(g), src, options=cgp.RunOptions(traversal_mode="push"),
+                  layout="query")
+    assert (got.kernel_launches < got.iterations) == fused
+    np.testing.assert_array_equal(got.values.view(np.uint32), oracle.batch("sssp", g, src)[0])
+
+
 def _islands(sizes, degree, seed):
     """Random components of the given sizes, about `degree` entries per vertex."""
     r = np.random.default_rng(seed)
