@@ -55,19 +55,6 @@ sys.path.insert(0, str(ROOT))
 L2_BYTES = 126 * 2**20
 BFS_INF = 2**31 - 1
 
-# DRAM bytes per level of a level class from ncu captures (dram__bytes_read.sum
-# + dram__bytes_write.sum summed over the level's kernels), with where and when
-# they were measured.  Reported beside the run's own numbers; never computed
-# from files at run time.
-NCU_TRAFFIC = {
-    ("c2", "sssp_gather"): {
-        "bytes_per_level": 2.93e10,
-        "source": "profiles/dram_traffic_sssp_gather_rmat22.md (ncu, full size, mean of 4 levels)",
-        "captured": "2026-12-05",
-    },
-}
-
-
 WORKLOADS = {
     "c1": {"graph": "rmat", "scale": 16, "edge_factor": 16, "weights": None,
            "groups": [("bfs", 64)], "wcc": False, "sources": "non-isolated"},
@@ -400,7 +387,6 @@ def roofline_line(args, kclass):
     sec = k["ms"] / 1e3
     achieved = k["compulsory"] / sec / 1e9
     alg = k["bytes"] / sec / 1e9
-    tr = NCU_TRAFFIC.get((args.workload, dom))
     line = {"bound": "hbm", "kernel": f"{dom} levels ({CLASS_KERNELS[dom]})",
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peak_src == "measured"
@@ -409,9 +395,6 @@ def roofline_line(args, kclass):
                      "written once",
             "per": "level", "compulsory_bytes_per_launch": k["compulsory"] / n,
             "ms_per_launch": k["ms"] / n,
-            "traffic": tr["bytes_per_level"] if tr else None,
-            "traffic_source": (f"{tr['source']}, captured {tr['captured']}" if tr else None),
-            "dram_frac": (tr["bytes_per_level"] / (k["ms"] / n / 1e3) / 1e9 / peak if tr else None),
             "l2_inclusive": {"achieved": alg, "frac": alg / peak,
                              "bytes_per_launch": k["bytes"] / n,
                              "note": "every (edge, slot) access charged, L2 hits included"},
