@@ -5,9 +5,9 @@
 // (puercgp/include/puercgp/engine/frontier_engine.hxx:2203-3139) and
 // hybrid_frontier_engine::run (hybrid_engine.hxx:793-1141).  The reference
 // copies one or two counters to the host and synchronises after every level;
-// here the direction decision, counter resets and convergence test run in a
-// one-thread kernel at the end of each level, and the host only looks at the
-// control block once per chunk of levels.
+// here the direction decision, counter resets and convergence test run in one
+// warp at the end of each level, and the host only looks at the control block
+// once per chunk of levels or once per launch of the fused loop.
 #include <algorithm>
 #include <atomic>
 #include <chrono>

@@ -736,11 +736,11 @@ __device__ __forceinline__ bool bfs_pull_uses_summary(const GroupDev& g, const L
 // Pull level (bottom-up): every non-heavy vertex with unvisited active bits
 // ORs the current-frontier masks of its in-neighbours until every needed bit
 // is found (early exit).  Reads only the current frontier, so depths are
-// exactly level-synchronous.  Vertex order by default (a tile is 32
+// exactly level-synchronous.  Vertex order by default (a tile is kGroups
 // consecutive vertices); with bfs_chunked == 2 the tiles run over the light
-// table's vertices of in-degree 1..32 in decreasing in-degree order, so the
-// lanes of a warp walk lists of about the same length (the next masks of the
-// vertices left out are zeroed by k_clear_next).
+// table's vertices of in-degree 1..mid_degree (8 or 32) in decreasing in-degree
+// order, so the lanes of a warp walk lists of about the same length (the next
+// masks of the vertices left out are zeroed by k_clear_next).
 template <int W, typename OT, int DEPTH>
 __device__ __forceinline__ void bfs_pull_tiles(const GroupDev& g, const DevGraph& G, unsigned bid,
                                                unsigned nblk) {
@@ -2880,11 +2880,10 @@ __device__ __forceinline__ uint32_t chunk_word(uint32_t bits, int lane, int* chu
 // current ones are worked on.  Groups of more than 256 slots are taken in
 // slices of 4 words, slice by slice over all items.
 //
-// What bounds it: reading rows from L2 (a loop that only reads and relaxes
-// 1 KB rows in R-MAT 20's order reaches 16.7 TB/s).  The form before it, a CTA
-// per 32 vertices with row minima merged in shared memory, spent most of its
-// time outside that: 8.4 TB/s when every row is read, and 1.4 ms for a level
-// that reads 1% of them.
+// What bounds it: reading rows from L2 where every row is read; the chain column
+// -> bound -> row where few are.  The form before it, a CTA per 32 vertices with
+// row minima merged in shared memory, spent most of its time outside that: 1.4 ms
+// for a level of R-MAT 20 that reads 1% of the row chunks.
 constexpr int kRowStage = 64;  // 32 in-edges and as many own rows
 
 struct GatherRowSmem {

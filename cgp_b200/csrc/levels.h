@@ -37,7 +37,7 @@ struct LevelLaunch {
   bool spull;        // SSSP gather kernels are part of the level
   bool gvec;         // rows allow the vectorised gather (alignment, width)
   bool lchunks;      // light vertices gathered by items (in 4-word slices above W = 4)
-  int dense_unroll;  // edges per step of the dense SSSP kernel (1 or 2)
+  int dense_unroll;  // edges per step of the SSSP list kernel (1: 4, 2: 8)
   KernelTimer* kt;   // per-class event timing (non-graph runs only)
   bool heavy_push = false;                // heavy-queue push kernels are part of a level
   bool bfs_chunked = false;               // chunked light-vertex BFS pull is part of a pull level
