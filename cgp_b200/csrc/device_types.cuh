@@ -21,6 +21,8 @@ constexpr int kGatherHeavy = 256;       // in-edges one warp of the row gather t
                                         // of 32; the 8 warps of a CTA share longer lists
 
 enum : int32_t { kDirPush = 0, kDirPull = 1 };
+// k_traverse: long lists go to the heavy queue; block 0 leaves at once (for tests).
+enum : int32_t { kTraverseHeavy = 1, kTraverseBlockMissing = 2 };
 enum : int32_t { kDepthNone = 0, kDepthDirect = 1, kDepthPlanes = 2 };
 enum : int32_t { kWeightNone = 0, kWeightU32 = 1, kWeightF32 = 2 };
 
@@ -30,12 +32,6 @@ enum : uint32_t {
   kStatusLevelCap = 2u,         // a device-looped traversal reached its level cap
   kStatusQueueOverflow = 4u,    // the heavy frontier queue was full (entry dropped)
   kStatusBarrier = 8u,          // a grid barrier gave up waiting (the traversal is incomplete)
-};
-
-// How the fused level loop's grid barrier waits: for this many blocks, this long.
-struct GridWait {
-  uint32_t blocks;
-  uint64_t limit_ns;
 };
 
 struct LevelProfile {
@@ -125,6 +121,7 @@ struct LevelCtl {
   int32_t bnd_wait;                 // gather levels left before bounds are tried again
   int32_t bnd_fail;                 // tries in a row that skipped too few
   int32_t gathers;                  // gather levels so far
+  unsigned long long bar_limit_ns;  // longest wait at a grid barrier
   uint32_t bar_arrived;             // grid barrier of the fused level loop: blocks arrived,
   uint32_t bar_release;             // barriers passed,
   uint32_t bar_abort;               // and nonzero once a wait has given up

@@ -46,6 +46,10 @@ namespace {
 // still allowed before one fails as if the device were out of memory; -1 off.
 std::atomic<int64_t> g_fail_alloc_countdown{-1};
 std::atomic<int32_t> g_grid_failure{CGP_GRID_OK};
+// A grid barrier's wait, on a device that runs every block of the launch; and
+// where a block is missing on purpose.
+constexpr unsigned long long kBarrierNs = 20ULL * 1000 * 1000 * 1000;
+constexpr unsigned long long kInjectedBarrierNs = 50ULL * 1000 * 1000;
 
 bool injected_alloc_failure() {
   int64_t c = g_fail_alloc_countdown.load();
@@ -673,6 +677,7 @@ void group_prepare(GraphImpl* g, Workspace* ws, GroupSpec& spec, const cgp_optio
                    hp.plight.chunks > 0) ? o.bfs_pull_form : 0;
   c.has_bfs = spec.has_bfs ? 1 : 0;
   c.bnd_avail = spec.bounds ? 1 : 0;
+  c.bar_limit_ns = g_grid_failure.load() == CGP_GRID_BLOCK_MISSING ? kInjectedBarrierNs : kBarrierNs;
   c.prev_dir = kDirPush;
   c.sssp_pull_edge_threshold = static_cast<unsigned long long>(
       std::max(1.0, o.sssp_pull_edge_ratio * static_cast<double>(g->E)));
@@ -786,20 +791,16 @@ bool fused_loop(const GraphImpl* g, const GroupSpec& spec, const cgp_options& o,
 // weights) keeps coming back to the host.
 constexpr int kFusedLevels = 256;
 
-// A grid barrier's wait, on a device that runs every block of the launch.
-constexpr uint64_t kBarrierLimitNs = 20ULL * 1000 * 1000 * 1000;
-
 // Enqueues up to `levels` levels as one cooperative launch; 0 when it does not fit.
 int enqueue_fused(GraphImpl* g, const GroupSpec& spec, const Dispatch& d, LevelLaunch& L,
                   cudaStream_t s, int levels) {
   const TraverseKernel k = d.traverse(spec.has_sssp);
   const int blocks = fused_blocks(g, k.per_sm * g->num_sms);
-  bool heavy = L.heavy_push;
-  GridWait wait{static_cast<uint32_t>(blocks), kBarrierLimitNs};
   const int32_t injected = g_grid_failure.load();
   if (injected == CGP_GRID_DOES_NOT_FIT) return 0;
-  if (injected == CGP_GRID_BLOCK_MISSING) wait = {wait.blocks + 1, 50 * 1000 * 1000};
-  void* args[] = {&L.g, &L.G, &levels, &heavy, &wait};
+  int flags = L.heavy_push ? kTraverseHeavy : 0;
+  if (injected == CGP_GRID_BLOCK_MISSING && blocks > 1) flags |= kTraverseBlockMissing;
+  void* args[] = {&L.g, &L.G, &levels, &flags};
   const cudaError_t e = cudaLaunchCooperativeKernel(k.fn, dim3(blocks), dim3(kBlock), args, 0, s);
   if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the GPU is reserved: launch the levels
     cudaGetLastError();

@@ -3537,8 +3537,8 @@ __global__ void k_level_end_loop(GroupDev g, cudaGraphConditionalHandle loop, in
 // Barrier over all blocks of a cooperative launch.  The last block to arrive
 // runs `last(lane)` with its first warp before it lets the others go, so the
 // end of a level costs no barrier of its own.  A wait gives up after
-// `limit_ns` (the other blocks are co-resident, so this means the device is not
-// running them), raises kStatusBarrier and tells every block to leave: wait()
+// ctl->bar_limit_ns (the other blocks are co-resident, so this means the device is
+// not running them), raises kStatusBarrier and tells every block to leave: wait()
 // then returns false in all of them.
 
 __device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
@@ -3559,14 +3559,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 struct GridBarrier {
   LevelCtl* ctl;
-  unsigned nblk;   // arrivals that complete a barrier
+  unsigned nblk;
   unsigned epoch;  // barriers passed
-  unsigned long long limit_ns;
 
   // Every block reads the epoch before it first arrives, so none can miss a
   // release of this launch.
-  __device__ __forceinline__ GridBarrier(LevelCtl* c, const GridWait& w)
-      : ctl(c), nblk(w.blocks), epoch(load_acquire(&c->bar_release)), limit_ns(w.limit_ns) {}
+  __device__ __forceinline__ GridBarrier(LevelCtl* c, unsigned n)
+      : ctl(c), nblk(n), epoch(load_acquire(&c->bar_release)) {}
 
   template <typename F>
   __device__ __forceinline__ bool wait(F&& last) {
@@ -3599,7 +3598,7 @@ struct GridBarrier {
           }
           const unsigned long long t = global_ns();
           if (t0 == 0) t0 = t;
-          if (t - t0 > limit_ns) {
+          if (t - t0 > ctl->bar_limit_ns) {
             atomicOr(&ctl->status, kStatusBarrier);
             __threadfence();
             store_release(&ctl->bar_abort, 1u);
@@ -3641,12 +3640,16 @@ union TraverseSmem {
 // their launches are the level's whole time.
 template <int W, typename OT, int DEPTH, int WK, bool kSssp>
 __global__ void __launch_bounds__(kBlock, 3) k_traverse(GroupDev g, DevGraph G,
-                                                        int levels, bool heavy, GridWait wait) {
+                                                        int levels, int flags) {
   static_assert(W <= 4, "wider groups are launched level by level");
   __shared__ TraverseSmem<W, kSssp> sm;
   const unsigned bid = blockIdx.x, nblk = gridDim.x;
   LevelCtl* ctl = g.ctl;
-  GridBarrier bar(ctl, wait);
+  // held across the levels, a limit or a count of blocks of its own would cost the
+  // phases registers they do not have
+  GridBarrier bar(ctl, nblk);
+  const bool heavy = flags & kTraverseHeavy;
+  if ((flags & kTraverseBlockMissing) && bid == 0) return;
   bool swept = false;  // the previous level zeroed its own frontier's masks
   for (int l = 0; l < levels; ++l) {
     if (ctl->done) return;
@@ -3709,16 +3712,14 @@ __global__ void __launch_bounds__(kBlock, 3) k_traverse(GroupDev g, DevGraph G,
       }
       if (gather) {
         // heavy vertices first: the light ones read their lowered distances
-        if (G.n_sheavy > 0) {
+        if (G.n_sheavy > 0)
           sssp_pull_heavy_chunks<W, OT, WK, 3>(g, G, bid, nblk, sm.gather_heavy);
-          if (!bar.wait()) return;
-        } else if (bfs && !bfs_pull && !scatter) {
-          // the light gather stores whole vectors of a row: depths a push of this
-          // level writes into the same vectors must be in place before their row
-          // is read (after a scatter, a pull or a heavy gather they are; the heavy
-          // gather itself only lowers its own words)
-          if (!bar.wait()) return;
-        }
+        // The light gather stores whole vectors of a row: depths a push of this
+        // level writes into the same vectors must be in place before their row is
+        // read.  After a scatter or a pull they are; the heavy gather only lowers
+        // its own words and may run beside a push.
+        const bool pushed = bfs && !bfs_pull && !scatter;
+        if ((G.n_sheavy > 0 || pushed) && !bar.wait()) return;
         sssp_pull_light_rows<W, OT, WK, W>(g, G, bid, nblk, sm.gather_light);
       }
       if (ctl->chunk_dir) {

@@ -285,8 +285,8 @@ cgp_status cgp_debug_fail_allocations(int64_t after);
 
 /* Fault-injection hook for tests: until it is called with CGP_GRID_OK, every
  * fused level loop (CGP_LOOP_AUTO) is launched as if the GPU could not hold its
- * blocks at once (the levels are launched one by one instead), or with a grid
- * barrier that waits for one block more than there are, for 50 ms (the call
+ * blocks at once (the levels are launched one by one instead), or one of its
+ * blocks leaves at once and the others wait for it, 50 ms at most (the call
  * returns CGP_ERR_DEVICE and leaves the graph usable). */
 #define CGP_GRID_OK 0
 #define CGP_GRID_DOES_NOT_FIT 1
