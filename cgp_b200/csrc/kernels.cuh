@@ -3717,8 +3717,9 @@ __global__ void __launch_bounds__(kBlock, 3) k_traverse(GroupDev g, DevGraph G,
         // The light gather stores whole vectors of a row: depths a push of this
         // level writes into the same vectors must be in place before their row is
         // read.  After a scatter or a pull they are; the heavy gather only lowers
-        // its own words and may run beside a push.
-        const bool pushed = bfs && !bfs_pull && !scatter;
+        // its own words and may run beside a push.  (Read again: as values kept over
+        // the heavy gather the level's flags cost it spills.)
+        const bool pushed = ctl->has_bfs && ctl->dir == kDirPush && !ctl->sscatter;
         if ((G.n_sheavy > 0 || pushed) && !bar.wait()) return;
         sssp_pull_light_rows<W, OT, WK, W>(g, G, bid, nblk, sm.gather_light);
       }
